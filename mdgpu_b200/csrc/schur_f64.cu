@@ -2,23 +2,33 @@
 // panel (the FP64 counterpart of the tensor-core kernel in schur_tc.cu, same
 // work lists and tile enumeration):
 //     C(I, J) -= A_I * A_J'     128 x 128 tile, K <= 256 panel columns
-// FP64 has no tcgen05 kind, so this is a register-tiled FMA kernel: 256
-// threads, 8 x 8 outputs per thread (rows ty*4+{0..3} and ty*4+64+{0..3},
-// columns likewise, which keeps shared-memory reads conflict-free), operand
-// chunks of 16 columns double-buffered in shared memory with cp.async.
+// on the FP64 matrix instructions (dmma.cuh): a tile is four CTAs of 64 x 64
+// (128 threads, warps of 32 x 32, three CTAs per SM, so one CTA's epilogue
+// runs under the others' products), operand chunks of 16 panel columns
+// through a three-stage cp.async ring.  Bound by the FP64 pipe (37 TFLOP/s
+// measured): 16.4 k cycles of an SM per CTA for 0.3 MB of operands and C.
+// Measured on the 48^3 grid's FP64 factor (80 launches): 6.5 ms, 18 TFLOP/s
+// with the launches' tails, against 14.1 ms for 128 x 128 tiles of register
+// FMAs (an LDS.128 per four of them) and 7.8 ms for CTAs of 64 x 128 (two per
+// SM, half as many to fill the chip's last wave).
 #include <cuda_runtime.h>
 
 #include <cstdint>
 
 #include "device_common.cuh"
+#include "dmma.cuh"
 #include "kernels.hpp"
 
 namespace mdgpu {
 
 namespace f64k {
-constexpr int BM = 128, KC = 16, THREADS = 256;
-constexpr int STAGE = 2 * KC * BM;  // doubles: A and B chunk
-constexpr size_t SMEM_BYTES = 2 * STAGE * sizeof(double);
+constexpr int BT = 128;  // the work lists' tile
+constexpr int KC = 16, THREADS = 128, STAGES = 3;
+constexpr int BM = 64, BN = 64, PIECES = (BT / BM) * (BT / BN);
+constexpr int LDA = BM + 4, LDB = BN + 4;
+constexpr int STAGE = KC * (LDA + LDB);  // doubles: A and B chunk
+constexpr size_t SMEM_BYTES = (size_t)STAGES * STAGE * sizeof(double);
+constexpr int MT = 2, NT = 2;  // a warp's 32 x 32
 }  // namespace f64k
 
 __device__ __forceinline__ void cp_async16(void* dst, const void* src, int src_bytes) {
@@ -28,103 +38,110 @@ __device__ __forceinline__ void cp_async16(void* dst, const void* src, int src_b
                  : "memory");
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
-__device__ __forceinline__ void cp_async_wait_one() { asm volatile("cp.async.wait_group 1;" ::: "memory"); }
 
-__global__ void __launch_bounds__(256)
+// rows r0 .. r0 + R - 1 (zeros from row m on) of the panel columns [col, col +
+// 16) that lie before kend, into dst (ld LD)
+template <int R, int LD>
+__device__ __forceinline__ void load_rows(double* dst, const double* panelp, int64_t ldl, int r0,
+                                          int m, int col, int kend) {
+    constexpr int PAIRS = R / 2, STEP = f64k::THREADS / PAIRS;
+    const int r2 = (threadIdx.x % PAIRS) * 2, row = r0 + r2;
+#pragma unroll
+    for (int q = threadIdx.x / PAIRS; q < f64k::KC; q += STEP) {
+        // rows beyond the front (or a partial pair) and columns beyond the
+        // panel are zero-filled; the source address then stays in bounds
+        const int bytes = (col + q < kend && row < m) ? min(2, m - row) * 8 : 0;
+        cp_async16(dst + q * LD + r2, panelp + (bytes ? (int64_t)(col + q) * ldl + row : 0), bytes);
+    }
+}
+
+__global__ void __launch_bounds__(f64k::THREADS, 3)
     k_schur_f64(const FrontDesc* __restrict__ fronts, const int* __restrict__ items,
                 const int* __restrict__ before, int nitems, int panel, int PW,
                 double* __restrict__ Ls, double* __restrict__ Us) {
     using namespace f64k;
     extern __shared__ __align__(16) double sm[];
-    const int it = find_item(before, nitems, blockIdx.x);
+    const int tile = blockIdx.x / PIECES, piece = blockIdx.x % PIECES;
+    const int it = find_item(before, nitems, tile);
     const FrontDesc f = fronts[items[it]];
     const int k0 = panel * PW;
     const int K = min(PW, f.c - k0);
     const int cbeg = min(k0 + PW, f.c);
     int ii, jj;
-    lower_index(blockIdx.x - before[it], ii, jj);
-    const int I = cbeg / BM + ii, J = cbeg / BM + jj;
-    const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+    lower_index(tile - before[it], ii, jj);
+    // this piece's first row and column
+    const int R0 = (cbeg / BT + ii) * BT + (piece % (BT / BM)) * BM;
+    const int C0 = (cbeg / BT + jj) * BT + (piece / (BT / BM)) * BN;
+    // nothing below the diagonal, or past the front, or before the update's
+    // first column
+    if (C0 > R0 + BM - 1 || R0 >= f.m || C0 + BN <= cbeg) return;
     const double* panelp = Ls + f.loff;
     const int nchunks = (K + KC - 1) / KC;
+    const int warp = threadIdx.x >> 5;
+    const int wr = (warp & 1) * 32, wc = (warp >> 1) * (BN / 2);
+    const bool active = C0 + wc <= R0 + wr + 31 && R0 + wr < f.m && C0 + wc + BN / 2 > cbeg;
 
-    // each thread copies 4 x 16 bytes of A and 4 x 16 bytes of B per chunk:
-    // element pair (row 2*(tid & 63), column (tid >> 6) + 4*u)
-    auto load_chunk = [&](int ch, int stage) {
-        double* As = sm + stage * STAGE;
-        double* Bs = As + KC * BM;
-        const int r2 = (tid & 63) * 2;
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const int q = (tid >> 6) + 4 * u;  // chunk column
-            const int col = k0 + ch * KC + q;
-            const bool colok = (ch * KC + q) < K;
-            const int ra = I * BM + r2, rb = J * BM + r2;
-            // rows beyond the front (or a partial pair) and columns beyond the
-            // panel are zero-filled; the source address then stays in bounds
-            const int na = (colok && ra < f.m) ? min(2, f.m - ra) * 8 : 0;
-            const int nb = (colok && rb < f.m) ? min(2, f.m - rb) * 8 : 0;
-            const double* sa = panelp + (na ? (int64_t)col * f.ldl + ra : 0);
-            const double* sb = panelp + (nb ? (int64_t)col * f.ldl + rb : 0);
-            cp_async16(As + q * BM + r2, sa, na);
-            cp_async16(Bs + q * BM + r2, sb, nb);
+    auto load_chunk = [&](int ch) {
+        if (ch < nchunks) {
+            double* As = sm + (ch % STAGES) * STAGE;
+            load_rows<BM, LDA>(As, panelp, f.ldl, R0, f.m, k0 + ch * KC, k0 + K);
+            load_rows<BN, LDB>(As + KC * LDA, panelp, f.ldl, C0, f.m, k0 + ch * KC, k0 + K);
         }
         cp_async_commit();
     };
 
-    double acc[8][8];
+    double acc[MT][NT][2][4];
 #pragma unroll
-    for (int a = 0; a < 8; ++a)
+    for (int m = 0; m < MT; ++m)
 #pragma unroll
-        for (int b = 0; b < 8; ++b) acc[a][b] = 0.0;
+        for (int n = 0; n < NT; ++n)
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) acc[m][n][h][e] = 0.0;
 
-    load_chunk(0, 0);
+    load_chunk(0);
+    load_chunk(1);
     for (int ch = 0; ch < nchunks; ++ch) {
-        if (ch + 1 < nchunks) {
-            load_chunk(ch + 1, (ch + 1) & 1);
-            cp_async_wait_one();
-        } else {
-            cp_async_wait_all();
-        }
-        __syncthreads();
-        const double* As = sm + (ch & 1) * STAGE;
-        const double* Bs = As + KC * BM;
-#pragma unroll 4
-        for (int q = 0; q < KC; ++q) {
-            const double2* ar = reinterpret_cast<const double2*>(As + q * BM);
-            const double2* br = reinterpret_cast<const double2*>(Bs + q * BM);
-            double2 a0 = ar[ty * 2], a1 = ar[ty * 2 + 1], a2 = ar[32 + ty * 2],
-                    a3 = ar[32 + ty * 2 + 1];
-            double2 b0 = br[tx * 2], b1 = br[tx * 2 + 1], b2 = br[32 + tx * 2],
-                    b3 = br[32 + tx * 2 + 1];
-            const double av[8] = {a0.x, a0.y, a1.x, a1.y, a2.x, a2.y, a3.x, a3.y};
-            const double bv[8] = {b0.x, b0.y, b1.x, b1.y, b2.x, b2.y, b3.x, b3.y};
-#pragma unroll
-            for (int a = 0; a < 8; ++a)
-#pragma unroll
-                for (int b = 0; b < 8; ++b) acc[a][b] = fma(av[a], bv[b], acc[a][b]);
-        }
-        __syncthreads();
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
+        __syncthreads();  // chunk ch landed for everyone; chunk ch - 1 is consumed
+        load_chunk(ch + 2);
+        const double* As = sm + (ch % STAGES) * STAGE;
+        if (active)
+            dmma_k16<MT, NT, LDA, LDB>(As + wr, As + KC * LDA + wc, acc);
     }
-    // epilogue: gather addresses and old values of a row, then write
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    if (!active) return;
+    // epilogue, 16 columns at a time: a lane's 4 columns of two adjacent rows
+    // per 16-row block, old values gathered first
+    const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
 #pragma unroll
-    for (int a = 0; a < 8; ++a) {
-        const int row = I * BM + (a < 4 ? ty * 4 + a : 64 + ty * 4 + (a - 4));
-        if (row >= f.m) continue;
-        double* p[8];
-        double old[8];
+    for (int n = 0; n < NT; ++n) {
+        double* p[MT][2][4];
+        double old[MT][2][4];
 #pragma unroll
-        for (int b = 0; b < 8; ++b) {
-            const int col = J * BM + (b < 4 ? tx * 4 + b : 64 + tx * 4 + (b - 4));
-            const bool ok = col >= cbeg && col < f.m && row >= col;
-            p[b] = ok ? front_elem(Ls, Us, f, row, col) : nullptr;
-        }
+        for (int m = 0; m < MT; ++m)
 #pragma unroll
-        for (int b = 0; b < 8; ++b) old[b] = p[b] ? *p[b] : 0.0;
+            for (int r = 0; r < 2; ++r)
 #pragma unroll
-        for (int b = 0; b < 8; ++b)
-            if (p[b]) *p[b] = old[b] - acc[a][b];
+                for (int k = 0; k < 4; ++k) {
+                    const int row = R0 + wr + 16 * m + 2 * g + r, col = C0 + wc + 16 * n + 4 * t + k;
+                    const bool ok = row < f.m && col >= cbeg && row >= col;
+                    p[m][r][k] = ok ? front_elem(Ls, Us, f, row, col) : nullptr;
+                }
+#pragma unroll
+        for (int m = 0; m < MT; ++m)
+#pragma unroll
+            for (int r = 0; r < 2; ++r)
+#pragma unroll
+                for (int k = 0; k < 4; ++k) old[m][r][k] = p[m][r][k] ? *p[m][r][k] : 0.0;
+#pragma unroll
+        for (int m = 0; m < MT; ++m)
+#pragma unroll
+            for (int r = 0; r < 2; ++r)
+#pragma unroll
+                for (int k = 0; k < 4; ++k)
+                    if (p[m][r][k]) *p[m][r][k] = old[m][r][k] - acc[m][n][k & 1][2 * r + (k >> 1)];
     }
 }
 
@@ -135,7 +152,7 @@ void init_schur_f64() {
 
 void launch_schur_f64(const DevPlan& D, const WorkList& w, int panel, int PW, double* Ls,
                       double* Us, cudaStream_t st) {
-    k_schur_f64<<<w.nctas, f64k::THREADS, f64k::SMEM_BYTES, st>>>(
+    k_schur_f64<<<w.nctas * f64k::PIECES, f64k::THREADS, f64k::SMEM_BYTES, st>>>(
         D.fronts, D.psched.items + w.off, D.psched.before + w.off, w.nitems, panel, PW, Ls, Us);
 }
 

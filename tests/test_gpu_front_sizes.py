@@ -1,0 +1,60 @@
+"""Fronts of chosen sizes (-m gpu): two leaf fronts of c1 and c2 pivot columns
+under one root of u rows, every block dense, so each front's rows and pivot
+columns sit where the kernels' tiles end (64 x 64 pieces, 128-tiles,
+256-column panels, the small / large boundary at 160 rows, odd leading rows).
+
+Oracle: dense FP64 numpy on the same matrix.  Tolerance: a backward stable
+Cholesky of order n and condition k returns L to n eps k; the matrices here
+are diagonally dominant with condition below 10 and n below 1000, so 1e-12
+leaves a factor of ten over 1000 * 2.2e-16 * 0.5.
+"""
+import numpy as np
+import pytest
+
+import mdgpu_b200 as M
+
+pytestmark = pytest.mark.gpu
+
+torch = pytest.importorskip("torch")
+if not torch.cuda.is_available():  # pragma: no cover - collected only on GPU boxes
+    pytest.skip("needs a CUDA device", allow_module_level=True)
+
+SIZES = [(1, 2, 161), (33, 97, 64), (64, 65, 127), (63, 129, 128), (161, 31, 130), (255, 192, 33),
+         (256, 257, 191), (300, 64, 257)]
+
+
+def _two_leaves(c1, c2, u, seed=0):
+    """Dense symmetric matrix of the two-leaf pattern and its lower CSC."""
+    n = c1 + c2 + u
+    r = np.random.default_rng(seed)
+    A = r.uniform(-1.0, 1.0, (n, n))
+    A = 0.5 * (A + A.T)
+    A[c1:c1 + c2, :c1] = 0.0
+    A[:c1, c1:c1 + c2] = 0.0
+    np.fill_diagonal(A, 1.5 * np.abs(A).sum(axis=1))
+    Ai, Ap = [], [0]
+    for j in range(n):
+        rows = np.arange(j, n)
+        if j < c1:
+            rows = rows[(rows < c1) | (rows >= c1 + c2)]
+        Ai.append(rows)
+        Ap.append(Ap[-1] + len(rows))
+    Ai = np.concatenate(Ai)
+    cols = np.repeat(np.arange(n), np.diff(Ap))
+    return n, A, np.array(Ap, np.int32), Ai.astype(np.int32), A[Ai, cols]
+
+
+def _dense_L(S):
+    Lp, Li, Lx = S.get_L()
+    L = np.zeros((S.n, S.n))
+    L[Li, np.repeat(np.arange(S.n), np.diff(Lp))] = Lx
+    return L
+
+
+@pytest.mark.parametrize("c1,c2,u", SIZES)
+def test_fp64_factor(c1, c2, u):
+    n, A, Ap, Ai, Ax = _two_leaves(c1, c2, u)
+    S = M.Solver(n, Ap, Ai, ordering=M.ORDER_NATURAL)
+    S.factor(torch.from_numpy(Ax).cuda(), M.FP64)
+    ref = np.linalg.cholesky(A)
+    assert np.linalg.norm(_dense_L(S) - ref) <= 1e-12 * np.linalg.norm(ref)
