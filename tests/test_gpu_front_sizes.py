@@ -58,3 +58,18 @@ def test_fp64_factor(c1, c2, u):
     S.factor(torch.from_numpy(Ax).cuda(), M.FP64)
     ref = np.linalg.cholesky(A)
     assert np.linalg.norm(_dense_L(S) - ref) <= 1e-12 * np.linalg.norm(ref)
+
+
+@pytest.mark.parametrize("c1,c2,u", SIZES)
+def test_fp32_factor(c1, c2, u):
+    """FP32 factor: sqrt(n) u_32 cond = 30 * 6e-8 * 10 = 2e-5 bounds the
+    expected forward error of L; refinement reaches 1e-14."""
+    n, A, Ap, Ai, Ax = _two_leaves(c1, c2, u)
+    S = M.Solver(n, Ap, Ai, ordering=M.ORDER_NATURAL)
+    S.factor(torch.from_numpy(Ax).cuda(), M.FP32)
+    ref = np.linalg.cholesky(A)
+    assert np.linalg.norm(_dense_L(S) - ref) <= 2e-5 * np.linalg.norm(ref)
+    b = np.random.default_rng(1).uniform(-1.0, 1.0, n)
+    x, berr, _ = S.refine(b)
+    r = b - A @ x
+    assert np.abs(r).max() <= 1e-14 * (np.abs(A).sum(1).max() * np.abs(x).max() + np.abs(b).max())
