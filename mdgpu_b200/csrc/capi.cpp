@@ -115,6 +115,7 @@ struct mdgpu_handle_s {
     float* dD32 = nullptr;
     double *d_xp = nullptr, *d_fv = nullptr, *d_B = nullptr, *d_X = nullptr, *d_R = nullptr,
            *d_D = nullptr;
+    int* d_ssync = nullptr;  // sync words of the solve
     int nrhs_cap = 0;
     // CUDA graphs of the numeric launch sequences (captured once, replayed)
     bool use_graphs = true;
@@ -161,7 +162,7 @@ struct mdgpu_handle_s {
         for (void* p : {(void*)d_Fb, (void*)d_Fu, (void*)d_W, (void*)d_Lbar, (void*)d_Abar})
             if (p) cudaFree(p);
         for (void* p : {(void*)dZ64, (void*)dZu64, (void*)d_Y, (void*)d_logdet, (void*)d_gx, (void*)d_gG,
-                        (void*)d_gm})
+                        (void*)d_gm, (void*)d_ssync})
             if (p) cudaFree(p);
         for (void* p : {(void*)d_Ax, (void*)dL64, (void*)dU64, (void*)dL32, (void*)dU32,
                         (void*)dD64, (void*)dD32,
@@ -492,8 +493,11 @@ void upload_plan(mdgpu_handle_s* h, bool check = false) {
         }
         D.solve.bwd_target = h->keep(upload(SS.bwd_target));
         D.solve.nfronts = P.nsuper;
-        D.solve.nsync = 3 + SS.nflags + 3 * P.nsuper;
-        D.solve.sync = h->keep(dalloc<int>(D.solve.nsync));
+        // one group of right-hand sides (all that a solve that may not
+        // allocate can count on; ensure_solve_storage grows it)
+        h->d_ssync = dalloc<int>(solve_sync_words(SS.nflags, P.nsuper, 1));
+        D.solve.sync = h->d_ssync;
+        D.solve.sync_groups = 1;
     }
     // algorithmic work per launch, for the profiler's roofline figures
     {
@@ -608,6 +612,7 @@ void ensure_factor_storage(mdgpu_handle_s* h, int precision) {
 void ensure_solve_storage(mdgpu_handle_s* h, int nrhs) {
     if (nrhs <= h->nrhs_cap) return;
     h->drop_solve_graphs();  // they reference the buffers replaced below
+    h->nrhs_cap = 0;
     for (double** p : {&h->d_xp, &h->d_fv, &h->d_B, &h->d_X, &h->d_R, &h->d_D})
         if (*p) {
             cudaFree(*p);
@@ -619,6 +624,14 @@ void ensure_solve_storage(mdgpu_handle_s* h, int nrhs) {
     }
     int64_t n = h->plan.n;
     int chunk = std::min(nrhs, 64);
+    const int groups = solve_groups(chunk);
+    if (groups > h->D.solve.sync_groups) {
+        int* grown = dalloc<int>(solve_sync_words(h->D.solve.nflags, h->plan.nsuper, groups));
+        cudaFree(h->d_ssync);
+        h->d_ssync = grown;
+        h->D.solve.sync = h->d_ssync;
+        h->D.solve.sync_groups = groups;
+    }
     h->d_xp = dalloc<double>(n * nrhs);
     h->d_fv = dalloc<double>(h->D.fv_total * chunk);
     h->d_B = dalloc<double>(n * nrhs);

@@ -92,12 +92,13 @@ struct DevSchedule {
 };
 
 // Solve: one launch per direction over every level's work items (see
-// SolveScheduleHost).  sync holds the two ticket counters, one count per
-// pivot tile (backward gathers counted in), the abort word, then per front
-// the forward count of finished children, the forward count of finished
-// update tiles and the backward count of finished completions; it is
-// cleared at the start of every solve.  err (not cleared by the solve) gets
-// bit 0 when a dependency wait ran out.
+// SolveScheduleHost).  sync holds the two ticket counters and the abort word,
+// then per group of right-hand sides (sync_groups of them) one count per
+// pivot tile (backward gathers counted in) and per front the forward count of
+// finished children, the forward count of finished update tiles and the
+// backward count of finished completions; it is cleared at the start of every
+// solve.  err (not cleared by the solve) gets bit 0 when a dependency wait ran
+// out.
 struct SolveSchedule {
     int2* tasks = nullptr;
     int4* fwd_items = nullptr;
@@ -111,7 +112,8 @@ struct SolveSchedule {
     std::vector<double> fwd_elems, bwd_elems;     // per level: L + Dinv elements
     std::vector<double> small_elems;              // per level: L elements of small fronts
     int* sync = nullptr;
-    int nsync = 0, nflags = 0;
+    int sync_groups = 0;  // groups of right-hand sides the sync words hold
+    int nflags = 0;
     int* err = nullptr;
     // backward update-row partial sums (see SolveScheduleHost)
     std::vector<int> gather_task_beg;
@@ -268,6 +270,10 @@ void factor_levels(const DevPlan& D, T* Ls, T* Us, T* Dinv, const double* Ax, in
 template <typename TL, typename TV>
 void solve_levels(const DevPlan& D, const TL* Ls, const TL* Dinv, TV* xp, TV* fv, int nrhs,
                   cudaStream_t st);
+
+// groups of right-hand sides of one solve launch, and the sync words they need
+int solve_groups(int nrhs);
+int64_t solve_sync_words(int nflags, int nfronts, int groups);
 
 // Per large front a map over its panel scratch (base scr + scr_off[s],
 // row-major, kPanel columns): bf16, the BF16 copy (mpad rows); else the

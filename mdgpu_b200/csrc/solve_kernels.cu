@@ -8,10 +8,9 @@
 // f[c:m] - L21 y as its own update part.  Backward reads the already final
 // solution entries of its update rows (ancestors) directly.
 //
-// Small fronts: one CTA per front.  Large fronts: tiled, one launch per
-// 64-row block of the diagonal block, many CTAs per launch; every CTA applies
-// the block's inverse (stored by the factorization) redundantly -- a 64 x 64
-// product, no serial substitution -- so no launch needs a second phase.
+// Small fronts: a warp (or a part of one) per front.  Large fronts: tasks of
+// 64-row tiles; a pivot tile applies its block's inverse (stored by the
+// factorization), a 64 x 64 product instead of a serial substitution.
 #include <algorithm>
 
 #include "device_common.cuh"
@@ -41,7 +40,9 @@ __device__ inline TV* front_vec(TV* fv, const int64_t* fv_off, int s, int nrhs) 
 
 constexpr int kSolveWaitPolls = 1 << 18;  // ~0.1-0.3 s at ~1 us per poll
 constexpr int kWarpSolveRhs = 4;   // right-hand sides per pass of the warp path
-constexpr int kSolvePassRhs = 32;  // right-hand sides per pass of the solve launches
+constexpr int kVecLD = kTile + 4;  // column stride of a vector block in shared memory: 4 mod 16
+                                   // doubles, a conflict-free operand of the matrix instructions
+constexpr int kGroupRhs = 8;       // right-hand sides of one group (a matrix instruction's columns)
 
 __device__ __forceinline__ int ld_acquire_gpu(const int* p) {
     int v;
@@ -99,6 +100,7 @@ __device__ __forceinline__ void st_relaxed_f64(double* p, double v) {
 __device__ __forceinline__ bool is_unpublished(double v) {
     return __double_as_longlong(v) == -1ll;
 }
+// (src: the slot, column after column of 64 rows; dst: columns kVecLD apart)
 __device__ bool poll_published(double* dst, const double* src, int nk, int nrhs, int* abort_flag,
                                int* err) {
     constexpr int T = kTile;
@@ -128,7 +130,7 @@ __device__ bool poll_published(double* dst, const double* src, int nk, int nrhs,
                 __nanosleep(32);
             }
         }
-        if (ok) dst[e] = need ? v : 0.0;
+        if (ok) dst[(e / T) * kVecLD + (e & (T - 1))] = need ? v : 0.0;
     }
     return __syncthreads_and(ok);
 }
@@ -159,12 +161,14 @@ __device__ __forceinline__ void cp_async_wait_groups() {
 // offsets of 32), the inverses' on 64 * 64 elements.
 template <typename TL>
 __host__ __device__ constexpr int blk_ld() {
-    return kTile + 16 / (int)sizeof(TL);
+    return kTile + 4;
 }
 template <typename TL>
 __device__ __forceinline__ int blk_off(int start) {
     return start & (16 / (int)sizeof(TL) - 1);
 }
+// (blk_ld = 68: 4 mod 16 doubles and 4 mod 32 floats, the bank spread of the
+// four columns that a matrix-instruction operand takes at once)
 // rows start .. start + nr - 1 and columns 0 .. nc - 1 of the matrix at src
 // (column stride ld)
 template <typename TL>
@@ -184,7 +188,7 @@ __device__ __forceinline__ void load_block_async(TL* dst, const TL* src, int64_t
 }
 
 // ---------------------------------------------------------------------------
-// large-front tile tasks: a pipeline of `stg` stages streams the L blocks a
+// large-front tile tasks: a pipeline of two stages streams the L blocks a
 // task multiplies, each with the vector block it is multiplied by (a pivot
 // tile's published solution, or gathered solution rows), by cp.async; the
 // block in use is consumed while the next ones load.  Published vectors come
@@ -192,57 +196,46 @@ __device__ __forceinline__ void load_block_async(TL* dst, const TL* src, int64_t
 // sentinel falls back to polling that slot.
 // ---------------------------------------------------------------------------
 
-template <typename TL>
-__host__ __device__ constexpr int level_stages(int nrhs) {
-    return 2;
-}
+constexpr int kSolveStages = 2;
 
-// shared memory: diagonal inverse block, stg L blocks, stg vector blocks, a
-// vector, the quarter reduction, the gather's row indices
-template <typename TL, typename TV>
-__host__ __device__ constexpr size_t level_smem_bytes(int nrhs) {
-    return (((1 + (size_t)level_stages<TL>(nrhs)) * kTile * blk_ld<TL>() * sizeof(TL) + 15) / 16) * 16 +
-           (((size_t)level_stages<TL>(nrhs) + 1) * kTile * nrhs + 4 * kTile) * sizeof(TV) +
+// shared memory of a tile task: the stages' L blocks, their vector blocks, a
+// vector, the gather's row indices; one right-hand side also keeps the
+// diagonal inverse in a block of its own (several take it through the stages,
+// after the last L block)
+template <typename TL, bool MULTI>
+__host__ __device__ constexpr size_t level_smem_bytes() {
+    return ((size_t)(kSolveStages + (MULTI ? 0 : 1)) * kTile * blk_ld<TL>()) * sizeof(TL) +
+           (size_t)(kSolveStages + 1) * kVecLD * (MULTI ? kGroupRhs : 1) * sizeof(double) +
            (size_t)SolveScheduleHost::kGatherTiles * kTile * sizeof(int);
 }
 
-template <typename TL, typename TV>
+template <typename TL, bool MULTI>
 struct LevelSmem {
-    TL* Dk;   // T x LD
-    TL* Lst;  // stg x T x LD
-    TV* Vst;  // stg x T x nrhs
-    TV* Y;    // T x nrhs
-    TV* red;  // 4 x T
-    int* idx; // kGatherTiles x T
-    int stg;
-    __device__ explicit LevelSmem(int nrhs) {
+    static constexpr int VB = kVecLD * (MULTI ? kGroupRhs : 1);
+    TL* Lst;      // stages x T x LD
+    TL* Dk;       // T x LD (one right-hand side)
+    double* Vst;  // stages x VB
+    double* Y;    // VB
+    int* idx;     // kGatherTiles x T
+    __device__ LevelSmem() {
         constexpr int T = kTile, LD = blk_ld<TL>();
         extern __shared__ __align__(16) unsigned char smem_raw[];
-        stg = level_stages<TL>(nrhs);
-        Dk = reinterpret_cast<TL*>(smem_raw);
-        Lst = Dk + T * LD;
-        Vst = reinterpret_cast<TV*>(smem_raw +
-                                    (((1 + (size_t)stg) * T * LD * sizeof(TL) + 15) / 16) * 16);
-        Y = Vst + (size_t)stg * T * nrhs;
-        red = Y + T * nrhs;
-        idx = reinterpret_cast<int*>(red + 4 * T);
+        Lst = reinterpret_cast<TL*>(smem_raw);
+        Dk = Lst + kSolveStages * T * LD;
+        Vst = reinterpret_cast<double*>(Dk + (MULTI ? 0 : T * LD));
+        Y = Vst + kSolveStages * VB;
+        idx = reinterpret_cast<int*>(Y + VB);
     }
-    __device__ TL* lb(int p) const { return Lst + (p % stg) * kTile * blk_ld<TL>(); }
-    __device__ TV* vb(int p, int nrhs) const { return Vst + (size_t)(p % stg) * kTile * nrhs; }
+    __device__ TL* lb(int p) const { return Lst + (p % kSolveStages) * kTile * blk_ld<TL>(); }
+    __device__ double* vb(int p) const { return Vst + (p % kSolveStages) * VB; }
 };
-
-__device__ __forceinline__ void cp_async_wait_stages(int stg) {
-    if (stg >= 3)
-        cp_async_wait_groups<2>();
-    else
-        cp_async_wait_groups<1>();
-}
 
 // a published T x nrhs slot into a stage (16-byte copies through L2; T * nrhs
 // is even and slots start on 16 bytes)
 __device__ __forceinline__ void load_slot_async(double* dst, const double* src, int nrhs) {
     for (int q = threadIdx.x; q < kTile * nrhs / 2; q += blockDim.x) {
-        const uint32_t da = static_cast<uint32_t>(__cvta_generic_to_shared(dst + 2 * q));
+        const uint32_t da = static_cast<uint32_t>(__cvta_generic_to_shared(
+            dst + (2 * q / kTile) * kVecLD + ((2 * q) & (kTile - 1))));
         asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(da), "l"(src + 2 * q)
                      : "memory");
     }
@@ -255,9 +248,10 @@ __device__ __forceinline__ bool settle_slot(double* v, const double* src, int nk
                                             int* abort_flag, int* err) {
     bool mine = true;
     for (int e = threadIdx.x; e < kTile * nrhs; e += blockDim.x) {
+        double& x = v[(e / kTile) * kVecLD + (e & (kTile - 1))];
         if ((e & (kTile - 1)) >= nk)
-            v[e] = 0.0;
-        else if (is_unpublished(v[e]))
+            x = 0.0;
+        else if (is_unpublished(x))
             mine = false;
     }
     if (__syncthreads_and(mine)) return true;
@@ -270,30 +264,159 @@ __device__ __forceinline__ bool settle_slot(double* v, const double* src, int nk
 // accumulates acc = sum_{k < min(i, nt1)} L(i, k) y_k over the pivot tiles.
 // A pivot tile (i0 < nt1, cnt = 1) then solves y_i = inv(L_ii) (f_i - acc)
 // into the solution and publishes it; an update tile leaves f_i - acc in the
-// front vector for the parent.  Threads: r = row in the tile; one
-// right-hand side splits the 64 columns of a block over four column phases
-// held by lanes of one warp, several split the right-hand sides (NQ per
-// thread).
-template <typename TL, typename TV, int NQ>
+// front vector for the parent.  One right-hand side: r = row in the tile, the
+// 64 columns of a block split over four column phases held by lanes of one
+// warp (rows 8w .. 8w + 7 of warp w), so a row's sum is two shuffles.
+template <typename TL>
 __device__ void fwd_tile_task(int2 tk, const FrontDesc* __restrict__ fronts,
                               double* __restrict__ pub, int* __restrict__ abort_flag,
                               int* __restrict__ err, const int64_t* __restrict__ fv_off,
                               const int* __restrict__ amap_off, const int* __restrict__ amap_row,
                               const int* __restrict__ amap_ent,
                               const int64_t* __restrict__ dinv_off, const TL* __restrict__ Ls,
-                              const TL* __restrict__ Dinv, TV* __restrict__ xp,
-                              TV* __restrict__ fv, int n, int nrhs) {
-    static_assert(sizeof(TV) == 8, "solve vectors are double");
+                              const TL* __restrict__ Dinv, double* __restrict__ xp,
+                              double* __restrict__ fv) {
     constexpr int T = kTile, LD = blk_ld<TL>();
-    const LevelSmem<TL, TV> sm(nrhs);
-    const bool lsplit = nrhs == 1;
-    // one right-hand side: r = row, g = column phase (columns g, g + 4, ...),
-    // the four phases of a row in one warp (rows 8w .. 8w + 7 of warp w), so
-    // a row's sum is two shuffles; several: r = row, g = quarter of the
-    // right-hand sides
+    const LevelSmem<TL, false> sm;
     const int tid = threadIdx.x;
-    const int r = lsplit ? 8 * (tid >> 5) + (tid & 7) : tid & (T - 1);
-    const int g = lsplit ? (tid >> 3) & 3 : tid >> 6;
+    const int r = 8 * (tid >> 5) + (tid & 7), g = (tid >> 3) & 3;
+    const int s = tk.x, i0 = tk.y & 0xffff, cnt = tk.y >> 16;
+    const FrontDesc F = fronts[s];
+    const int nt1 = tiles_l(F.c, T);
+    const bool pivot = i0 < nt1;
+    const int kend = pivot ? i0 : nt1;  // L blocks per tile
+    const int P = cnt * kend;
+    const TL* L = Ls + F.loff;
+    double* pb = pub + (dinv_off[s] / (T * T)) * T;  // this front's pivot tiles
+    double* f = front_vec(fv, fv_off, s, 1);
+    // the row offset of this task's blocks in their stage columns (every row
+    // tile of a task starts at the same residue: 0 for a pivot tile, c for
+    // update tiles)
+    const int db = blk_off<TL>(tile_range(i0, F.m, F.c, T).start);
+    const int aoff = amap_off[s];
+    // this thread's row of tile i of the front vector
+    auto gather_row = [&](int i) -> double {
+        const TileRange ti = tile_range(i, F.m, F.c, T);
+        const int R = ti.start + r;
+        if (g != 0 || r >= ti.size) return 0.0;
+        double x = R < F.c ? xp[F.first_col + R] : 0.0;
+        const int e1 = amap_row[aoff + R + 1];
+        for (int e = amap_row[aoff + R]; e < e1; ++e) x += __ldcg(fv + (int64_t)amap_ent[e]);
+        return x;
+    };
+    auto issue = [&](int p) {
+        if (p < P) {
+            const int i = i0 + p / kend, k = p % kend;
+            const TileRange ti = tile_range(i, F.m, F.c, T);
+            load_block_async(sm.lb(p), L + (int64_t)k * T * F.ldl, F.ldl, ti.start, ti.size,
+                             min(T, F.c - k * T));
+            load_slot_async(sm.vb(p), pb + (int64_t)k * T, 1);
+        }
+        cp_async_commit_group();
+    };
+    if (pivot) {
+        const TileRange ti = tile_range(i0, F.m, F.c, T);
+        load_block_async(sm.Dk, Dinv + dinv_off[s] + (int64_t)i0 * T * T, T, 0, ti.size, ti.size);
+    }
+    issue(0);
+    double fcur = gather_row(i0), acc = 0.0;
+    double fnext = cnt > 1 ? gather_row(i0 + 1) : 0.0;
+    bool ok = true;
+    for (int p = 0; p < P; ++p) {
+        issue(p + 1);
+        cp_async_wait_groups<1>();
+        __syncthreads();
+        const int i = i0 + p / kend, k = p % kend;
+        double* Yk = sm.vb(p);
+        if (!settle_slot(Yk, pb + (int64_t)k * T, min(T, F.c - k * T), 1, abort_flag, err)) {
+            ok = false;
+            break;
+        }
+        const TL* B = sm.lb(p);
+#pragma unroll
+        for (int l = 0; l < 16; ++l) acc += (double)B[db + r + (g + 4 * l) * LD] * Yk[g + 4 * l];
+        if (!pivot && k == kend - 1) {  // update tile i complete: f_i - acc to the front vector
+            const TileRange ti = tile_range(i, F.m, F.c, T);
+            double v = acc + __shfl_xor_sync(0xffffffffu, acc, 8);
+            v += __shfl_xor_sync(0xffffffffu, v, 16);
+            if (g == 0 && r < ti.size) f[ti.start + r] = fcur - v;
+            acc = 0.0;
+            fcur = fnext;
+            if (i + 2 < i0 + cnt) fnext = gather_row(i + 2);
+        }
+        if (p + 1 < P) __syncthreads();  // the stages are reused; after the last, nothing is
+    }
+    cp_async_wait_groups<0>();
+    if (!ok || !pivot) return;
+    // pivot tile: F = f_i - acc (zero beyond the tile), then y = Dk F; one
+    // barrier: the row's phases summed by shuffles, F into sm.Y, then y the
+    // same way
+    const TileRange ti = tile_range(i0, F.m, F.c, T);
+    double* Y = sm.Y;
+    const TL* Dk = sm.Dk;
+    double a = acc + __shfl_xor_sync(0xffffffffu, acc, 8);
+    a += __shfl_xor_sync(0xffffffffu, a, 16);
+    if (g == 0) Y[r] = r < ti.size ? fcur - a : 0.0;
+    __syncthreads();
+    double y = 0.0;
+#pragma unroll
+    for (int l = 0; l < 16; ++l) y += (double)Dk[r + (g + 4 * l) * LD] * Y[g + 4 * l];
+    y += __shfl_xor_sync(0xffffffffu, y, 8);
+    y += __shfl_xor_sync(0xffffffffu, y, 16);
+    if (g == 0 && r < ti.size) {
+        xp[F.first_col + ti.start + r] = y;
+        st_relaxed_f64(pb + (int64_t)i0 * T + r, y);
+    }
+}
+
+// ---------------------------------------------------------------------------
+// several right-hand sides: groups of up to eight, the columns of one matrix
+// instruction, each group a sweep of its own inside the launch (item k of the
+// list runs for every group in turn, and a group's waits, publication slots
+// and front vectors are its own).  A sweep is a chain of hand-overs between
+// tiles, so eight right-hand sides take about as long as one, and further
+// groups run beside the first on SMs that would idle; L is read once per
+// group, from L2 where the groups follow each other closely.  A warp owns
+// eight rows of a 64-row block: lane (g, t) holds row 8 w + g, right-hand
+// sides 2 t and 2 t + 1 (the accumulator of mma m8n8k4 over FP64).
+// ---------------------------------------------------------------------------
+
+__device__ __forceinline__ void dmma_884(double (&c)[2], double a, double b) {
+    asm volatile(
+        "mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1},{%2},{%3},{%0,%1};"
+        : "+d"(c[0]), "+d"(c[1])
+        : "d"(a), "d"(b));
+}
+// acc += M V over 64 columns of M; M(r, k) at B[db + r + k LD] (TRANS: at
+// B[db + k + r LD]), V(k, q) at V[k + q kVecLD]; two chains of accumulators
+template <typename TL, bool TRANS>
+__device__ __forceinline__ void group_product(const TL* B, int db, const double* V,
+                                              double (&acc)[2][2]) {
+    constexpr int LD = blk_ld<TL>();
+    const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    const int r = 8 * (threadIdx.x >> 5) + g;
+    const TL* Br = B + db + (TRANS ? t + r * LD : r + t * LD);
+    const double* Vg = V + g * kVecLD + t;
+#pragma unroll
+    for (int s = 0; s < kTile / 4; ++s)
+        dmma_884(acc[s & 1], (double)Br[TRANS ? 4 * s : 4 * s * LD], Vg[4 * s]);
+}
+
+// As fwd_tile_task for a group of nrhs <= 8 right-hand sides (xp, fv, pub:
+// the group's own).
+template <typename TL>
+__device__ void fwd_tile_group(int2 tk, const FrontDesc* __restrict__ fronts,
+                               double* __restrict__ pub, int* __restrict__ abort_flag,
+                               int* __restrict__ err, const int64_t* __restrict__ fv_off,
+                               const int* __restrict__ amap_off, const int* __restrict__ amap_row,
+                               const int* __restrict__ amap_ent,
+                               const int64_t* __restrict__ dinv_off, const TL* __restrict__ Ls,
+                               const TL* __restrict__ Dinv, double* __restrict__ xp,
+                               double* __restrict__ fv, int n, int nrhs) {
+    constexpr int T = kTile;
+    const LevelSmem<TL, true> sm;
+    const int r = threadIdx.x >> 2, q = 2 * (threadIdx.x & 3);
+    const bool q0 = q < nrhs, q1 = q + 1 < nrhs;
     const int s = tk.x, i0 = tk.y & 0xffff, cnt = tk.y >> 16;
     const FrontDesc F = fronts[s];
     const int nt1 = tiles_l(F.c, T);
@@ -302,30 +425,23 @@ __device__ void fwd_tile_task(int2 tk, const FrontDesc* __restrict__ fronts,
     const int P = cnt * kend;
     const TL* L = Ls + F.loff;
     double* pb = pub + (dinv_off[s] / (T * T)) * T * nrhs;  // this front's pivot tiles
-    TV* f = front_vec(fv, fv_off, s, nrhs);
-    // the row offset of this task's blocks in their stage columns (every row
-    // tile of a task starts at the same residue: 0 for a pivot tile, c for
-    // update tiles)
+    double* f = front_vec(fv, fv_off, s, nrhs);
     const int db = blk_off<TL>(tile_range(i0, F.m, F.c, T).start);
     const int aoff = amap_off[s];
-    // rows of tile i of the front vector into v (this thread's share)
-    auto gather_rows = [&](int i, TV (&v)[NQ]) {
+    auto gather_row = [&](int i, double (&v)[2]) {
         const TileRange ti = tile_range(i, F.m, F.c, T);
         const int R = ti.start + r;
-        int e0 = 0, e1 = 0;
-        if (r < ti.size) {
-            e0 = amap_row[aoff + R];
-            e1 = amap_row[aoff + R + 1];
+        v[0] = v[1] = 0.0;
+        if (r >= ti.size || !q0) return;
+        if (R < F.c) {
+            v[0] = xp[F.first_col + R + (int64_t)q * n];
+            if (q1) v[1] = xp[F.first_col + R + (int64_t)(q + 1) * n];
         }
-#pragma unroll
-        for (int j = 0; j < NQ; ++j) {
-            const int q = lsplit ? 0 : g + 4 * j;
-            TV x = TV(0);
-            if (r < ti.size && q < nrhs && (!lsplit || (g == 0 && j == 0))) {
-                if (R < F.c) x = xp[F.first_col + R + (int64_t)q * n];
-                for (int e = e0; e < e1; ++e) x += __ldcg(fv + (int64_t)amap_ent[e] * nrhs + q);
-            }
-            v[j] = x;
+        const int e1 = amap_row[aoff + R + 1];
+        for (int e = amap_row[aoff + R]; e < e1; ++e) {
+            const double* w = fv + (int64_t)amap_ent[e] * nrhs + q;
+            v[0] += __ldcg(w);
+            if (q1) v[1] += __ldcg(w + 1);
         }
     };
     auto issue = [&](int p) {
@@ -334,126 +450,63 @@ __device__ void fwd_tile_task(int2 tk, const FrontDesc* __restrict__ fronts,
             const TileRange ti = tile_range(i, F.m, F.c, T);
             load_block_async(sm.lb(p), L + (int64_t)k * T * F.ldl, F.ldl, ti.start, ti.size,
                              min(T, F.c - k * T));
-            load_slot_async(sm.vb(p, nrhs), pb + (int64_t)k * T * nrhs, nrhs);
+            load_slot_async(sm.vb(p), pb + (int64_t)k * T * nrhs, nrhs);
+        } else if (pivot && p == P) {
+            const int sz = tile_range(i0, F.m, F.c, T).size;
+            load_block_async(sm.lb(p), Dinv + dinv_off[s] + (int64_t)i0 * T * T, T, 0, sz, sz);
         }
         cp_async_commit_group();
     };
-    if (pivot) {
-        const TileRange ti = tile_range(i0, F.m, F.c, T);
-        load_block_async(sm.Dk, Dinv + dinv_off[s] + (int64_t)i0 * T * T, T, 0, ti.size, ti.size);
-    }
-    for (int p = 0; p < sm.stg - 1; ++p) issue(p);
-    TV fcur[NQ], fnext[NQ], acc[NQ];
-    gather_rows(i0, fcur);
-#pragma unroll
-    for (int j = 0; j < NQ; ++j) {
-        fnext[j] = TV(0);
-        acc[j] = TV(0);
-    }
-    if (cnt > 1) gather_rows(i0 + 1, fnext);
+    issue(0);
+    double fcur[2], fnext[2] = {0.0, 0.0}, acc[2][2] = {};
+    gather_row(i0, fcur);
+    if (cnt > 1) gather_row(i0 + 1, fnext);
     bool ok = true;
     for (int p = 0; p < P; ++p) {
-        issue(p + sm.stg - 1);
-        cp_async_wait_stages(sm.stg);
+        issue(p + 1);
+        cp_async_wait_groups<1>();
         __syncthreads();
         const int i = i0 + p / kend, k = p % kend;
-        TV* Yk = sm.vb(p, nrhs);
-        if (!settle_slot(Yk, pb + (int64_t)k * T * nrhs, min(T, F.c - k * T), nrhs, abort_flag,
-                         err)) {
+        if (!settle_slot(sm.vb(p), pb + (int64_t)k * T * nrhs, min(T, F.c - k * T), nrhs,
+                         abort_flag, err)) {
             ok = false;
             break;
         }
-        const TL* B = sm.lb(p);
-        if (lsplit) {
-#pragma unroll
-            for (int l = 0; l < 16; ++l)
-                acc[0] += (TV)B[db + r + (g + 4 * l) * LD] * Yk[g + 4 * l];
-        } else {
-#pragma unroll 4
-            for (int l = 0; l < T; ++l) {
-                const TV lv = (TV)B[db + r + l * LD];
-#pragma unroll
-                for (int j = 0; j < NQ; ++j) {
-                    const int q = g + 4 * j;
-                    if (q < nrhs) acc[j] += lv * Yk[l + T * q];
-                }
-            }
-        }
-        if (!pivot && k == kend - 1) {  // update tile i complete: f_i - acc to the front vector
+        group_product<TL, false>(sm.lb(p), db, sm.vb(p), acc);
+        if (!pivot && k == kend - 1) {  // update tile i complete
             const TileRange ti = tile_range(i, F.m, F.c, T);
-            if (lsplit) {
-                TV v = acc[0] + __shfl_xor_sync(0xffffffffu, acc[0], 8);
-                v += __shfl_xor_sync(0xffffffffu, v, 16);
-                if (g == 0 && r < ti.size) f[ti.start + r] = fcur[0] - v;
-            } else if (r < ti.size) {
-#pragma unroll
-                for (int j = 0; j < NQ; ++j) {
-                    const int q = g + 4 * j;
-                    if (q < nrhs) f[(int64_t)(ti.start + r) * nrhs + q] = fcur[j] - acc[j];
-                }
+            if (r < ti.size) {
+                double* o = f + (int64_t)(ti.start + r) * nrhs + q;
+                if (q0) o[0] = fcur[0] - (acc[0][0] + acc[1][0]);
+                if (q1) o[1] = fcur[1] - (acc[0][1] + acc[1][1]);
             }
 #pragma unroll
-            for (int j = 0; j < NQ; ++j) {
-                acc[j] = TV(0);
+            for (int j = 0; j < 2; ++j) {
+                acc[0][j] = acc[1][j] = 0.0;
                 fcur[j] = fnext[j];
             }
-            if (i + 2 < i0 + cnt) gather_rows(i + 2, fnext);
+            if (i + 2 < i0 + cnt) gather_row(i + 2, fnext);
         }
-        if (p + 1 < P) __syncthreads();  // the stages are reused; after the last, nothing is
+        if (p + 1 < P || pivot) __syncthreads();  // the stages are reused
     }
     cp_async_wait_groups<0>();
     if (!ok || !pivot) return;
-    // pivot tile: F = f_i - acc (zero beyond the tile), then y = Dk F
     const TileRange ti = tile_range(i0, F.m, F.c, T);
-    TV* Y = sm.Y;
-    const TL* Dk = sm.Dk;
-    if (lsplit) {
-        // one right-hand side, one barrier: the row's phases summed by
-        // shuffles, F into sm.Y, then y = Dk F the same way
-        TV a = acc[0] + __shfl_xor_sync(0xffffffffu, acc[0], 8);
-        a += __shfl_xor_sync(0xffffffffu, a, 16);
-        if (g == 0) Y[r] = r < ti.size ? fcur[0] - a : TV(0);
-        __syncthreads();
-        TV y = TV(0);
-#pragma unroll
-        for (int l = 0; l < 16; ++l) y += (TV)Dk[r + (g + 4 * l) * LD] * Y[g + 4 * l];
-        y += __shfl_xor_sync(0xffffffffu, y, 8);
-        y += __shfl_xor_sync(0xffffffffu, y, 16);
-        if (g == 0 && r < ti.size) {
-            xp[F.first_col + ti.start + r] = y;
-            st_relaxed_f64(pb + (int64_t)i0 * T + r, y);
-        }
-        return;
-    }
+    const bool in = r < ti.size;
+    sm.Y[r + q * kVecLD] = in && q0 ? fcur[0] - (acc[0][0] + acc[1][0]) : 0.0;
+    sm.Y[r + (q + 1) * kVecLD] = in && q1 ? fcur[1] - (acc[0][1] + acc[1][1]) : 0.0;
     __syncthreads();
-#pragma unroll
-    for (int j = 0; j < NQ; ++j) {
-        const int q = g + 4 * j;
-        if (q < nrhs) Y[r + T * q] = r < ti.size ? fcur[j] - acc[j] : TV(0);
-    }
-    __syncthreads();
-    {
-        TV y[NQ];
-#pragma unroll
-        for (int j = 0; j < NQ; ++j) y[j] = TV(0);
-#pragma unroll 4
-        for (int l = 0; l < T; ++l) {
-            const TV dv = (TV)Dk[r + l * LD];
-#pragma unroll
-            for (int j = 0; j < NQ; ++j) {
-                const int q = g + 4 * j;
-                if (q < nrhs) y[j] += dv * Y[l + T * q];
-            }
+    double y[2][2] = {};
+    group_product<TL, false>(sm.lb(P), 0, sm.Y, y);
+    if (in) {
+        double* o = pb + (int64_t)i0 * nrhs * T + r;
+        if (q0) {
+            xp[F.first_col + ti.start + r + (int64_t)q * n] = y[0][0] + y[1][0];
+            st_relaxed_f64(o + q * T, y[0][0] + y[1][0]);
         }
-        if (r < ti.size) {
-#pragma unroll
-            for (int j = 0; j < NQ; ++j) {
-                const int q = g + 4 * j;
-                if (q < nrhs) {
-                    xp[F.first_col + ti.start + r + (int64_t)q * n] = y[j];
-                    st_relaxed_f64(pb + ((int64_t)i0 * nrhs + q) * T + r, y[j]);
-                }
-            }
+        if (q1) {
+            xp[F.first_col + ti.start + r + (int64_t)(q + 1) * n] = y[0][1] + y[1][1];
+            st_relaxed_f64(o + (q + 1) * T, y[0][1] + y[1][1]);
         }
     }
 }
@@ -462,30 +515,29 @@ __device__ void fwd_tile_task(int2 tk, const FrontDesc* __restrict__ fronts,
 // L(k, j)' x_k over the update row tiles k of chunk h (kGatherTiles tiles;
 // x final: ancestors, read through the row list) for pivot column tile j,
 // written as a T x nrhs vector for the pivot task to add in chunk order, then
-// counted in.  Threads: l = column in the tile, g = quarter.
-template <typename TL, typename TV, int NQ>
+// counted in.  MULTI: a group of nrhs <= 8 right-hand sides on the matrix
+// instructions; one: warp w takes columns 8w .. 8w + 7, lane (c1 = column,
+// q1 = row phase) the rows q1, q1 + 4, ...: conflict-free reads of the stage
+// layout, the phases summed by shuffles.
+template <typename TL, bool MULTI>
 __device__ void bwd_gather_task(int2 tk, const FrontDesc* __restrict__ fronts,
                                 const int* __restrict__ rows, const int* __restrict__ gather_nch,
                                 const int* __restrict__ gather_off, int* __restrict__ gcount,
                                 const int64_t* __restrict__ dinv_off, const TL* __restrict__ Ls,
-                                const TV* __restrict__ xp, TV* __restrict__ part, int n,
+                                const double* __restrict__ xp, double* __restrict__ part, int n,
                                 int nrhs) {
     constexpr int T = kTile, LD = blk_ld<TL>(), GC = SolveScheduleHost::kGatherTiles;
-    const LevelSmem<TL, TV> sm(nrhs);
-    const int tid = threadIdx.x, l = tid & (T - 1), g = tid >> 6;
+    const LevelSmem<TL, MULTI> sm;
+    const int tid = threadIdx.x;
     const int s = tk.x, j = tk.y & 0xffff, h = tk.y >> 16;
     const FrontDesc F = fronts[s];
     const int nt1 = tiles_l(F.c, T), NT = nt1 + tiles_l(F.m - F.c, T);
     const TileRange tj = tile_range(j, F.m, F.c, T);
-    const bool lsplit = nrhs == 1;
     const TL* Lc = Ls + F.loff + (int64_t)tj.start * F.ldl;
     const int* rw = rows + F.rows_off;
     const int k0 = nt1 + h * GC, P = min(NT, k0 + GC) - k0;
     // update row tiles start at c + 64 u: one row offset for every block
     const int db = blk_off<TL>(F.c);
-    // one right-hand side: warp w takes columns 8w .. 8w + 7, lane (c1 =
-    // column, q1 = row phase) the rows q1, q1 + 4, ...: conflict-free reads
-    // of the 16-byte-column stage layout, the phases summed by shuffles
     const int c1 = 8 * (tid >> 5) + (tid & 7), q1 = (tid >> 3) & 3;
     // the chunk's solution rows (ancestors), then the pipeline
     for (int e = tid; e < P * T; e += blockDim.x) {
@@ -497,14 +549,13 @@ __device__ void bwd_gather_task(int2 tk, const FrontDesc* __restrict__ fronts,
     // two stages: the L blocks by cp.async; the ancestors' solution rows
     // (written in this launch) through L2 into registers one stage ahead,
     // stored into their stage after the previous stage's products
-    static_assert(kTile * kSolvePassRhs % 256 == 0, "whole vector elements per thread");
-    constexpr int VPT = kTile * kSolvePassRhs / 256;
-    TV pend[VPT];
+    constexpr int VPT = MULTI ? kTile * kGroupRhs / 256 : 1;
+    double pend[VPT];
     auto fetch = [&](int p) {
 #pragma unroll
         for (int k = 0; k < VPT; ++k) {
             const int e = tid + 256 * k;
-            pend[k] = TV(0);
+            pend[k] = 0.0;
             if (p < P && e < T * nrhs) {
                 const int row = sm.idx[p * T + (e & (T - 1))], q = e / T;
                 if (row >= 0) pend[k] = __ldcg(xp + row + (int64_t)q * n);
@@ -513,11 +564,11 @@ __device__ void bwd_gather_task(int2 tk, const FrontDesc* __restrict__ fronts,
     };
     auto put = [&](int p) {
         if (p >= P) return;
-        TV* v = sm.vb(p, nrhs);
+        double* v = sm.vb(p);
 #pragma unroll
         for (int k = 0; k < VPT; ++k) {
             const int e = tid + 256 * k;
-            if (e < T * nrhs) v[e] = pend[k];
+            if (e < T * nrhs) v[(e / T) * kVecLD + (e & (T - 1))] = pend[k];
         }
     };
     auto issue = [&](int p) {
@@ -527,50 +578,38 @@ __device__ void bwd_gather_task(int2 tk, const FrontDesc* __restrict__ fronts,
         }
         cp_async_commit_group();
     };
-    static_assert(level_stages<TL>(1) == 2, "the gather's vector pipeline has two stages");
+    static_assert(kSolveStages == 2, "the gather's vector pipeline has two stages");
     issue(0);
     fetch(0);
     put(0);
-    TV acc[NQ];
-#pragma unroll
-    for (int a = 0; a < NQ; ++a) acc[a] = TV(0);
+    double acc[2][2] = {};
     for (int p = 0; p < P; ++p) {
         issue(p + 1);
         fetch(p + 1);
         cp_async_wait_groups<1>();
         __syncthreads();
         const TL* Bk = sm.lb(p);
-        const TV* X = sm.vb(p, nrhs);
-        if (lsplit) {
+        const double* X = sm.vb(p);
+        if constexpr (MULTI) {
+            group_product<TL, true>(Bk, db, X, acc);
+        } else {
 #pragma unroll
             for (int u = 0; u < 16; ++u)
-                acc[0] += (TV)Bk[db + q1 + 4 * u + c1 * LD] * X[q1 + 4 * u];
-        } else {
-#pragma unroll 4
-            for (int r = 0; r < T; ++r) {
-                const TV lv = (TV)Bk[db + r + l * LD];
-#pragma unroll
-                for (int a = 0; a < NQ; ++a) {
-                    const int q = g + 4 * a;
-                    if (q < nrhs) acc[a] += lv * X[r + T * q];
-                }
-            }
+                acc[0][0] += (double)Bk[db + q1 + 4 * u + c1 * LD] * X[q1 + 4 * u];
         }
         __syncthreads();
         put(p + 1);
     }
     cp_async_wait_groups<0>();
-    TV* out = part + ((int64_t)gather_off[s] + (int64_t)j * gather_nch[s] + h) * T * nrhs;
-    if (lsplit) {
-        TV v = acc[0] + __shfl_xor_sync(0xffffffffu, acc[0], 8);
+    double* out = part + ((int64_t)gather_off[s] + (int64_t)j * gather_nch[s] + h) * T * nrhs;
+    if constexpr (MULTI) {
+        const int l = tid >> 2, q = 2 * (tid & 3);
+        if (q < nrhs) out[l + T * q] = acc[0][0] + acc[1][0];
+        if (q + 1 < nrhs) out[l + T * (q + 1)] = acc[0][1] + acc[1][1];
+    } else {
+        double v = acc[0][0] + __shfl_xor_sync(0xffffffffu, acc[0][0], 8);
         v += __shfl_xor_sync(0xffffffffu, v, 16);
         if (q1 == 0) out[c1] = v;
-    } else {
-#pragma unroll
-        for (int a = 0; a < NQ; ++a) {
-            const int q = g + 4 * a;
-            if (q < nrhs) out[l + T * q] = acc[a];
-        }
     }
     // count this chunk in for the pivot task (s, j): the CTA's stores, then
     // a device-scope fence, then the increment
@@ -896,8 +935,8 @@ __device__ void bwd_warp_front(int s, const FrontDeps& deps, const FrontDesc* __
 // per-warp shared buffer of the warp path: MR = rows rounded up to 32, times
 // the right-hand sides of one pass
 __host__ __device__ constexpr int warp_rows(int msmall) { return ((msmall + 31) / 32) * 32; }
-__host__ __device__ constexpr int warp_buf_stride(int msmall, int nrhs) {
-    return warp_rows(msmall) * (nrhs == 1 ? 1 : kWarpSolveRhs);
+__host__ __device__ constexpr int warp_buf_stride(int msmall, bool multi) {
+    return warp_rows(msmall) * (multi ? kWarpSolveRhs : 1);
 }
 
 // Warp tasks of one warp item (its slice of the direction's warp list):
@@ -977,58 +1016,54 @@ __device__ void bwd_warp_task(const WarpTasks& wt, int t, const FrontDeps& deps,
 // the update-row gathers of (s, j) have all counted in, their partial sums
 // in chunk order, then acc += sum_{k > j} L(k, j)' x_k over the pivot tiles
 // nt1-1 .. j+1 of this front as they publish, and solves
-// x_j = inv(L_jj)' (y_j - acc).  Threads: l = column in the tile.
-template <typename TL, typename TV, int NQ>
+// x_j = inv(L_jj)' (y_j - acc).  MULTI as in bwd_gather_task.
+template <typename TL, bool MULTI>
 __device__ void bwd_chain_task(int2 tk, const FrontDesc* __restrict__ fronts,
                                double* __restrict__ pub, int* __restrict__ abort_flag,
                                int* __restrict__ err, const int* __restrict__ gather_nch,
                                const int* __restrict__ gather_off, const int* __restrict__ gcount,
-                               const TV* __restrict__ part, const int64_t* __restrict__ dinv_off,
-                               const TL* __restrict__ Ls, const TL* __restrict__ Dinv,
-                               TV* __restrict__ xp, int n, int nrhs) {
-    static_assert(sizeof(TV) == 8, "solve vectors are double");
+                               const double* __restrict__ part,
+                               const int64_t* __restrict__ dinv_off, const TL* __restrict__ Ls,
+                               const TL* __restrict__ Dinv, double* __restrict__ xp, int n,
+                               int nrhs) {
     constexpr int T = kTile, LD = blk_ld<TL>();
-    const LevelSmem<TL, TV> sm(nrhs);
+    const LevelSmem<TL, MULTI> sm;
     __shared__ int s_ok;
-    const int tid = threadIdx.x, l = tid & (T - 1), g = tid >> 6;
-    // one right-hand side: warp w takes columns 8w .. 8w + 7, lane (c1 =
-    // column, q1 = row phase) the rows q1, q1 + 4, ...: conflict-free reads
-    // of the 16-byte-column stage layout, the phases summed by shuffles
-    const int c1 = 8 * (tid >> 5) + (tid & 7), q1 = (tid >> 3) & 3;
+    const int tid = threadIdx.x;
+    // this thread's column of the tile and right-hand sides: several, two of
+    // column tid / 4; one, phase 0 of column c1
+    const int q1 = (tid >> 3) & 3;
+    const int l = MULTI ? tid >> 2 : 8 * (tid >> 5) + (tid & 7), q = MULTI ? 2 * (tid & 3) : 0;
+    const bool own0 = MULTI ? q < nrhs : q1 == 0, own1 = MULTI && q + 1 < nrhs;
     const int s = tk.x, j = tk.y;
     const FrontDesc F = fronts[s];
     const int nt1 = tiles_l(F.c, T);
     const TileRange tj = tile_range(j, F.m, F.c, T);
-    const bool lsplit = nrhs == 1;
     const TL* Lc = Ls + F.loff + (int64_t)tj.start * F.ldl;  // column tile j
     const int64_t tile0 = dinv_off[s] / (T * T);               // this front's first pivot tile
     double* pb = pub + tile0 * T * nrhs;
     const int P = nt1 - 1 - j;  // pivot row tiles k = nt1-1 down to j+1
+    auto load_inv = [&](TL* dst) {
+        load_block_async(dst, Dinv + dinv_off[s] + (int64_t)j * T * T, T, 0, tj.size, tj.size);
+    };
     auto issue = [&](int p) {
         if (p < P) {
             const TileRange tkr = tile_range(nt1 - 1 - p, F.m, F.c, T);
             load_block_async(sm.lb(p), Lc, F.ldl, tkr.start, tkr.size, tj.size);
-            load_slot_async(sm.vb(p, nrhs), pb + (int64_t)(nt1 - 1 - p) * T * nrhs, nrhs);
+            load_slot_async(sm.vb(p), pb + (int64_t)(nt1 - 1 - p) * T * nrhs, nrhs);
+        } else if (MULTI && p == P) {
+            load_inv(sm.lb(p));
         }
         cp_async_commit_group();
     };
-    load_block_async(sm.Dk, Dinv + dinv_off[s] + (int64_t)j * T * T, T, 0, tj.size, tj.size);
-    for (int p = 0; p < sm.stg - 1; ++p) issue(p);
-    TV acc[NQ];
-#pragma unroll
-    for (int a = 0; a < NQ; ++a) acc[a] = TV(0);
+    if (!MULTI) load_inv(sm.Dk);
+    issue(0);
+    double acc[2][2] = {};
     // this tile's y_j, before the first wait
-    const int64_t xj = F.first_col + tj.start;
-    TV ypre[NQ];
-#pragma unroll
-    for (int a = 0; a < NQ; ++a) {
-        if (lsplit)
-            ypre[a] = (a == 0 && q1 == 0 && c1 < tj.size) ? __ldcg(xp + xj + c1) : TV(0);
-        else
-            ypre[a] = (l < tj.size && g + 4 * a < nrhs)
-                          ? __ldcg(xp + xj + l + (int64_t)(g + 4 * a) * n)
-                          : TV(0);
-    }
+    const int64_t xj = F.first_col + tj.start + l;
+    const bool in = l < tj.size;
+    const double y0 = in && own0 ? __ldcg(xp + xj + (int64_t)q * n) : 0.0;
+    const double y1 = in && own1 ? __ldcg(xp + xj + (int64_t)(q + 1) * n) : 0.0;
     // the update-row partial sums of (s, j) (gathers hold lower tickets), in
     // chunk order, before the chain's first wait
     {
@@ -1040,101 +1075,69 @@ __device__ void bwd_chain_task(int2 tk, const FrontDesc* __restrict__ fronts,
                 cp_async_wait_groups<0>();
                 return;
             }
-            const TV* pj = part + ((int64_t)gather_off[s] + (int64_t)j * nch) * T * nrhs;
+            const double* pj = part + ((int64_t)gather_off[s] + (int64_t)j * nch) * T * nrhs;
             for (int h = 0; h < nch; ++h, pj += (int64_t)T * nrhs) {
-                if (lsplit) {
-                    if (q1 == 0) acc[0] += __ldcg(pj + c1);
-                } else {
-#pragma unroll
-                    for (int a = 0; a < NQ; ++a) {
-                        const int q = g + 4 * a;
-                        if (q < nrhs) acc[a] += __ldcg(pj + l + T * q);
-                    }
-                }
+                if (own0) acc[0][0] += __ldcg(pj + l + T * q);
+                if (own1) acc[0][1] += __ldcg(pj + l + T * (q + 1));
             }
         }
     }
     bool ok = true;
     for (int p = 0; p < P; ++p) {
-        issue(p + sm.stg - 1);
-        cp_async_wait_stages(sm.stg);
+        issue(p + 1);
+        cp_async_wait_groups<1>();
         __syncthreads();
         const int k = nt1 - 1 - p;
-        TV* X = sm.vb(p, nrhs);
+        double* X = sm.vb(p);
         if (!settle_slot(X, pb + (int64_t)k * T * nrhs, tile_range(k, F.m, F.c, T).size, nrhs,
                          abort_flag, err)) {
             ok = false;
             break;
         }
         const TL* B = sm.lb(p);
-        if (lsplit) {
-#pragma unroll
-            for (int u = 0; u < 16; ++u) acc[0] += (TV)B[q1 + 4 * u + c1 * LD] * X[q1 + 4 * u];
+        if constexpr (MULTI) {
+            group_product<TL, true>(B, 0, X, acc);
         } else {
-#pragma unroll 4
-            for (int r = 0; r < T; ++r) {
-                const TV lv = (TV)B[r + l * LD];
 #pragma unroll
-                for (int a = 0; a < NQ; ++a) {
-                    const int q = g + 4 * a;
-                    if (q < nrhs) acc[a] += lv * X[r + T * q];
-                }
-            }
+            for (int u = 0; u < 16; ++u)
+                acc[0][0] += (double)B[q1 + 4 * u + l * LD] * X[q1 + 4 * u];
         }
-        if (p + 1 < P) __syncthreads();  // the stages are reused; after the last, nothing is
+        if (p + 1 < P || MULTI) __syncthreads();  // the stages are reused
     }
     cp_async_wait_groups<0>();
     if (!ok) return;
-    TV* X = sm.Y;
-    const TL* Dk = sm.Dk;
+    double* X = sm.Y;
     // t = y_j - acc (y_j: this front's forward solution), then x_j = Dk' t
-    if (lsplit) {
+    if constexpr (MULTI) {
+        X[l + q * kVecLD] = in && own0 ? y0 - (acc[0][0] + acc[1][0]) : 0.0;
+        X[l + (q + 1) * kVecLD] = in && own1 ? y1 - (acc[0][1] + acc[1][1]) : 0.0;
+        __syncthreads();
+        double x[2][2] = {};
+        group_product<TL, true>(sm.lb(P), 0, X, x);
+        if (in && own0) {
+            xp[xj + (int64_t)q * n] = x[0][0] + x[1][0];
+            st_relaxed_f64(pb + ((int64_t)j * nrhs + q) * T + l, x[0][0] + x[1][0]);
+        }
+        if (in && own1) {
+            xp[xj + (int64_t)(q + 1) * n] = x[0][1] + x[1][1];
+            st_relaxed_f64(pb + ((int64_t)j * nrhs + q + 1) * T + l, x[0][1] + x[1][1]);
+        }
+    } else {
         // one right-hand side, one barrier: the row phases' sums by
         // shuffles, t into sm.Y, then x_j = Dk' t the same way
-        TV a = acc[0] + __shfl_xor_sync(0xffffffffu, acc[0], 8);
+        const TL* Dk = sm.Dk;
+        double a = acc[0][0] + __shfl_xor_sync(0xffffffffu, acc[0][0], 8);
         a += __shfl_xor_sync(0xffffffffu, a, 16);
-        if (q1 == 0) X[c1] = c1 < tj.size ? ypre[0] - a : TV(0);
+        if (q1 == 0) X[l] = in ? y0 - a : 0.0;
         __syncthreads();
-        TV x = TV(0);
+        double x = 0.0;
 #pragma unroll
-        for (int u = 0; u < 16; ++u) x += (TV)Dk[q1 + 4 * u + c1 * LD] * X[q1 + 4 * u];
+        for (int u = 0; u < 16; ++u) x += (double)Dk[q1 + 4 * u + l * LD] * X[q1 + 4 * u];
         x += __shfl_xor_sync(0xffffffffu, x, 8);
         x += __shfl_xor_sync(0xffffffffu, x, 16);
-        if (q1 == 0 && c1 < tj.size) {
-            xp[xj + c1] = x;
-            st_relaxed_f64(pb + (int64_t)j * T + c1, x);
-        }
-        return;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int a = 0; a < NQ; ++a) {
-        const int q = g + 4 * a;
-        if (q < nrhs) X[l + T * q] = l < tj.size ? ypre[a] - acc[a] : TV(0);
-    }
-    __syncthreads();
-    {
-        TV x[NQ];
-#pragma unroll
-        for (int a = 0; a < NQ; ++a) x[a] = TV(0);
-#pragma unroll 4
-        for (int r = 0; r < T; ++r) {
-            const TV dv = (TV)Dk[r + l * LD];
-#pragma unroll
-            for (int a = 0; a < NQ; ++a) {
-                const int q = g + 4 * a;
-                if (q < nrhs) x[a] += dv * X[r + T * q];
-            }
-        }
-        if (l < tj.size) {
-#pragma unroll
-            for (int a = 0; a < NQ; ++a) {
-                const int q = g + 4 * a;
-                if (q < nrhs) {
-                    xp[xj + l + (int64_t)q * n] = x[a];
-                    st_relaxed_f64(pb + ((int64_t)j * nrhs + q) * T + l, x[a]);
-                }
-            }
+        if (q1 == 0 && in) {
+            xp[xj] = x;
+            st_relaxed_f64(pb + (int64_t)j * T + l, x);
         }
     }
 }
@@ -1247,40 +1250,61 @@ __device__ __forceinline__ bool cta_wait(const int* word, int target, int* abort
     return s_wok != 0;
 }
 
-template <typename TL, typename TV, int NQ>
-__global__ void __launch_bounds__(256, NQ == 1 ? 4 : 2)
+// A group's own words in the sync array (its front counts and gather counts)
+// and its slices of the work vectors.
+struct SolveGroups {
+    int n, nrhs;        // unknowns, right-hand sides of the launch
+    int stride;         // sync words of a group
+    int64_t fv_total;   // work vector rows
+    __device__ int count() const { return (nrhs + kGroupRhs - 1) / kGroupRhs; }
+    __device__ int size(int g) const { return min(kGroupRhs, nrhs - kGroupRhs * g); }
+    __device__ int64_t xp_off(int g) const { return (int64_t)kGroupRhs * g * n; }
+    __device__ int64_t fv_off(int g) const { return kGroupRhs * fv_total * g; }
+};
+
+// residency by shared memory: one right-hand side keeps three blocks of L per
+// CTA (FP32 52 KB, FP64 104 KB), a group two and its vectors (49 and 83 KB)
+template <typename TL, bool MULTI>
+constexpr int solve_ctas_per_sm() {
+    return sizeof(TL) == 8 ? 2 : MULTI ? 3 : 4;
+}
+
+template <typename TL, bool MULTI>
+__global__ void __launch_bounds__(256, solve_ctas_per_sm<TL, MULTI>())
     k_fwd_solve(const FrontDesc* __restrict__ fronts, const int4* __restrict__ items, int nitems,
-                int* __restrict__ counter, double* __restrict__ pub, int* __restrict__ abort_flag,
-                int* __restrict__ err, int* __restrict__ fdone, int* __restrict__ udone,
+                int* __restrict__ counter, int64_t pub_rows, int* __restrict__ abort_flag,
+                int* __restrict__ err, int* __restrict__ fdone0, int* __restrict__ udone0,
                 const int64_t* __restrict__ fv_off, const int* __restrict__ amap_off,
                 const int* __restrict__ amap_row, const int* __restrict__ amap_ent,
                 const int64_t* __restrict__ dinv_off, const int* __restrict__ wlist,
                 const int* __restrict__ child,
                 const int* __restrict__ relmap, const TL* __restrict__ Ls,
-                const TL* __restrict__ Dinv, TV* __restrict__ xp, TV* __restrict__ fv, int n,
-                int nrhs, int MR) {
+                const TL* __restrict__ Dinv, double* __restrict__ xp0, double* __restrict__ fv0,
+                SolveGroups grp, int MR) {
     constexpr int T = kTile;
     __shared__ int s_item;
-    const FrontDeps deps{fdone, nullptr, abort_flag, err};
+    const int ngroups = MULTI ? grp.count() : 1, n = grp.n;
     for (;;) {
         if (threadIdx.x == 0) s_item = atomicAdd(counter, 1);
         __syncthreads();
         const int k = s_item;
-        if (k >= nitems) return;
-        const int4 it = items[k];
+        if (k >= nitems * ngroups) return;
+        const int4 it = items[MULTI ? k / ngroups : k];
+        const int gi = MULTI ? k % ngroups : 0, nrhs = MULTI ? grp.size(gi) : 1;
+        double* xp = xp0 + grp.xp_off(gi);
+        double* fv = fv0 + grp.fv_off(gi);
+        double* pub = fv + pub_rows * nrhs;
+        int* fdone = fdone0 + gi * grp.stride;
+        int* udone = udone0 + gi * grp.stride;
+        const FrontDeps deps{fdone, nullptr, abort_flag, err};
         if (it.x == SolveScheduleHost::kItemWarps) {
             extern __shared__ __align__(16) unsigned char smem_raw[];
             const WarpTasks wt{wlist + it.y, it.z & 0xff, (it.z >> 8) & 0xff, it.z >> 16};
             const int w = threadIdx.x >> 5, t = w;
-            TV* wbuf = reinterpret_cast<TV*>(smem_raw) + w * warp_buf_stride(MR, nrhs);
-            if (t < wt.count()) {
-                if (nrhs == 1)
-                    fwd_warp_task<TL, TV, 1>(wt, t, deps, fronts, child, relmap, fv_off, Ls, xp,
-                                             fv, n, nrhs, wbuf, MR);
-                else
-                    fwd_warp_task<TL, TV, kWarpSolveRhs>(wt, t, deps, fronts, child, relmap,
-                                                         fv_off, Ls, xp, fv, n, nrhs, wbuf, MR);
-            }
+            double* wbuf = reinterpret_cast<double*>(smem_raw) + w * warp_buf_stride(MR, MULTI);
+            if (t < wt.count())
+                fwd_warp_task<TL, double, MULTI ? kWarpSolveRhs : 1>(
+                    wt, t, deps, fronts, child, relmap, fv_off, Ls, xp, fv, n, nrhs, wbuf, MR);
         } else {
             // a tile task of a large front: its children first
             const int2 tk = make_int2(it.y, it.z);
@@ -1288,26 +1312,24 @@ __global__ void __launch_bounds__(256, NQ == 1 ? 4 : 2)
             const FrontDesc F = fronts[s];
             const int nt1 = tiles_l(F.c, T);
             if (cta_wait(fdone + s, F.child_end - F.child_beg, abort_flag, err)) {
-                bool done = false;
-                if constexpr (NQ == 1) {
+                if constexpr (MULTI) {
+                    fwd_tile_group<TL>(tk, fronts, pub, abort_flag, err, fv_off, amap_off,
+                                       amap_row, amap_ent, dinv_off, Ls, Dinv, xp, fv, n, nrhs);
+                } else if (i0 >= nt1 && nt1 <= kRt1MaxPivotTiles) {
                     // update tiles of fronts with at most kRt1MaxPivotTiles
                     // pivot tiles, one right-hand side: registers straight
                     // from L (measured faster there; the staged pipeline
                     // streams long column ranges better)
-                    if (nrhs == 1 && i0 >= nt1 && nt1 <= kRt1MaxPivotTiles) {
-                        double* pb = pub + (dinv_off[s] / (T * T)) * T;
-                        const TileRange a = tile_range(i0, F.m, F.c, T);
-                        const TileRange b = tile_range(i0 + cnt - 1, F.m, F.c, T);
-                        fwd_update_rt1<TL>(s, a.start, b.start + b.size, F, pb, abort_flag, err,
-                                           amap_off, amap_row, amap_ent, Ls, xp,
-                                           front_vec(fv, fv_off, s, 1), fv);
-                        done = true;
-                    }
+                    double* pb = pub + (dinv_off[s] / (T * T)) * T;
+                    const TileRange a = tile_range(i0, F.m, F.c, T);
+                    const TileRange b = tile_range(i0 + cnt - 1, F.m, F.c, T);
+                    fwd_update_rt1<TL>(s, a.start, b.start + b.size, F, pb, abort_flag, err,
+                                       amap_off, amap_row, amap_ent, Ls, xp,
+                                       front_vec(fv, fv_off, s, 1), fv);
+                } else {
+                    fwd_tile_task<TL>(tk, fronts, pub, abort_flag, err, fv_off, amap_off,
+                                      amap_row, amap_ent, dinv_off, Ls, Dinv, xp, fv);
                 }
-                if (!done)
-                    fwd_tile_task<TL, TV, NQ>(tk, fronts, pub, abort_flag, err, fv_off, amap_off,
-                                              amap_row, amap_ent, dinv_off, Ls, Dinv, xp, fv, n,
-                                              nrhs);
                 // update tiles counted in; the front's last one counts the
                 // front in at its parent
                 if (i0 >= nt1) {
@@ -1327,49 +1349,53 @@ __global__ void __launch_bounds__(256, NQ == 1 ? 4 : 2)
     }
 }
 
-template <typename TL, typename TV, int NQ>
-__global__ void __launch_bounds__(256, NQ == 1 ? 4 : 2)
+template <typename TL, bool MULTI>
+__global__ void __launch_bounds__(256, solve_ctas_per_sm<TL, MULTI>())
     k_bwd_solve(const FrontDesc* __restrict__ fronts, const int4* __restrict__ items, int nitems,
-                int* __restrict__ counter, double* __restrict__ pub, int* __restrict__ abort_flag,
-                int* __restrict__ err, int* __restrict__ bdone, const int* __restrict__ btarget,
-                const int* __restrict__ gather_nch, const int* __restrict__ gather_off,
-                int* __restrict__ gcount, TV* __restrict__ part,
+                int* __restrict__ counter, int64_t pub_rows, int64_t part_rows,
+                int* __restrict__ abort_flag, int* __restrict__ err, int* __restrict__ bdone0,
+                const int* __restrict__ btarget, const int* __restrict__ gather_nch,
+                const int* __restrict__ gather_off, int* __restrict__ gcount0,
                 const int64_t* __restrict__ dinv_off, const int* __restrict__ wlist,
-                const int* __restrict__ rows,
-                const TL* __restrict__ Ls, const TL* __restrict__ Dinv, TV* __restrict__ xp,
-                int n, int nrhs, int MR) {
+                const int* __restrict__ rows, const TL* __restrict__ Ls,
+                const TL* __restrict__ Dinv, double* __restrict__ xp0, double* __restrict__ fv0,
+                SolveGroups grp, int MR) {
     __shared__ int s_item;
-    const FrontDeps deps{bdone, btarget, abort_flag, err};
+    const int ngroups = MULTI ? grp.count() : 1, n = grp.n;
     for (;;) {
         if (threadIdx.x == 0) s_item = atomicAdd(counter, 1);
         __syncthreads();
         const int k = s_item;
-        if (k >= nitems) return;
-        const int4 it = items[k];
+        if (k >= nitems * ngroups) return;
+        const int4 it = items[MULTI ? k / ngroups : k];
+        const int gi = MULTI ? k % ngroups : 0, nrhs = MULTI ? grp.size(gi) : 1;
+        double* xp = xp0 + grp.xp_off(gi);
+        double* fv = fv0 + grp.fv_off(gi);
+        double* pub = fv + pub_rows * nrhs;
+        double* part = fv + part_rows * nrhs;
+        int* bdone = bdone0 + gi * grp.stride;
+        int* gcount = gcount0 + gi * grp.stride;
+        const FrontDeps deps{bdone, btarget, abort_flag, err};
         if (it.x == SolveScheduleHost::kItemWarps) {
             extern __shared__ __align__(16) unsigned char smem_raw[];
             const WarpTasks wt{wlist + it.y, it.z & 0xff, (it.z >> 8) & 0xff, it.z >> 16};
             const int w = threadIdx.x >> 5, t = w;
-            TV* wbuf = reinterpret_cast<TV*>(smem_raw) + w * warp_buf_stride(MR, nrhs);
-            if (t < wt.count()) {
-                if (nrhs == 1)
-                    bwd_warp_task<TL, TV, 1>(wt, t, deps, fronts, rows, Ls, xp, n, nrhs, wbuf, MR);
-                else
-                    bwd_warp_task<TL, TV, kWarpSolveRhs>(wt, t, deps, fronts, rows, Ls, xp, n,
-                                                         nrhs, wbuf, MR);
-            }
+            double* wbuf = reinterpret_cast<double*>(smem_raw) + w * warp_buf_stride(MR, MULTI);
+            if (t < wt.count())
+                bwd_warp_task<TL, double, MULTI ? kWarpSolveRhs : 1>(wt, t, deps, fronts, rows, Ls,
+                                                                     xp, n, nrhs, wbuf, MR);
         } else if (it.x == SolveScheduleHost::kItemGather) {
             // the update rows' partial sums need the ancestors' solution
             const int2 tk = make_int2(it.y, it.z);
             const int p = fronts[tk.x].parent;
             if (p < 0 || cta_wait(bdone + p, btarget[p], abort_flag, err))
-                bwd_gather_task<TL, TV, NQ>(tk, fronts, rows, gather_nch, gather_off, gcount,
-                                            dinv_off, Ls, xp, part, n, nrhs);
+                bwd_gather_task<TL, MULTI>(tk, fronts, rows, gather_nch, gather_off, gcount,
+                                           dinv_off, Ls, xp, part, n, nrhs);
         } else {
             // a pivot tile: its gathers (counted) waited for the ancestors
             const int2 tk = make_int2(it.y, it.z);
-            bwd_chain_task<TL, TV, NQ>(tk, fronts, pub, abort_flag, err, gather_nch, gather_off,
-                                       gcount, part, dinv_off, Ls, Dinv, xp, n, nrhs);
+            bwd_chain_task<TL, MULTI>(tk, fronts, pub, abort_flag, err, gather_nch, gather_off,
+                                      gcount, part, dinv_off, Ls, Dinv, xp, n, nrhs);
             __syncthreads();
             if (threadIdx.x == 0) {
                 __threadfence();
@@ -1377,6 +1403,23 @@ __global__ void __launch_bounds__(256, NQ == 1 ? 4 : 2)
             }
         }
         __syncthreads();  // shared memory and s_item free for the next item
+    }
+}
+
+// Before the sweeps: the sync words cleared, every group's publication slots
+// set to the unpublished pattern.
+__global__ void __launch_bounds__(256)
+    k_solve_init(int4* __restrict__ sync, int64_t nsync4, double* __restrict__ fv0,
+                 int64_t pub_rows, int64_t slot_rows, SolveGroups grp) {
+    const int64_t tid = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    const int64_t nt = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t i = tid; i < nsync4; i += nt) sync[i] = make_int4(0, 0, 0, 0);
+    for (int g = 0; g < grp.count(); ++g) {
+        // slots start on 16 bytes and hold 64 rows each
+        double2* p = reinterpret_cast<double2*>(fv0 + grp.fv_off(g) + pub_rows * grp.size(g));
+        const int64_t cnt = slot_rows * grp.size(g) / 2;
+        const double v = __longlong_as_double(-1ll);
+        for (int64_t i = tid; i < cnt; i += nt) p[i] = make_double2(v, v);
     }
 }
 
@@ -1427,53 +1470,60 @@ constexpr int kWarpBufRows = ((Plan::kSmallMaxRows + 31) / 32) * 32;
 
 // dynamic shared memory of a solve launch: the tile tasks' stages or the
 // eight warps' buffers, whichever is larger
-template <typename TL, typename TV>
-static size_t solve_smem(int nrhs) {
-    size_t m = level_smem_bytes<TL, TV>(nrhs);
-    if (nrhs == 1) m = std::max(m, rt1_smem_bytes<TL>());
-    return std::max(m, 8 * (size_t)warp_buf_stride(kWarpBufRows, nrhs) * sizeof(TV));
+template <typename TL, bool MULTI>
+static size_t solve_smem() {
+    size_t m = level_smem_bytes<TL, MULTI>();
+    if (!MULTI) m = std::max(m, rt1_smem_bytes<TL>());
+    return std::max(m, 8 * (size_t)warp_buf_stride(kWarpBufRows, MULTI) * sizeof(double));
 }
 
-template <typename TL, typename TV, int NQ>
-static void set_solve_attributes_nq() {
-    const int sm = (int)solve_smem<TL, TV>(kSolvePassRhs);
-    cudaFuncSetAttribute(k_fwd_solve<TL, TV, NQ>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
-    cudaFuncSetAttribute(k_bwd_solve<TL, TV, NQ>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
-}
-
-template <typename TL, typename TV>
+template <typename TL, bool MULTI>
 static void set_solve_attributes() {
-    set_solve_attributes_nq<TL, TV, 1>();
-    set_solve_attributes_nq<TL, TV, 4>();
-    set_solve_attributes_nq<TL, TV, 8>();
+    const int sm = (int)solve_smem<TL, MULTI>();
+    cudaFuncSetAttribute(k_fwd_solve<TL, MULTI>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
+    cudaFuncSetAttribute(k_bwd_solve<TL, MULTI>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
 }
 
 void init_solve_kernels() {
-    set_solve_attributes<double, double>();
-    set_solve_attributes<float, double>();
+    set_solve_attributes<double, false>();
+    set_solve_attributes<float, false>();
+    set_solve_attributes<double, true>();
+    set_solve_attributes<float, true>();
 }
 
-template <typename TL, typename TV, int NQ>
-static void solve_levels_nq(const DevPlan& D, const TL* Ls, const TL* Dinv, TV* xp, TV* fv,
-                            int nrhs, cudaStream_t st) {
+int solve_groups(int nrhs) { return nrhs == 1 ? 1 : (nrhs + kGroupRhs - 1) / kGroupRhs; }
+int64_t solve_sync_words(int nflags, int nfronts, int groups) {
+    return (4 + (int64_t)groups * (nflags + 3 * (int64_t)nfronts) + 3) & ~(int64_t)3;
+}
+
+template <typename TL, bool MULTI>
+static void solve_launch(const DevPlan& D, const TL* Ls, const TL* Dinv, double* xp, double* fv,
+                         int nrhs, cudaStream_t st) {
     const SolveSchedule& S = D.solve;
     static_assert(Plan::kSmallMaxRows <= 32 * 5, "the warp path holds 160 rows in shared memory");
-    // sync: the two ticket counters, the gathers' counts per pivot tile, the
-    // abort word, then per front the forward finished-children and
-    // finished-update-tile counts and the backward completions
+    // sync: the two ticket counters and the abort word, then per group the
+    // gathers' counts per pivot tile, and per front the forward
+    // finished-children and finished-update-tile counts and the backward
+    // completions
     int* counters = S.sync;
-    int* gcount = S.sync + 2;
-    int* abort_flag = gcount + S.nflags;
-    int* fdone = abort_flag + 1;
+    int* abort_flag = S.sync + 2;
+    int* gcount = S.sync + 4;
+    int* fdone = gcount + S.nflags;
     int* udone = fdone + S.nfronts;
     int* bdone = udone + S.nfronts;
-    cudaMemsetAsync(S.sync, 0, (size_t)S.nsync * sizeof(int), st);
-    // publication slots of the forward and backward pivot tiles: all-ones bits
-    cudaMemsetAsync(fv + D.fv_pub_off * nrhs, 0xff,
-                    (size_t)2 * S.nflags * kTile * nrhs * sizeof(TV), st);
-    const size_t sm = solve_smem<TL, TV>(nrhs);
+    const SolveGroups grp{D.n, nrhs, S.nflags + 3 * S.nfronts, D.fv_total};
+    const int64_t slots = (int64_t)S.nflags * kTile;  // rows of one direction
+    const int64_t nsync = solve_sync_words(S.nflags, S.nfronts, solve_groups(nrhs));
     const int sms = D.num_sms > 0 ? D.num_sms : 148;
-    const int grid = sms * (NQ == 1 ? 4 : 2);  // the launch bounds' residency
+    {
+        const int64_t work = std::max(nsync / 4, slots * nrhs);
+        const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>((work + 1023) / 1024, sms * 8));
+        k_solve_init<<<blocks, 256, 0, st>>>(reinterpret_cast<int4*>(S.sync), nsync / 4, fv,
+                                             D.fv_pub_off, 2 * slots, grp);
+    }
+    const size_t sm = solve_smem<TL, MULTI>();
+    const int grid = sms * solve_ctas_per_sm<TL, MULTI>();
+    const int ng = MULTI ? solve_groups(nrhs) : 1;
     double fbytes = 0, bbytes = 0;
     for (int l = 0; l < D.nlevels; ++l) {
         fbytes += (S.small_elems[l] + S.fwd_elems[l]) * sizeof(TL);
@@ -1481,37 +1531,33 @@ static void solve_levels_nq(const DevPlan& D, const TL* Ls, const TL* Dinv, TV* 
     }
     if (S.nfwd_items > 0) {
         ProfScope ps(D.prof, KC_SOLVE_LARGE, st, 0, fbytes);
-        k_fwd_solve<TL, TV, NQ><<<std::min(grid, S.nfwd_items), 256, sm, st>>>(
-            D.fronts, S.fwd_items, S.nfwd_items, counters, fv + D.fv_pub_off * nrhs, abort_flag,
+        k_fwd_solve<TL, MULTI><<<std::min(grid, S.nfwd_items * ng), 256, sm, st>>>(
+            D.fronts, S.fwd_items, S.nfwd_items, counters, D.fv_pub_off, abort_flag,
             S.err, fdone, udone, D.fv_off, S.amap_off, S.amap_row, S.amap_ent, D.dinv_off,
-            S.fwd_wlist, D.child, D.relmap, Ls, Dinv, xp, fv, D.n, nrhs,
-            kWarpBufRows);
+            S.fwd_wlist, D.child, D.relmap, Ls, Dinv, xp, fv, grp, kWarpBufRows);
     }
     if (S.nbwd_items > 0) {
         ProfScope ps(D.prof, KC_SOLVE_LARGE, st, 0, bbytes);
-        k_bwd_solve<TL, TV, NQ><<<std::min(grid, S.nbwd_items), 256, sm, st>>>(
-            D.fronts, S.bwd_items, S.nbwd_items, counters + 1,
-            fv + (D.fv_pub_off + (int64_t)S.nflags * kTile) * nrhs, abort_flag, S.err, bdone,
-            S.bwd_target, S.gather_nch, S.gather_off, gcount, fv + D.fv_fronts * nrhs,
-            D.dinv_off, S.bwd_wlist, D.rows, Ls, Dinv, xp, D.n, nrhs,
-            kWarpBufRows);
+        k_bwd_solve<TL, MULTI><<<std::min(grid, S.nbwd_items * ng), 256, sm, st>>>(
+            D.fronts, S.bwd_items, S.nbwd_items, counters + 1, D.fv_pub_off + slots, D.fv_fronts,
+            abort_flag, S.err, bdone, S.bwd_target, S.gather_nch, S.gather_off, gcount,
+            D.dinv_off, S.bwd_wlist, D.rows, Ls, Dinv, xp, fv, grp, kWarpBufRows);
     }
 }
 
 template <typename TL, typename TV>
 void solve_levels(const DevPlan& D, const TL* Ls, const TL* Dinv, TV* xp, TV* fv, int nrhs,
                   cudaStream_t st) {
-    // passes of at most kSolvePassRhs right-hand sides (xp columns q0 ..;
-    // the work vectors, sized for more, are reused with the pass's count)
-    for (int q0 = 0; q0 < nrhs; q0 += kSolvePassRhs) {
-        const int nq = std::min(kSolvePassRhs, nrhs - q0);
-        TV* x = xp + (int64_t)q0 * D.n;
-        if (nq <= 4)
-            solve_levels_nq<TL, TV, 1>(D, Ls, Dinv, x, fv, nq, st);
-        else if (nq <= 16)
-            solve_levels_nq<TL, TV, 4>(D, Ls, Dinv, x, fv, nq, st);
+    // as many groups of right-hand sides per launch as the sync words hold
+    // (the work vectors are reused by the next launch)
+    const int pass = kGroupRhs * D.solve.sync_groups;
+    for (int q0 = 0; q0 < nrhs; q0 += pass) {
+        const int nq = std::min(pass, nrhs - q0);
+        double* x = xp + (int64_t)q0 * D.n;
+        if (nq == 1)
+            solve_launch<TL, false>(D, Ls, Dinv, x, fv, nq, st);
         else
-            solve_levels_nq<TL, TV, 8>(D, Ls, Dinv, x, fv, nq, st);
+            solve_launch<TL, true>(D, Ls, Dinv, x, fv, nq, st);
     }
 }
 

@@ -73,3 +73,25 @@ def test_fp32_factor(c1, c2, u):
     x, berr, _ = S.refine(b)
     r = b - A @ x
     assert np.abs(r).max() <= 1e-14 * (np.abs(A).sum(1).max() * np.abs(x).max() + np.abs(b).max())
+
+
+@pytest.mark.parametrize("c1,c2,u", SIZES)
+@pytest.mark.parametrize("precision", [M.FP64, M.FP32])
+def test_solve_groups(c1, c2, u, precision):
+    """Right-hand sides around the groups of eight of the solve; a column's
+    values do not depend on the columns beside it (each group, and each column
+    of a group, is a sum of its own in a fixed order)."""
+    n, A, Ap, Ai, Ax = _two_leaves(c1, c2, u)
+    S = M.Solver(n, Ap, Ai, ordering=M.ORDER_NATURAL)
+    S.factor(torch.from_numpy(Ax).cuda(), precision)
+    B = np.random.default_rng(2).uniform(-1.0, 1.0, (n, 65))
+    tol = 1e-14 if precision == M.FP64 else 2e-5  # as the factors' bounds above
+    scale = np.abs(A).sum(1).max()
+    full = None
+    for k in (65, 2, 7, 8, 9, 17, 64):
+        X = S.solve(B[:, :k])
+        r = np.abs(B[:, :k] - A @ X).max(0)
+        assert (r <= tol * (scale * np.abs(X).max(0) + np.abs(B[:, :k]).max(0))).all()
+        full = X if full is None else full
+        same = k if k % 8 != 1 else k - 1  # a lone last column of a pass takes the one-column sweep
+        assert np.array_equal(X[:, :min(same, 64)], full[:, :min(same, 64)])
