@@ -132,6 +132,7 @@ struct mdgpu_handle_s {
     double *d_Fb = nullptr, *d_Fu = nullptr, *d_W = nullptr, *d_Lbar = nullptr,
            *d_Abar = nullptr;
     double* d_Y = nullptr;         // its Y scratch
+    double* d_selpart = nullptr;   // its partial sums
     double* d_logdet = nullptr;    // logdet partial sums, then the result
     double* d_gx = nullptr;        // gradient: x and G on the device (host entry)
     double* d_gG = nullptr;
@@ -162,7 +163,7 @@ struct mdgpu_handle_s {
         for (void* p : {(void*)d_Fb, (void*)d_Fu, (void*)d_W, (void*)d_Lbar, (void*)d_Abar})
             if (p) cudaFree(p);
         for (void* p : {(void*)dZ64, (void*)dZu64, (void*)d_Y, (void*)d_logdet, (void*)d_gx, (void*)d_gG,
-                        (void*)d_gm, (void*)d_ssync})
+                        (void*)d_gm, (void*)d_ssync, (void*)d_selpart})
             if (p) cudaFree(p);
         for (void* p : {(void*)d_Ax, (void*)dL64, (void*)dU64, (void*)dL32, (void*)dU32,
                         (void*)dD64, (void*)dD32,
@@ -343,8 +344,8 @@ void upload_plan(mdgpu_handle_s* h, bool check = false) {
         for (int s = 0; s < P.nsuper; ++s) ll[nxt[lv[s]]++] = s;
         D.level_list = h->keep(upload(ll));
         // Y scratch: m x 16 for a small front (one CTA), 2 m x 64 for a
-        // large one (Y and a row-major copy of Z_RK); a level's fronts side
-        // by side, levels reuse it
+        // large one (Y of the even and the odd block steps); a level's
+        // fronts side by side, levels reuse it
         std::vector<char> large(P.nsuper, 0);
         for (int s : P.large_list) large[s] = 1;
         std::vector<int64_t> yo(P.nsuper, 0);
@@ -1635,8 +1636,9 @@ int mdgpu_selinv(mdgpu_handle h, void* stream) {
         if (!h->dZ64) h->dZ64 = dalloc<double>(h->plan.lstore);
         if (!h->dZu64) h->dZu64 = dalloc<double>(h->plan.zustore);
         if (!h->d_Y) h->d_Y = dalloc<double>(std::max<int64_t>(h->D.yscr_total, 1));
+        if (!h->d_selpart) h->d_selpart = dalloc<double>(selinv_partials(h->D));
         NvtxRange nvtx("mdgpu_selinv");
-        launch_selinv(h->D, h->dL64, h->dD64, h->dZ64, h->dZu64, h->d_Y, st);
+        launch_selinv(h->D, h->dL64, h->dD64, h->dZ64, h->dZu64, h->d_Y, h->d_selpart, st);
         ck(cudaGetLastError(), "selected inverse launch");
         ck(cudaStreamSynchronize(st), "selected inverse");
         h->selinv_done = true;

@@ -305,7 +305,8 @@ void permute_scatter(const int* perm, const double* xp, double* x, int n, int nr
 
 // selected inverse and adjoint (selinv.cu)
 void launch_selinv(const DevPlan& D, const double* Ls, const double* Dinv, double* Zs,
-                   double* Zu, double* Yscr, cudaStream_t st);
+                   double* Zu, double* Yscr, double* part, cudaStream_t st);
+int64_t selinv_partials(const DevPlan& D);  // doubles of part
 void launch_grad_lower(const DevPlan& D, int nnz, const int* perm, const double* Zs,
                        const double* x, double* G, cudaStream_t st);
 template <typename T>

@@ -23,10 +23,12 @@
 // 2 (Z(i,j) - x_i x_j) and a diagonal entry Z(i,i) - x_i^2.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdint>
 
 #include "device_common.cuh"
 #include "kernels.hpp"
+#include "tile64.cuh"
 
 namespace mdgpu {
 
@@ -135,48 +137,37 @@ __global__ void __launch_bounds__(256, 2)
 
 // ---------------------------------------------------------------------------
 // large fronts: the same recurrence in blocks of kSelT = 64 pivot columns
-// (the factor's diagonal tiles, whose inverses W it stored), one launch per
-// phase and block step over every large front of the level, many CTAs per
-// front:
-//   gather  Z_UU from the parent's Z (CTA per front and 16 columns)
-//   y       Y = L_RK W                (CTA per front and 64-row tile of R)
-//   zrk     Z_RK = -Z_RR Y            (CTA per front and 64-row tile of R)
-//   zkk     Z_KK = W'W - Y' Z_RK      (CTA per front)
-// Y and a row-major copy of Z_RK sit in the front's scratch (2 m x 64).
+// (the factor's diagonal tiles, whose inverses W it stored), many CTAs per
+// front, per level one gather of Z_UU from the parent's Z (CTA per front and
+// 16 columns), then per block step over every large front of the level:
+//   zrk     Z_RK = -Z_RR Y, CTA per front, 64-row tile of R and split of the
+//           sum over R, as partial 64 x 64 sums; the same launch computes the
+//           next step's Y = L_RK W (it needs only L)
+//   fin     the partial sums added in split order, Z_RK written, and the
+//           tile's part of Y' Z_RK kept for zkk (done by zrk itself where a
+//           launch has tiles enough and the sum is not split)
+//   zkk     Z_KK = W'W - Y' Z_RK, eight CTAs per front
+// The products are FP64 matrix instructions over gathered operands
+// (tile64.cuh).  A step is a chain of three launches, so the sums are split
+// until the launch has three CTAs for every SM.  32^3 grid (root of 2108
+// columns: 33 steps of up to 33 x 33 tiles): 5.4 ms in all, against 36.4 ms
+// with one CTA per tile row, register FMAs and a front's Y' Z_RK on one CTA.
+// Y of the even and the odd steps sit in the front's scratch (2 m x 64).
 // ---------------------------------------------------------------------------
 
 constexpr int kSelT = 64;
-// dynamic shared memory of the tiled phases: two 64 x 65 FP64 blocks
-constexpr int kSelSmem = 2 * kSelT * (kSelT + 1) * (int)sizeof(double);
+constexpr int kSelSlabs = 8;  // CTAs of zkk per front
 
-__device__ __forceinline__ double zget(const double* __restrict__ Zs,
-                                       const double* __restrict__ Zu, const FrontDesc& f,
-                                       int64_t zoff, int r, int col) {
+__device__ __forceinline__ const double* zat(const double* __restrict__ Zs,
+                                             const double* __restrict__ Zu, const FrontDesc& f,
+                                             int64_t zoff, int r, int col) {
     if (r < col) {
         const int t = r;
         r = col;
         col = t;
     }
-    if (col < f.c) return Zs[f.loff + r + (int64_t)col * f.ldl];
-    return Zu[zoff + (r - f.c) + (int64_t)(col - f.c) * f.ldu];
-}
-
-// acc[a][b] += sum over q < K of As[q lda + r0 + a] Bs[q ldb + c0 + b]
-__device__ __forceinline__ void sel_gemm(const double* As, int lda, const double* Bs, int ldb,
-                                         int K, double (&acc)[4][4]) {
-    const int tid = threadIdx.x;
-    const int r0 = (tid & 15) * 4, c0 = (tid >> 4) * 4;
-    for (int q = 0; q < K; ++q) {
-        double av[4], bv[4];
-#pragma unroll
-        for (int a = 0; a < 4; ++a) av[a] = As[q * lda + r0 + a];
-#pragma unroll
-        for (int b = 0; b < 4; ++b) bv[b] = Bs[q * ldb + c0 + b];
-#pragma unroll
-        for (int a = 0; a < 4; ++a)
-#pragma unroll
-            for (int b = 0; b < 4; ++b) acc[a][b] += av[a] * bv[b];
-    }
+    return col < f.c ? Zs + f.loff + r + (int64_t)col * f.ldl
+                     : Zu + zoff + (r - f.c) + (int64_t)(col - f.c) * f.ldu;
 }
 
 struct SelStep {
@@ -211,138 +202,178 @@ __global__ void __launch_bounds__(256)
     }
 }
 
-__global__ void __launch_bounds__(256)
-    k_sel_y(const FrontDesc* __restrict__ fronts, const int* __restrict__ items,
-            const int* __restrict__ before, int nitems, int step, const double* __restrict__ Ls,
-            const double* __restrict__ Dinv, const int64_t* __restrict__ dinv_off,
-            double* __restrict__ Yscr, const int64_t* __restrict__ yoff) {
-    extern __shared__ double sel_sm[];
-    double* As = sel_sm;                  // kSelT x kSelT
-    double* Bs = As + kSelT * kSelT;      // kSelT x (kSelT + 1)
-    const int it = find_item(before, nitems, blockIdx.x);
-    const int s = items[it], rt = blockIdx.x - before[it];
-    const FrontDesc f = fronts[s];
-    const SelStep t = sel_step(f, step);
-    const int a0 = t.k1 + kSelT * rt, rows = min(kSelT, f.m - a0);
-    const double* W = Dinv + dinv_off[s] + (int64_t)t.kb * kSelT * kSelT;
-    for (int idx = threadIdx.x; idx < kSelT * kSelT; idx += 256) {
-        const int r = idx & 63, q = idx >> 6;
-        As[q * kSelT + r] =
-            (r < rows && q < t.nb) ? Ls[f.loff + a0 + r + (int64_t)(t.k0 + q) * f.ldl] : 0.0;
-        // W(r, q) column-major: Bs[k][c] = W(k, c) with k = r, c = q
-        Bs[r * (kSelT + 1) + q] = W[r + q * kSelT];
+// a launch's work list on the device: item k of CTAs before[k] .. before[k + 1]
+struct SelList {
+    const int* items;
+    const int* before;
+    int nitems, nctas, step;
+};
+struct SelData {
+    const FrontDesc* fronts;
+    const double* Ls;
+    const double* Dinv;
+    const int64_t* dinv_off;
+    double* Zs;
+    double* Zu;
+    const int64_t* zuoff;
+    double* Yscr;
+    const int64_t* yoff;
+    double* part;  // 64 x 64 partial sums of Z_RK, then of Y' Z_RK
+    double* Q;
+    // Y of a step ((m - k1) x 64, row-major)
+    __device__ double* Y(int s, const FrontDesc& f, int step) const {
+        return Yscr + yoff[s] + (int64_t)(step & 1) * f.m * kSelT;
     }
-    __syncthreads();
-    double acc[4][4] = {};
-    sel_gemm(As, kSelT, Bs, kSelT + 1, t.nb, acc);
-    const int r0 = (threadIdx.x & 15) * 4, c0 = (threadIdx.x >> 4) * 4;
-    double* Y = Yscr + yoff[s];
-#pragma unroll
-    for (int a = 0; a < 4; ++a)
-        if (r0 + a < rows)
-#pragma unroll
-            for (int b = 0; b < 4; ++b) Y[(int64_t)(a0 + r0 + a - t.k1) * kSelT + c0 + b] = acc[a][b];
+};
+
+// one 64-row tile of Y = L_RK W
+__device__ void sel_y_tile(const SelData& D, const SelList& w, int cta, double* sm) {
+    using namespace t64;
+    const int it = find_item(w.before, w.nitems, cta);
+    const int s = w.items[it];
+    const FrontDesc f = D.fronts[s];
+    const SelStep t = sel_step(f, w.step);
+    const int a0 = t.k1 + T * (cta - w.before[it]), rows = min(T, f.m - a0), nb = t.nb;
+    const double* L = D.Ls + f.loff + a0 + (int64_t)t.k0 * f.ldl;
+    const double* W = D.Dinv + D.dinv_off[s] + (int64_t)t.kb * T * T;
+    Acc acc;
+    zero(acc);
+    product<false, true>(
+        sm, 0, nb,
+        op(L, [=](int k, int x) { return k < nb && x < rows ? L + x + (int64_t)k * f.ldl : nullptr; }),
+        op(W, [=](int k, int x) { return k < nb ? W + k + x * T : nullptr; }), acc);
+    double* Y = D.Y(s, f, w.step) + (int64_t)(a0 - t.k1) * T;
+    each(acc, [&](int r, int c, double v) {
+        if (r < rows) Y[(int64_t)r * T + c] = v;
+    });
 }
 
-__global__ void __launch_bounds__(256)
-    k_sel_zrk(const FrontDesc* __restrict__ fronts, const int* __restrict__ items,
-              const int* __restrict__ before, int nitems, int step, double* __restrict__ Zs,
-              const double* __restrict__ Zu, const int64_t* __restrict__ zuoff,
-              double* __restrict__ Yscr, const int64_t* __restrict__ yoff) {
-    extern __shared__ double sel_sm[];
-    double* As = sel_sm;                      // kSelT x (kSelT + 1)
-    double* Bs = As + kSelT * (kSelT + 1);    // kSelT x kSelT
-    const int it = find_item(before, nitems, blockIdx.x);
-    const int s = items[it], rt = blockIdx.x - before[it];
-    const FrontDesc f = fronts[s];
-    const SelStep t = sel_step(f, step);
-    const int a0 = t.k1 + kSelT * rt, rows = min(kSelT, f.m - a0);
-    const int64_t zf = (f.parent >= 0 && f.m > f.c) ? zuoff[s] : -1;
-    double* Y = Yscr + yoff[s];
-    const int ylen = f.m - t.k1;
-    double* Zrk = Y + (int64_t)f.m * kSelT;
-    double acc[4][4] = {};
-    for (int b0 = t.k1; b0 < f.m; b0 += kSelT) {
-        const int cols = min(kSelT, f.m - b0);
-        // As[q][r] = Z(a0 + r, b0 + q): read along the stored columns
-        const bool upper = b0 >= a0 + kSelT;  // every b above every a
-        for (int idx = threadIdx.x; idx < kSelT * kSelT; idx += 256) {
-            const int fast = idx & 63, slow = idx >> 6;
-            const int r = upper ? slow : fast, q = upper ? fast : slow;
-            As[q * (kSelT + 1) + r] =
-                (r < rows && q < cols) ? zget(Zs, Zu, f, zf, a0 + r, b0 + q) : 0.0;
-        }
-        for (int idx = threadIdx.x; idx < kSelT * kSelT; idx += 256) {
-            const int c = idx & 63, q = idx >> 6;
-            Bs[q * kSelT + c] = q < cols ? Y[(int64_t)(b0 + q - t.k1) * kSelT + c] : 0.0;
-        }
-        __syncthreads();
-        sel_gemm(As, kSelT + 1, Bs, kSelT, kSelT, acc);
-        __syncthreads();
+// the finished 64 x 64 sum of Z_RR Y at rows a0 ..: Z_RK and the tile's Y' Z_RK
+__device__ void sel_finish(const SelData& D, const FrontDesc& f, const SelStep& t, const double* Y,
+                           int a0, int rows, const t64::Acc& acc, double* sm, double* q) {
+    using namespace t64;
+    double* Zt = sm;           // [row][column of the block]
+    double* Yt = sm + T * LD;  // [row][column of the block]
+    each(acc, [&](int r, int c, double v) {
+        Zt[r * LD + c] = r < rows ? -v : 0.0;
+        if (r < rows && c < t.nb) D.Zs[f.loff + a0 + r + (int64_t)(t.k0 + c) * f.ldl] = -v;
+    });
+    for (int e = threadIdx.x; e < T * T; e += THREADS) {
+        const int r = e / T, c = e % T;
+        Yt[r * LD + c] = r < rows ? Y[(int64_t)(a0 - t.k1 + r) * T + c] : 0.0;
     }
-    (void)ylen;
-    const int r0 = (threadIdx.x & 15) * 4, c0 = (threadIdx.x >> 4) * 4;
-#pragma unroll
-    for (int a = 0; a < 4; ++a) {
-        const int r = r0 + a;
-        if (r >= rows) continue;
-#pragma unroll
-        for (int b = 0; b < 4; ++b) {
-            const int c = c0 + b;
-            const double v = -acc[a][b];
-            Zrk[(int64_t)(a0 + r - t.k1) * kSelT + c] = v;
-            if (c < t.nb) Zs[f.loff + a0 + r + (int64_t)(t.k0 + c) * f.ldl] = v;
-        }
+    __syncthreads();
+    Acc z;
+    zero(z);
+    for (int k = 0; k < T; k += 16) step16(Yt + k * LD, Zt + k * LD, z);
+    each(z, [&](int r, int c, double v) { q[r * T + c] = v; });
+}
+
+template <bool SPLIT>
+__global__ void __launch_bounds__(t64::THREADS, 3)
+    k_sel_zrk(SelData D, SelList w, int nsplit, SelList next) {
+    using namespace t64;
+    extern __shared__ __align__(16) double sel_sm[];
+    if ((int)blockIdx.x >= w.nctas * nsplit) {
+        sel_y_tile(D, next, blockIdx.x - w.nctas * nsplit, sel_sm);
+        return;
+    }
+    const int cta = blockIdx.x / nsplit, ks = blockIdx.x % nsplit;
+    const int it = find_item(w.before, w.nitems, cta);
+    const int s = w.items[it];
+    const FrontDesc f = D.fronts[s];
+    const SelStep t = sel_step(f, w.step);
+    const int a0 = t.k1 + T * (cta - w.before[it]), rows = min(T, f.m - a0);
+    const int64_t zf = (f.parent >= 0 && f.m > f.c) ? D.zuoff[s] : -1;
+    const double* Y = D.Y(s, f, w.step);
+    // this split's tiles of R
+    const int nt = (f.m - t.k1 + T - 1) / T;
+    const int b0 = t.k1 + T * (int)((int64_t)ks * nt / nsplit);
+    const int b1 = min(f.m, t.k1 + T * (int)((int64_t)(ks + 1) * nt / nsplit));
+    Acc acc;
+    zero(acc);
+    auto z = op(D.Zs, [&](int k, int x) -> const double* {
+        return k < b1 && x < rows ? zat(D.Zs, D.Zu, f, zf, a0 + x, k) : nullptr;
+    });
+    auto y = op(Y, [&](int k, int x) -> const double* {
+        return k < b1 ? Y + (int64_t)(k - t.k1) * T + x : nullptr;
+    });
+    // columns of R before this row tile are stored along its rows, the others
+    // along theirs
+    const int mid = min(max(a0 + T, b0), b1);
+    if (b0 < mid) {
+        auto z0 = op(D.Zs, [&](int k, int x) -> const double* {
+            return k < mid && x < rows ? zat(D.Zs, D.Zu, f, zf, a0 + x, k) : nullptr;
+        });
+        auto y0 = op(Y, [&](int k, int x) -> const double* {
+            return k < mid ? Y + (int64_t)(k - t.k1) * T + x : nullptr;
+        });
+        product<false, false>(sel_sm, b0, mid, z0, y0, acc);
+    }
+    if (mid < b1) product<true, false>(sel_sm, mid, b1, z, y, acc);
+    if constexpr (SPLIT) {
+        double* p = D.part + (int64_t)blockIdx.x * T * T;
+        each(acc, [&](int r, int c, double v) { p[r * T + c] = v; });
+    } else {
+        sel_finish(D, f, t, Y, a0, rows, acc, sel_sm, D.Q + (int64_t)cta * T * T);
     }
 }
 
-__global__ void __launch_bounds__(256)
-    k_sel_zkk(const FrontDesc* __restrict__ fronts, const int* __restrict__ items, int step,
-              double* __restrict__ Zs, const double* __restrict__ Dinv,
-              const int64_t* __restrict__ dinv_off, const double* __restrict__ Yscr,
-              const int64_t* __restrict__ yoff) {
-    extern __shared__ double sel_sm[];
-    double* As = sel_sm;                      // kSelT x (kSelT + 1) each
-    double* Bs = As + kSelT * (kSelT + 1);
-    const int s = items[blockIdx.x];
-    const FrontDesc f = fronts[s];
-    const SelStep t = sel_step(f, step);
-    const double* W = Dinv + dinv_off[s] + (int64_t)t.kb * kSelT * kSelT;
-    const double* Y = Yscr + yoff[s];
-    const double* Zrk = Y + (int64_t)f.m * kSelT;
-    // W'W: As[q][i] = W(q, i)
-    for (int idx = threadIdx.x; idx < kSelT * kSelT; idx += 256) {
-        const int q = idx & 63, i = idx >> 6;
-        const double w = W[q + i * kSelT];
-        As[q * (kSelT + 1) + i] = w;
-        Bs[q * (kSelT + 1) + i] = w;
-    }
-    __syncthreads();
-    double pos[4][4] = {}, neg[4][4] = {};
-    sel_gemm(As, kSelT + 1, Bs, kSelT + 1, t.nb, pos);
-    __syncthreads();
-    // Y' Z_RK over the rows of R
-    for (int a0 = t.k1; a0 < f.m; a0 += kSelT) {
-        const int rows = min(kSelT, f.m - a0);
-        for (int idx = threadIdx.x; idx < kSelT * kSelT; idx += 256) {
-            const int i = idx & 63, q = idx >> 6;
-            const int64_t o = (int64_t)(a0 + q - t.k1) * kSelT + i;
-            As[q * (kSelT + 1) + i] = q < rows ? Y[o] : 0.0;
-            Bs[q * (kSelT + 1) + i] = q < rows ? Zrk[o] : 0.0;
-        }
-        __syncthreads();
-        sel_gemm(As, kSelT + 1, Bs, kSelT + 1, kSelT, neg);
-        __syncthreads();
-    }
-    const int r0 = (threadIdx.x & 15) * 4, c0 = (threadIdx.x >> 4) * 4;
+__global__ void __launch_bounds__(t64::THREADS, 3) k_sel_fin(SelData D, SelList w, int nsplit) {
+    using namespace t64;
+    extern __shared__ __align__(16) double sel_sm[];
+    const int cta = blockIdx.x;
+    const int it = find_item(w.before, w.nitems, cta);
+    const int s = w.items[it];
+    const FrontDesc f = D.fronts[s];
+    const SelStep t = sel_step(f, w.step);
+    const int a0 = t.k1 + T * (cta - w.before[it]), rows = min(T, f.m - a0);
+    Acc acc;
+    zero(acc);
+    for (int ks = 0; ks < nsplit; ++ks) {
+        const double* p = D.part + ((int64_t)cta * nsplit + ks) * T * T;
+        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, q = lane & 3;
+        const int wr = (warp & 1) * 32, wc = (warp >> 1) * 32;
 #pragma unroll
-    for (int a = 0; a < 4; ++a)
+        for (int m = 0; m < 2; ++m)
 #pragma unroll
-        for (int b = 0; b < 4; ++b) {
-            const int i = r0 + a, j = c0 + b;
-            if (i < t.nb && j < t.nb && i >= j)
-                Zs[f.loff + (t.k0 + i) + (int64_t)(t.k0 + j) * f.ldl] = pos[a][b] - neg[a][b];
-        }
+            for (int n = 0; n < 2; ++n)
+#pragma unroll
+                for (int r = 0; r < 2; ++r) {
+                    const double* e = p + (wr + 16 * m + 2 * g + r) * T + wc + 16 * n + 4 * q;
+                    const double2 u = *reinterpret_cast<const double2*>(e);
+                    const double2 v = *reinterpret_cast<const double2*>(e + 2);
+                    acc[m][n][0][2 * r] += u.x;
+                    acc[m][n][1][2 * r] += u.y;
+                    acc[m][n][0][2 * r + 1] += v.x;
+                    acc[m][n][1][2 * r + 1] += v.y;
+                }
+    }
+    sel_finish(D, f, t, D.Y(s, f, w.step), a0, rows, acc, sel_sm, D.Q + (int64_t)cta * T * T);
+}
+
+__global__ void __launch_bounds__(256) k_sel_zkk(SelData D, SelList w) {
+    constexpr int T = kSelT;
+    __shared__ double Ws[T * (T + 1)];
+    const int it = blockIdx.x / kSelSlabs, slab = blockIdx.x % kSelSlabs;
+    const int s = w.items[it];
+    const FrontDesc f = D.fronts[s];
+    const SelStep t = sel_step(f, w.step);
+    if (slab * (T / kSelSlabs) >= t.nb) return;
+    const double* W = D.Dinv + D.dinv_off[s] + (int64_t)t.kb * T * T;
+    for (int e = threadIdx.x; e < T * T; e += 256) Ws[(e & 63) * (T + 1) + (e >> 6)] = W[e];
+    __syncthreads();
+    const int cta0 = w.before[it], cta1 = w.before[it + 1];
+    for (int e = threadIdx.x; e < T * (T / kSelSlabs); e += 256) {
+        const int j = slab * (T / kSelSlabs) + e % (T / kSelSlabs), i = e / (T / kSelSlabs);
+        if (i < j || i >= t.nb) continue;
+        double neg = 0.0, pos = 0.0;
+        const double* q = D.Q + (int64_t)cta0 * T * T + i * T + j;
+#pragma unroll 8
+        for (int b = cta0; b < cta1; ++b, q += T * T) neg += *q;
+        for (int k = i; k < t.nb; ++k) pos += Ws[k * (T + 1) + i] * Ws[k * (T + 1) + j];
+        D.Zs[f.loff + (t.k0 + i) + (int64_t)(t.k0 + j) * f.ldl] = pos - neg;
+    }
 }
 
 // G (caller order; zeroed by the caller) of every lower-triangle entry e:
@@ -368,15 +399,17 @@ __global__ void k_grad_lower(int nnz, const FrontDesc* __restrict__ fronts,
 }
 
 // logdet = 2 sum log L(j, j): per block a fixed-order sum over its
-// supernodes, then one block sums the partials (deterministic)
+// supernodes, a warp each (a root of thousands of columns read by one thread
+// took 1.1 ms), then one block sums the partials (deterministic)
 template <typename T>
 __global__ void k_logdet_partial(int nsuper, const FrontDesc* __restrict__ fronts,
                                  const T* __restrict__ Ls, double* __restrict__ partial) {
     __shared__ double red[256];
     double v = 0.0;
-    for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < nsuper; s += gridDim.x * blockDim.x) {
+    const int lane = threadIdx.x & 31, wpb = blockDim.x >> 5;
+    for (int s = blockIdx.x * wpb + (threadIdx.x >> 5); s < nsuper; s += gridDim.x * wpb) {
         const FrontDesc f = fronts[s];
-        for (int j = 0; j < f.c; ++j) v += log((double)Ls[f.loff + j + (int64_t)j * f.ldl]);
+        for (int j = lane; j < f.c; j += 32) v += log((double)Ls[f.loff + j + (int64_t)j * f.ldl]);
     }
     red[threadIdx.x] = v;
     __syncthreads();
@@ -403,34 +436,77 @@ __global__ void k_logdet_final(int nparts, const double* __restrict__ partial,
 
 constexpr int kLogdetBlocks = 148 * 2;
 
+// splits of a step's sums: until the launch has three CTAs per SM
+static int sel_splits(int nctas, int num_sms) {
+    const int want = 3 * num_sms;
+    return nctas >= want || nctas == 0 ? 1 : std::min((want + nctas - 1) / nctas, 16);
+}
+// doubles of the partial sums and of the Y' Z_RK parts over every step
+int64_t selinv_partials(const DevPlan& D) {
+    int64_t p = 1, q = 1;
+    for (const WorkList& w : D.sel.h_steps) {
+        const int ns = sel_splits(w.nctas, D.num_sms);
+        if (ns > 1) p = std::max<int64_t>(p, (int64_t)w.nctas * ns);
+        q = std::max<int64_t>(q, w.nctas);
+    }
+    return (p + q) * kSelT * kSelT;
+}
+
 // Level by level from the root: the small fronts one CTA each
-// (k_selinv_front), the large fronts by the tiled phases above, block step
-// by block step (fronts with fewer pivot blocks join the later steps).
+// (k_selinv_front) on a stream of their own, the large fronts by the tiled
+// phases above beside them, block step by block step (fronts with fewer
+// pivot blocks join the later steps).
 void launch_selinv(const DevPlan& D, const double* Ls, const double* Dinv, double* Zs,
-                   double* Zu, double* Yscr, cudaStream_t st) {
+                   double* Zu, double* Yscr, double* part, cudaStream_t st) {
     const SelSchedule& S = D.sel;
+    int64_t psize = 1;
+    for (const WorkList& w : S.h_steps) {
+        const int ns = sel_splits(w.nctas, D.num_sms);
+        if (ns > 1) psize = std::max<int64_t>(psize, (int64_t)w.nctas * ns);
+    }
+    const SelData data{D.fronts, Ls, Dinv, D.dinv_off, Zs, Zu, D.zuoff, Yscr, D.yoff,
+                       part, part + psize * kSelT * kSelT};
+    auto list = [&](const WorkList& w) {
+        return SelList{S.items + w.off, S.before + w.off, w.nitems, w.nctas, w.step};
+    };
+    const SelList none{nullptr, nullptr, 0, 0, 0};
+    constexpr size_t SM = t64::SMEM_BYTES;
     for (int l = D.nlevels - 1; l >= 0; --l) {
         const int sb = D.h_small_ptr[l * kSmallBuckets], se = D.h_small_ptr[(l + 1) * kSmallBuckets];
+        const int q0 = S.h_step_beg[l], q1 = S.h_step_beg[l + 1];
+        const bool fork = se > sb && q1 > q0 && D.piece_st[0];
+        const cudaStream_t ss = fork ? D.piece_st[0] : st;
+        if (fork) {
+            cudaEventRecord(D.fork_ev, st);
+            cudaStreamWaitEvent(ss, D.fork_ev, 0);
+        }
         if (se > sb)
-            k_selinv_front<<<se - sb, 256, 0, st>>>(D.fronts, D.small_list + sb, D.relmap, Ls, Zs,
+            k_selinv_front<<<se - sb, 256, 0, ss>>>(D.fronts, D.small_list + sb, D.relmap, Ls, Zs,
                                                     Zu, D.zuoff, Yscr, D.yoff);
+        if (fork) cudaEventRecord(D.piece_join[0], ss);
+        if (q1 > q0) {
+            const SelList y = list(S.h_steps[q0]);
+            if (y.nctas > 0)
+                k_sel_zrk<false><<<y.nctas, t64::THREADS, SM, st>>>(data, none, 1, y);
+        }
         const WorkList& g = S.h_gather[l];
         if (g.nctas > 0)
             k_sel_gather<<<g.nctas, 256, 0, st>>>(D.fronts, S.items + g.off, S.before + g.off,
                                                   g.nitems, D.relmap, Zs, Zu, D.zuoff);
-        for (int q = S.h_step_beg[l]; q < S.h_step_beg[l + 1]; ++q) {
-            const WorkList& w = S.h_steps[q];
-            if (w.nctas > 0) {
-                k_sel_y<<<w.nctas, 256, kSelSmem, st>>>(D.fronts, S.items + w.off,
-                                                        S.before + w.off, w.nitems, w.step, Ls,
-                                                        Dinv, D.dinv_off, Yscr, D.yoff);
-                k_sel_zrk<<<w.nctas, 256, kSelSmem, st>>>(D.fronts, S.items + w.off,
-                                                          S.before + w.off, w.nitems, w.step, Zs,
-                                                          Zu, D.zuoff, Yscr, D.yoff);
+        for (int q = q0; q < q1; ++q) {
+            const SelList w = list(S.h_steps[q]);
+            const SelList next = q + 1 < q1 ? list(S.h_steps[q + 1]) : none;
+            const int ns = sel_splits(w.nctas, D.num_sms);
+            const int grid = w.nctas * ns + next.nctas;
+            if (ns > 1) {
+                k_sel_zrk<true><<<grid, t64::THREADS, SM, st>>>(data, w, ns, next);
+                k_sel_fin<<<w.nctas, t64::THREADS, SM, st>>>(data, w, ns);
+            } else if (grid > 0) {
+                k_sel_zrk<false><<<grid, t64::THREADS, SM, st>>>(data, w, ns, next);
             }
-            k_sel_zkk<<<w.nitems, 256, kSelSmem, st>>>(D.fronts, S.items + w.off, w.step, Zs,
-                                                       Dinv, D.dinv_off, Yscr, D.yoff);
+            k_sel_zkk<<<w.nitems * kSelSlabs, 256, 0, st>>>(data, w);
         }
+        if (fork) cudaStreamWaitEvent(st, D.piece_join[0], 0);
     }
 }
 
@@ -453,9 +529,10 @@ int logdet_partials() { return kLogdetBlocks; }
 int selinv_block() { return kSelBlock; }
 
 void init_selinv() {
-    cudaFuncSetAttribute(k_sel_y, cudaFuncAttributeMaxDynamicSharedMemorySize, kSelSmem);
-    cudaFuncSetAttribute(k_sel_zrk, cudaFuncAttributeMaxDynamicSharedMemorySize, kSelSmem);
-    cudaFuncSetAttribute(k_sel_zkk, cudaFuncAttributeMaxDynamicSharedMemorySize, kSelSmem);
+    const int sm = (int)t64::SMEM_BYTES;
+    cudaFuncSetAttribute(k_sel_zrk<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
+    cudaFuncSetAttribute(k_sel_zrk<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
+    cudaFuncSetAttribute(k_sel_fin, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
 }
 int selinv_tile() { return kSelT; }
 

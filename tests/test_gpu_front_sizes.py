@@ -95,3 +95,18 @@ def test_solve_groups(c1, c2, u, precision):
         full = X if full is None else full
         same = k if k % 8 != 1 else k - 1  # a lone last column of a pass takes the one-column sweep
         assert np.array_equal(X[:, :min(same, 64)], full[:, :min(same, 64)])
+
+
+@pytest.mark.parametrize("c1,c2,u", SIZES)
+def test_selected_inverse(c1, c2, u):
+    """The gradient of log det A on A's pattern is the inverse there (twice it
+    off the diagonal); a backward stable inverse is good to n eps cond, as L."""
+    n, A, Ap, Ai, Ax = _two_leaves(c1, c2, u)
+    S = M.Solver(n, Ap, Ai, ordering=M.ORDER_NATURAL)
+    S.factor(torch.from_numpy(Ax).cuda(), M.FP64)
+    sign, ref = np.linalg.slogdet(A)
+    assert abs(S.logdet() - ref) <= 1e-12 * abs(ref)
+    S.selinv()
+    cols = np.repeat(np.arange(n), np.diff(Ap))
+    Z = np.linalg.inv(A)[Ai, cols] * np.where(Ai == cols, 1.0, 2.0)
+    assert np.linalg.norm(S.grad_lower() - Z) <= 1e-12 * np.linalg.norm(Z)
