@@ -130,7 +130,7 @@ struct mdgpu_handle_s {
     double* dZu64 = nullptr;       // its update parts (plan.zuoff offsets)
     // general reverse mode: Fbar panels, Ubar store, c x c scratch, Lbar / Abar
     double *d_Fb = nullptr, *d_Fu = nullptr, *d_W = nullptr, *d_Lbar = nullptr,
-           *d_Abar = nullptr;
+           *d_Abar = nullptr, *d_adjpart = nullptr;
     double* d_Y = nullptr;         // its Y scratch
     double* d_selpart = nullptr;   // its partial sums
     double* d_logdet = nullptr;    // logdet partial sums, then the result
@@ -163,7 +163,8 @@ struct mdgpu_handle_s {
         for (void* p : {(void*)d_Fb, (void*)d_Fu, (void*)d_W, (void*)d_Lbar, (void*)d_Abar})
             if (p) cudaFree(p);
         for (void* p : {(void*)dZ64, (void*)dZu64, (void*)d_Y, (void*)d_logdet, (void*)d_gx, (void*)d_gG,
-                        (void*)d_gm, (void*)d_ssync, (void*)d_selpart})
+                        (void*)d_gm, (void*)d_ssync, (void*)d_selpart,
+                        (void*)d_adjpart})
             if (p) cudaFree(p);
         for (void* p : {(void*)d_Ax, (void*)dL64, (void*)dU64, (void*)dL32, (void*)dU32,
                         (void*)dD64, (void*)dD32,
@@ -231,6 +232,7 @@ void init_kernels_once() {
     init_schur_f64();
     init_panel_kernels();
     init_selinv();
+    init_adjoint();
     done = true;
 }
 
@@ -404,6 +406,7 @@ void upload_plan(mdgpu_handle_s* h, bool check = false) {
             AdjSchedule& AS = D.adj;
             ListStore st;
             AS.h_gather.assign(P.nlevels, WorkList{0, 0, 0, 0});
+            AS.h_large.assign(P.nlevels, AdjLevel{});
             std::vector<int64_t> wo(P.nsuper, 0);
             AS.wtotal = 1;
             for (int l = 0; l < P.nlevels; ++l) {
@@ -418,6 +421,28 @@ void upload_plan(mdgpu_handle_s* h, bool check = false) {
                 }
                 AS.wtotal = std::max(AS.wtotal, off);
                 if (!g.empty()) AS.h_gather[l] = st.add(g, 0);
+                std::vector<std::pair<int, int>> nr, wl, wr, wt, wp;
+                for (int q = P.large_ptr[l]; q < P.large_ptr[l + 1]; ++q) {
+                    const int s = P.large_list[q];
+                    const FrontDesc& f = P.fronts[s];
+                    const int rt = (f.m - f.c + kTile - 1) / kTile, ct = (f.c + kTile - 1) / kTile;
+                    if (ct == 1) {
+                        nr.push_back({s, rt});
+                    } else {
+                        wl.push_back({s, rt * ct});
+                        wr.push_back({s, rt});
+                        wt.push_back({s, ct * (ct + 1) / 2});
+                        wp.push_back({s, ct});
+                    }
+                }
+                AdjLevel& A = AS.h_large[l];
+                if (!nr.empty()) A.rows = st.add(nr, 0);
+                if (!wl.empty()) {
+                    A.wide_l21 = st.add(wl, 0);
+                    A.wide_rows = st.add(wr, 0);
+                    A.wide_low = st.add(wt, 0);
+                    A.wide_piv = st.add(wp, 0);
+                }
             }
             if (st.items.empty()) {
                 st.items.assign(1, -1);
@@ -1774,8 +1799,9 @@ int mdgpu_adjoint_device(mdgpu_handle h, const double* dLbar, double* dAbar, voi
         if (!h->d_Fb) h->d_Fb = dalloc<double>(P.lstore);
         if (!h->d_Fu) h->d_Fu = dalloc<double>(P.zustore);
         if (!h->d_W) h->d_W = dalloc<double>(h->D.adj.wtotal);
-        launch_adjoint(h->D, (int)P.a_src.size(), h->dL64, dLbar, h->d_Fb, h->d_Fu, h->d_W,
-                       dAbar, st);
+        if (!h->d_adjpart) h->d_adjpart = dalloc<double>(adjoint_parts(h->D));
+        launch_adjoint(h->D, (int)P.a_src.size(), h->dL64, h->dD64, dLbar, h->d_Fb, h->d_Fu,
+                       h->d_W, h->d_adjpart, dAbar, st);
         ck(cudaGetLastError(), "adjoint launch");
         return MDGPU_OK;
     });

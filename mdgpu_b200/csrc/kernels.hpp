@@ -144,8 +144,17 @@ struct SelSchedule {
 // General reverse mode (adjoint.cu): per level the fronts with an update
 // part and a parent, for the gather of their Ubar (CTA per 16 columns); L's
 // column pointers; per front the offset of its c x c scratch (a level's
-// fronts side by side, levels reuse it).
+// fronts side by side, levels reuse it).  Large fronts by level: the narrow
+// ones (one pivot tile) with a CTA per 64 update rows, the wide ones with a
+// CTA per 64 x 64 tile of L21, per 64 update rows, per lower tile and per 64
+// columns of the pivot block.
+struct AdjLevel {
+    WorkList rows{0, 0, 0, 0};
+    WorkList wide_l21{0, 0, 0, 0}, wide_rows{0, 0, 0, 0}, wide_low{0, 0, 0, 0},
+        wide_piv{0, 0, 0, 0};
+};
 struct AdjSchedule {
+    std::vector<AdjLevel> h_large;  // per level
     int* items = nullptr;
     int* before = nullptr;
     std::vector<WorkList> h_gather;  // per level
@@ -247,6 +256,7 @@ void init_schur_tc();
 void init_schur_f64();
 void init_panel_kernels();
 void init_selinv();
+void init_adjoint();
 
 // panel scratch rows of a large front (m rounded up to the 128-row tile)
 __host__ __device__ inline int panel_mpad(int m) { return (m + 127) & ~127; }
@@ -313,9 +323,12 @@ template <typename T>
 void launch_logdet(const DevPlan& D, const T* Ls, double* partial, double* out, cudaStream_t st);
 int logdet_partials();
 // Abar (nnz entries, caller order) from Lbar (L's CSC values) with the FP64
-// factor Ls: Fb, Fu, Wscr stores of plan lstore, zustore, adj.wtotal doubles
-void launch_adjoint(const DevPlan& D, int nnz, const double* Ls, const double* Lbar, double* Fb,
-                    double* Fu, double* Wscr, double* Abar, cudaStream_t st);
+// factor Ls, Dinv: Fb, Fu, Wscr, part stores of plan lstore, zustore,
+// adj.wtotal and adjoint_parts() doubles
+void launch_adjoint(const DevPlan& D, int nnz, const double* Ls, const double* Dinv,
+                    const double* Lbar, double* Fb, double* Fu, double* Wscr, double* part,
+                    double* Abar, cudaStream_t st);
+int64_t adjoint_parts(const DevPlan& D);
 int selinv_block();  // pivot columns per block of the one-CTA (small-front) kernel
 int selinv_tile();   // pivot columns per block step of the large fronts
 

@@ -193,12 +193,23 @@ __global__ void __launch_bounds__(256)
     const FrontDesc f = fronts[s];
     const FrontDesc p = fronts[f.parent];
     const int u = f.m - f.c;
+    const int lane = threadIdx.x & 31;
     const int64_t zf = zuoff[s], zp = zuoff[f.parent];
     const int* rm = relmap + f.rows_off + f.c;
-    for (int b = 16 * blk; b < min(16 * blk + 16, u); ++b) {
+    for (int b = 16 * blk + (threadIdx.x >> 5); b < min(16 * blk + 16, u); b += 8) {
         const int pb = rm[b];
-        for (int a = b + (int)threadIdx.x; a < u; a += blockDim.x)
-            Zu[zf + a + (int64_t)b * f.ldu] = zelem(Zs, Zu, p, zp, rm[a], pb);
+        // the parent's column, by front row
+        const double* src = pb < p.c ? Zs + p.loff + (int64_t)pb * p.ldl
+                                     : Zu + zp - p.c + (int64_t)(pb - p.c) * p.ldu;
+        double* dst = Zu + zf + (int64_t)b * f.ldu;
+        for (int a0 = b + lane; a0 < u; a0 += 4 * 32) {
+            double v[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) v[k] = a0 + 32 * k < u ? src[rm[a0 + 32 * k]] : 0.0;
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+                if (a0 + 32 * k < u) dst[a0 + 32 * k] = v[k];
+        }
     }
 }
 

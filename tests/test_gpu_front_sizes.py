@@ -110,3 +110,25 @@ def test_selected_inverse(c1, c2, u):
     cols = np.repeat(np.arange(n), np.diff(Ap))
     Z = np.linalg.inv(A)[Ai, cols] * np.where(Ai == cols, 1.0, 2.0)
     assert np.linalg.norm(S.grad_lower() - Z) <= 1e-12 * np.linalg.norm(Z)
+
+
+@pytest.mark.parametrize("c1,c2,u", SIZES)
+def test_reverse_mode(c1, c2, u):
+    """Abar of a random Lbar against the dense adjoint of Cholesky (Murray
+    2016): two more triangular solves than the inverse, so ten times its
+    bound."""
+    n, A, Ap, Ai, Ax = _two_leaves(c1, c2, u)
+    S = M.Solver(n, Ap, Ai, ordering=M.ORDER_NATURAL)
+    S.factor(torch.from_numpy(Ax).cuda(), M.FP64)
+    Lp, Li, _ = S.get_L(values=False)
+    lbar = np.random.default_rng(3).uniform(-1.0, 1.0, len(Li))
+    Lbar = np.zeros((n, n))
+    Lbar[Li, np.repeat(np.arange(n), np.diff(Lp))] = lbar
+    L = np.linalg.cholesky(A)
+    P = np.tril(L.T @ Lbar)
+    P[np.diag_indices(n)] *= 0.5
+    inv = np.linalg.inv(L)
+    H = 0.5 * inv.T @ (P + P.T) @ inv
+    cols = np.repeat(np.arange(n), np.diff(Ap))
+    ref = H[Ai, cols] * np.where(Ai == cols, 1.0, 2.0)
+    assert np.linalg.norm(S.adjoint(lbar) - ref) <= 1e-11 * np.linalg.norm(ref)
