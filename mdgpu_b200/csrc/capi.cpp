@@ -115,7 +115,6 @@ struct mdgpu_handle_s {
     float* dD32 = nullptr;
     double *d_xp = nullptr, *d_fv = nullptr, *d_B = nullptr, *d_X = nullptr, *d_R = nullptr,
            *d_D = nullptr;
-    int* d_ssync = nullptr;  // sync words of the solve
     int nrhs_cap = 0;
     // CUDA graphs of the numeric launch sequences (captured once, replayed)
     bool use_graphs = true;
@@ -163,7 +162,7 @@ struct mdgpu_handle_s {
         for (void* p : {(void*)d_Fb, (void*)d_Fu, (void*)d_W, (void*)d_Lbar, (void*)d_Abar})
             if (p) cudaFree(p);
         for (void* p : {(void*)dZ64, (void*)dZu64, (void*)d_Y, (void*)d_logdet, (void*)d_gx, (void*)d_gG,
-                        (void*)d_gm, (void*)d_ssync, (void*)d_selpart,
+                        (void*)d_gm, (void*)d_selpart,
                         (void*)d_adjpart})
             if (p) cudaFree(p);
         for (void* p : {(void*)d_Ax, (void*)dL64, (void*)dU64, (void*)dL32, (void*)dU32,
@@ -517,13 +516,7 @@ void upload_plan(mdgpu_handle_s* h, bool check = false) {
             D.solve.fwd_wlist = h->keep(upload(wf));
             D.solve.bwd_wlist = h->keep(upload(wb));
         }
-        D.solve.bwd_target = h->keep(upload(SS.bwd_target));
-        D.solve.nfronts = P.nsuper;
-        // one group of right-hand sides (all that a solve that may not
-        // allocate can count on; ensure_solve_storage grows it)
-        h->d_ssync = dalloc<int>(solve_sync_words(SS.nflags, P.nsuper, 1));
-        D.solve.sync = h->d_ssync;
-        D.solve.sync_groups = 1;
+        D.solve.sync = h->keep(dalloc<int>(4));
     }
     // algorithmic work per launch, for the profiler's roofline figures
     {
@@ -650,14 +643,6 @@ void ensure_solve_storage(mdgpu_handle_s* h, int nrhs) {
     }
     int64_t n = h->plan.n;
     int chunk = std::min(nrhs, 64);
-    const int groups = solve_groups(chunk);
-    if (groups > h->D.solve.sync_groups) {
-        int* grown = dalloc<int>(solve_sync_words(h->D.solve.nflags, h->plan.nsuper, groups));
-        cudaFree(h->d_ssync);
-        h->d_ssync = grown;
-        h->D.solve.sync = h->d_ssync;
-        h->D.solve.sync_groups = groups;
-    }
     h->d_xp = dalloc<double>(n * nrhs);
     h->d_fv = dalloc<double>(h->D.fv_total * chunk);
     h->d_B = dalloc<double>(n * nrhs);
@@ -751,9 +736,9 @@ void do_solve(mdgpu_handle_s* h, const double* dB, int ldb, double* dX, int ldx,
         const int prec = h->factored;
         auto run = [h, prec, nq](cudaStream_t s) {
             if (prec == MDGPU_FP64)
-                solve_levels<double, double>(h->D, h->dL64, h->dD64, h->d_xp, h->d_fv, nq, s);
+                solve_levels<double>(h->D, h->dL64, h->dD64, h->d_xp, h->d_fv, nq, s);
             else
-                solve_levels<float, double>(h->D, h->dL32, h->dD32, h->d_xp, h->d_fv, nq, s);
+                solve_levels<float>(h->D, h->dL32, h->dD32, h->d_xp, h->d_fv, nq, s);
         };
         if (h->use_graphs && !h->prof.on) {
             cudaGraphExec_t& g = h->sgraph[prec * 1024 + nq];
@@ -762,7 +747,7 @@ void do_solve(mdgpu_handle_s* h, const double* dB, int ldb, double* dX, int ldx,
         } else {
             run(st);
         }
-        permute_scatter(h->d_perm, h->d_xp, dX + (int64_t)q0 * ldx, n, nq, ldx, st);
+        permute_solution(h->D, h->d_perm, h->d_fv, dX + (int64_t)q0 * ldx, nq, ldx, st);
     }
     ck(cudaGetLastError(), "solve launch");
 }
@@ -1903,10 +1888,10 @@ int mdgpu_solve_device_noalloc(mdgpu_handle h, const double* dB, int ldb, double
             const int nq = std::min(64, nrhs - q0);
             permute_gather(h->d_perm, dB + (int64_t)q0 * ldb, xp, n, nq, ldb, st);
             if (h->factored == MDGPU_FP64)
-                solve_levels<double, double>(h->D, h->dL64, h->dD64, xp, fv, nq, st);
+                solve_levels<double>(h->D, h->dL64, h->dD64, xp, fv, nq, st);
             else
-                solve_levels<float, double>(h->D, h->dL32, h->dD32, xp, fv, nq, st);
-            permute_scatter(h->d_perm, xp, dX + (int64_t)q0 * ldx, n, nq, ldx, st);
+                solve_levels<float>(h->D, h->dL32, h->dD32, xp, fv, nq, st);
+            permute_solution(h->D, h->d_perm, fv, dX + (int64_t)q0 * ldx, nq, ldx, st);
         }
         ck(cudaGetLastError(), "solve launch");
         return solve_status_check(h, st);

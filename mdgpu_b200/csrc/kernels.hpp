@@ -93,12 +93,8 @@ struct DevSchedule {
 
 // Solve: one launch per direction over every level's work items (see
 // SolveScheduleHost).  sync holds the two ticket counters and the abort word,
-// then per group of right-hand sides (sync_groups of them) one count per
-// pivot tile (backward gathers counted in) and per front the forward count of
-// finished children, the forward count of finished update tiles and the
-// backward count of finished completions; it is cleared at the start of every
-// solve.  err (not cleared by the solve) gets bit 0 when a dependency wait ran
-// out.
+// cleared at the start of every solve.  err (not cleared by the solve) gets
+// bit 0 when a wait ran out.
 struct SolveSchedule {
     int2* tasks = nullptr;
     int4* fwd_items = nullptr;
@@ -106,13 +102,10 @@ struct SolveSchedule {
     int nfwd_items = 0, nbwd_items = 0;
     int* fwd_wlist = nullptr;    // the warp items' fronts, per direction
     int* bwd_wlist = nullptr;
-    int* bwd_target = nullptr;   // per front
-    int nfronts = 0;
     std::vector<int> fwd_task_beg, bwd_task_beg;  // nlevels + 1
     std::vector<double> fwd_elems, bwd_elems;     // per level: L + Dinv elements
     std::vector<double> small_elems;              // per level: L elements of small fronts
     int* sync = nullptr;
-    int sync_groups = 0;  // groups of right-hand sides the sync words hold
     int nflags = 0;
     int* err = nullptr;
     // backward update-row partial sums (see SolveScheduleHost)
@@ -274,16 +267,12 @@ template <typename T>
 void factor_levels(const DevPlan& D, T* Ls, T* Us, T* Dinv, const double* Ax, int* status,
                    cudaStream_t st, int smode = kSchur3xTF32);
 
-// Solves with the factor L (scalar TL) on vectors of type TV.  xp holds the
-// permuted right-hand sides on entry (n x nrhs, ld n) and the permuted
-// solution on exit; fv is scratch of fv_total * nrhs entries.
-template <typename TL, typename TV>
-void solve_levels(const DevPlan& D, const TL* Ls, const TL* Dinv, TV* xp, TV* fv, int nrhs,
+// Solves with the factor L (scalar TL).  xp holds the permuted right-hand
+// sides on entry as permute_gather leaves them (overwritten); fv is scratch of fv_total *
+// nrhs entries and holds the solution on exit, for permute_solution.
+template <typename TL>
+void solve_levels(const DevPlan& D, const TL* Ls, const TL* Dinv, double* xp, double* fv, int nrhs,
                   cudaStream_t st);
-
-// groups of right-hand sides of one solve launch, and the sync words they need
-int solve_groups(int nrhs);
-int64_t solve_sync_words(int nflags, int nfronts, int groups);
 
 // Per large front a map over its panel scratch (base scr + scr_off[s],
 // row-major, kPanel columns): bf16, the BF16 copy (mpad rows); else the
@@ -310,8 +299,8 @@ double* noalloc_scratch(std::string& msg);
 // gather / scatter with the fill-reducing permutation (perm: new -> old)
 void permute_gather(const int* perm, const double* b, double* xp, int n, int nrhs, int ldb,
                     cudaStream_t st);
-void permute_scatter(const int* perm, const double* xp, double* x, int n, int nrhs, int ldx,
-                     cudaStream_t st);
+void permute_solution(const DevPlan& D, const int* perm, const double* fv, double* x, int nrhs,
+                      int ldx, cudaStream_t st);
 
 // selected inverse and adjoint (selinv.cu)
 void launch_selinv(const DevPlan& D, const double* Ls, const double* Dinv, double* Zs,

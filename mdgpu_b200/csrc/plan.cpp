@@ -722,8 +722,6 @@ void build_solve_schedule(const Plan& P, int T, SolveScheduleHost& S) {
             flush();
         }
     }
-    S.bwd_target.assign(P.nsuper, 1);
-    for (int s : P.large_list) S.bwd_target[s] = (P.fronts[s].c + T - 1) / T;
 }
 
 void build_panel_schedule(const Plan& P, int T, int PW, int CB, PanelSchedule& S) {

@@ -248,10 +248,6 @@ struct SolveScheduleHost {
     static constexpr int kWarpsPerItem = 8;
     std::vector<int> fwd_items, bwd_items;
     std::vector<int> fwd_wlist, bwd_wlist;  // the warp items' fronts
-    // backward: the solution rows of front s are final once bwd_target[s]
-    // completions are counted (one per pivot tile of a large front, one for
-    // a small front)
-    std::vector<int> bwd_target;
     // small fronts of each level for the warp-per-front factor, by rows
     // descending (same level ranges as small_list): warp_cnt[3 l + k] fronts
     // of more than 16 rows (k = 0, a warp each), of 9..16 rows (k = 1, two

@@ -350,10 +350,6 @@ std::string check_plan(const Plan& P, const Symbolic& S, const SolveScheduleHost
                     }
                 }
             }
-            if ((int)Q.bwd_target.size() != ns) bad("backward targets");
-            for (int s = 0; s < ns; ++s)
-                if (Q.bwd_target[s] != (is_large[s] ? (P.fronts[s].c + T - 1) / T : 1))
-                    bad("backward target", s);
         }
         // the residual's CSR of the caller's matrix
         if ((int)csr_rowptr.size() != n + 1 || csr_rowptr[0] != 0 || csr_rowptr[n] != csr_nnz)

@@ -12,6 +12,7 @@
 // 64-row tiles; a pivot tile applies its block's inverse (stored by the
 // factorization), a 64 x 64 product instead of a serial substitution.
 #include <algorithm>
+#include <type_traits>
 
 #include "device_common.cuh"
 #include "kernels.hpp"
@@ -21,69 +22,41 @@ namespace mdgpu {
 // Front vector of supernode s: rows fv_off[s] .. fv_off[s] + m - 1 of one
 // array whose row holds the nrhs right-hand sides side by side, so row r,
 // right-hand side q is front_vec(...)[r * nrhs + q].
-template <typename TV>
-__device__ inline TV* front_vec(TV* fv, const int64_t* fv_off, int s, int nrhs) {
+__device__ inline double* front_vec(double* fv, const int64_t* fv_off, int s, int nrhs) {
     return fv + fv_off[s] * nrhs;
 }
 
 // ---------------------------------------------------------------------------
-// one launch per level and direction: dependency-ordered tile tasks
+// one launch per direction: dependency-ordered work items
 //
-// Each CTA takes the next task by an atomic ticket, so every task that
-// started before it holds a lower ticket; the task lists are ordered so that
-// a task only waits for tasks earlier in its list, hence for CTAs that are
-// already resident, and the waits cannot deadlock.  A pivot tile publishes
-// its solution values and then a flag (release); a dependent task polls the
-// flag (acquire) with an iteration limit, after which the solve is aborted
-// (every waiter leaves) and the error word is set for the host.
+// Each CTA takes the next item by an atomic ticket, so every item that
+// started before it holds a lower ticket; the lists are ordered so that an
+// item only waits for items earlier in its list, hence for CTAs that are
+// already resident, and the waits cannot deadlock.  A consumer polls the values
+// themselves with an iteration limit, after which the solve is aborted (every
+// waiter leaves) and the error word is set for the host.
 // ---------------------------------------------------------------------------
 
 constexpr int kSolveWaitPolls = 1 << 18;  // ~0.1-0.3 s at ~1 us per poll
-constexpr int kWarpSolveRhs = 4;   // right-hand sides per pass of the warp path
 constexpr int kVecLD = kTile + 4;  // column stride of a vector block in shared memory: 4 mod 16
                                    // doubles, a conflict-free operand of the matrix instructions
 constexpr int kGroupRhs = 8;       // right-hand sides of one group (a matrix instruction's columns)
 
-__device__ __forceinline__ int ld_acquire_gpu(const int* p) {
-    int v;
-    asm volatile("ld.acquire.gpu.global.b32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-    return v;
-}
 __device__ __forceinline__ int ld_relaxed_gpu(const int* p) {
     int v;
     asm volatile("ld.relaxed.gpu.global.b32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
     return v;
 }
-__device__ __forceinline__ void st_release_gpu(int* p, int v) {
-    asm volatile("st.release.gpu.global.b32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
-}
-// load of a value another CTA of this launch published (ordered after the
-// acquire by the CTA barrier; never served from this SM's L1)
-__device__ __forceinline__ double ld_shared_value(const double* p) {
-    double v;
-    asm volatile("ld.relaxed.gpu.global.f64 %0, [%1];" : "=d"(v) : "l"(p) : "memory");
-    return v;
-}
-
-__device__ bool wait_flag(const int* flag, int target, int* abort_flag, int* err) {
-    for (int it = 0; it < kSolveWaitPolls; ++it) {
-        if (ld_acquire_gpu(flag) >= target) return true;
-        if (ld_relaxed_gpu(abort_flag)) return false;
-        __nanosleep(64);
-    }
-    atomicExch(abort_flag, 1);
-    atomicOr(err, 1);
-    return false;
-}
-
-// Published pivot-tile values: every slot starts as the all-ones bit pattern
-// (a NaN that arithmetic never produces), and a producer stores final values
-// only (aligned 8-byte stores are single-copy atomic), so a consumer that
-// sees no sentinel has the data: one round trip instead of flag then data.
-// All threads poll together (uniform result): the warps that hold slot
-// elements spin on their own elements (a warp vote per round, no block
-// barrier, a short sleep and an abort check every 32 rounds), the others go
-// straight to the closing barrier; iteration limit as wait_flag.
+// Published values.  Everything that one task of a launch hands to another
+// -- a front's update rows, a pivot tile's solution, the backward partial sums,
+// the solution rows -- sits in words preset to the all-ones bit pattern (a NaN
+// that arithmetic never produces), and a producer stores final values only
+// (aligned 8-byte stores are single-copy atomic), so a consumer that sees no
+// sentinel has the data: one trip through L2 hands a value over, where a
+// fence, a counter and a poll of it took three.  A chain of one-column fronts of
+// 5 rows, FP64: 0.7 + 1.0 us per front forward and backward (4.8 + 4.1 with
+// counters); 24 x 23 grid 203 + 159 us -> 32 + 32; 333 x 257 grid FP32, three
+// right-hand sides 0.97 + 0.85 ms -> 0.35 + 0.44.
 __device__ __forceinline__ double ld_relaxed_f64(const double* p) {
     double v;
     asm volatile("ld.relaxed.gpu.global.f64 %0, [%1];" : "=d"(v) : "l"(p) : "memory");
@@ -100,9 +73,19 @@ __device__ __forceinline__ void st_relaxed_f64(double* p, double v) {
 __device__ __forceinline__ bool is_unpublished(double v) {
     return __double_as_longlong(v) == -1ll;
 }
+struct SolveAbort {
+    int* flag;
+    int* err;
+};
+
+// All threads of the CTA poll a slot together (uniform result): the warps that
+// hold slot elements spin on their own elements (a warp vote per round, no
+// block barrier, a short sleep and an abort check every 32 rounds), the others
+// go straight to the closing barrier; with an iteration limit, after which the
+// launch is aborted and the error word set.
 // (src: the slot, column after column of 64 rows; dst: columns kVecLD apart)
-__device__ bool poll_published(double* dst, const double* src, int nk, int nrhs, int* abort_flag,
-                               int* err) {
+__device__ bool poll_published(double* dst, const double* src, int nk, int nrhs,
+                               const SolveAbort& ab) {
     constexpr int T = kTile;
     const int total = T * nrhs, lane = threadIdx.x & 31;  // total: a multiple of 64
     bool ok = true;
@@ -115,14 +98,14 @@ __device__ bool poll_published(double* dst, const double* src, int nk, int nrhs,
             if (__all_sync(0xffffffffu, !need || !is_unpublished(v))) break;
             if (it + 1 >= kSolveWaitPolls) {
                 if (lane == 0) {
-                    atomicExch(abort_flag, 1);
-                    atomicOr(err, 1);
+                    atomicExch(ab.flag, 1);
+                    atomicOr(ab.err, 1);
                 }
                 ok = false;
                 break;
             }
             if ((it & 31) == 31) {
-                const int a = lane == 0 ? ld_relaxed_gpu(abort_flag) : 0;
+                const int a = lane == 0 ? ld_relaxed_gpu(ab.flag) : 0;
                 if (__shfl_sync(0xffffffffu, a, 0)) {
                     ok = false;
                     break;
@@ -135,14 +118,95 @@ __device__ bool poll_published(double* dst, const double* src, int nk, int nrhs,
     return __syncthreads_and(ok);
 }
 
-template <typename TL>
-__device__ __forceinline__ void cp_async_elem(TL* dst, const TL* src) {
-    const uint32_t d = static_cast<uint32_t>(__cvta_generic_to_shared(dst));
-    if constexpr (sizeof(TL) == 4)
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(d), "l"(src) : "memory");
-    else
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(d), "l"(src) : "memory");
+// NQ neighbouring published values p[0 .. nq - 1]: a first look (the loads of
+// several places are issued together), then the wait for the ones not there
+// yet, each thread for its own, with a short sleep between the looks.
+template <int NQ>
+__device__ __forceinline__ void peek_values(const double* p, bool need, int nq, double (&v)[NQ]) {
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) {
+        v[q] = 0.0;
+        if (need && q < nq) v[q] = ld_relaxed_f64(p + q);
+    }
 }
+template <int NQ>
+__device__ __forceinline__ void await_values(const double* p, int nq, double (&v)[NQ],
+                                             const SolveAbort& ab) {
+    for (int it = 1;; ++it) {
+        bool miss = false;
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) miss = miss || is_unpublished(v[q]);
+        if (!miss) return;
+        if (it > 2) __nanosleep(it < 64 ? 40 : 200);
+        if ((it & 15) == 0) {
+            if (it >= kSolveWaitPolls) {
+                atomicExch(ab.flag, 1);
+                atomicOr(ab.err, 1);
+            }
+            if (ld_relaxed_gpu(ab.flag)) return;
+        }
+#pragma unroll
+        for (int q = 0; q < NQ; ++q)
+            if (is_unpublished(v[q])) v[q] = ld_relaxed_f64(p + q);
+    }
+}
+
+// The same for the lanes of `mask` together (converged), each with values from
+// R places: the rounds are uniform, so the lanes leave converged.  After loops
+// of their own lanes ran the rest of a front in pieces, also past a
+// __syncwarp, and every shuffle waited about 500 cycles for the pieces to meet
+// (8 us per front in the chain above).  at(k): place k, which a lane needs
+// where v[k] is unpublished.
+template <int R, int NQ, typename F>
+__device__ __forceinline__ void await_together(F&& at, int nq, double (&v)[R][NQ], unsigned mask,
+                                               const SolveAbort& ab) {
+    for (int it = 1;; ++it) {
+        bool miss = false;
+#pragma unroll
+        for (int k = 0; k < R; ++k)
+#pragma unroll
+            for (int q = 0; q < NQ; ++q) miss = miss || is_unpublished(v[k][q]);
+        if (!__any_sync(mask, miss)) return;
+        if (it > 2) __nanosleep(it < 64 ? 40 : 200);
+        if ((it & 15) == 0) {
+            if (miss && it >= kSolveWaitPolls) {
+                atomicExch(ab.flag, 1);
+                atomicOr(ab.err, 1);
+            }
+            if (__any_sync(mask, ld_relaxed_gpu(ab.flag))) return;
+        }
+#pragma unroll
+        for (int k = 0; k < R; ++k)
+#pragma unroll
+            for (int q = 0; q < NQ; ++q)
+                if (is_unpublished(v[k][q])) v[k][q] = ld_relaxed_f64(at(k) + q);
+    }
+}
+
+// four neighbouring elements on 16 bytes
+__device__ __forceinline__ void ld4(const float* p, float (&v)[4]) {
+    const float4 a = *reinterpret_cast<const float4*>(p);
+    v[0] = a.x, v[1] = a.y, v[2] = a.z, v[3] = a.w;
+}
+__device__ __forceinline__ void ld4(const double* p, double (&v)[4]) {
+    const double2 a = *reinterpret_cast<const double2*>(p);
+    const double2 b = *reinterpret_cast<const double2*>(p + 2);
+    v[0] = a.x, v[1] = a.y, v[2] = b.x, v[3] = b.y;
+}
+
+// Backward, update-row gathers: the solution rows of a front's ancestors are
+// final once its parent's first pivot row (at global column pcol; none for a
+// root) is: a large front publishes its tiles from the last, and the rows above
+// the parent came before it.  One warp waits for that row, as many gathers wait
+// for the same few.
+__device__ __forceinline__ void await_parent(int pcol, const double* xs, int nrhs,
+                                             const SolveAbort& ab) {
+    if (pcol < 0) return;
+    const double* p = xs + (int64_t)pcol * nrhs;
+    double v[1][1] = {{ld_relaxed_f64(p)}};
+    await_together<1, 1>([&](int) { return p; }, 1, v, 0xffffffffu, ab);
+}
+
 __device__ __forceinline__ void cp_async_commit_group() {
     asm volatile("cp.async.commit_group;" ::: "memory");
 }
@@ -245,7 +309,7 @@ __device__ __forceinline__ void load_slot_async(double* dst, const double* src, 
 // the sentinel; an unpublished row sends the CTA to poll the slot.  Uniform
 // result; false = the solve was aborted.
 __device__ __forceinline__ bool settle_slot(double* v, const double* src, int nk, int nrhs,
-                                            int* abort_flag, int* err) {
+                                            const SolveAbort& ab) {
     bool mine = true;
     for (int e = threadIdx.x; e < kTile * nrhs; e += blockDim.x) {
         double& x = v[(e / kTile) * kVecLD + (e & (kTile - 1))];
@@ -255,7 +319,28 @@ __device__ __forceinline__ bool settle_slot(double* v, const double* src, int nk
             mine = false;
     }
     if (__syncthreads_and(mine)) return true;
-    return poll_published(v, src, nk, nrhs, abort_flag, err);
+    return poll_published(v, src, nk, nrhs, ab);
+}
+
+// x[q] += the front-vector rows that the assembly map adds into a row (fv row
+// e at fv + e * nrhs; NQ neighbouring right-hand sides), in child order, every
+// entry waited for, two in flight.  ar: the row's entry range.
+template <int NQ>
+__device__ __forceinline__ void gather_entries(const int* ar, const int* __restrict__ amap_ent,
+                                               const double* fv, int nrhs, int nq, double (&x)[NQ],
+                                               const SolveAbort& ab) {
+    const int e1 = ar[1];
+    for (int e = ar[0]; e < e1; e += 2) {
+        const double* p0 = fv + (int64_t)amap_ent[e] * nrhs;
+        const double* p1 = e + 1 < e1 ? fv + (int64_t)amap_ent[e + 1] * nrhs : p0;
+        double v[NQ], w[NQ];
+        peek_values<NQ>(p0, true, nq, v);
+        peek_values<NQ>(p1, e + 1 < e1, nq, w);
+        await_values<NQ>(p0, nq, v, ab);
+        await_values<NQ>(p1, nq, w, ab);
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) x[q] = (x[q] + v[q]) + w[q];
+    }
 }
 
 // Forward, task (s, i0 | cnt << 16): row tiles i0 .. i0 + cnt - 1 of front s.
@@ -269,8 +354,8 @@ __device__ __forceinline__ bool settle_slot(double* v, const double* src, int nk
 // warp (rows 8w .. 8w + 7 of warp w), so a row's sum is two shuffles.
 template <typename TL>
 __device__ void fwd_tile_task(int2 tk, const FrontDesc* __restrict__ fronts,
-                              double* __restrict__ pub, int* __restrict__ abort_flag,
-                              int* __restrict__ err, const int64_t* __restrict__ fv_off,
+                              double* __restrict__ pub, const SolveAbort& ab,
+                              const int64_t* __restrict__ fv_off,
                               const int* __restrict__ amap_off, const int* __restrict__ amap_row,
                               const int* __restrict__ amap_ent,
                               const int64_t* __restrict__ dinv_off, const TL* __restrict__ Ls,
@@ -294,15 +379,15 @@ __device__ void fwd_tile_task(int2 tk, const FrontDesc* __restrict__ fronts,
     // update tiles)
     const int db = blk_off<TL>(tile_range(i0, F.m, F.c, T).start);
     const int aoff = amap_off[s];
-    // this thread's row of tile i of the front vector
+    // this thread's row of tile i of the front vector (after an abort what is
+    // gathered and published no longer matters, and every later wait returns)
     auto gather_row = [&](int i) -> double {
         const TileRange ti = tile_range(i, F.m, F.c, T);
         const int R = ti.start + r;
         if (g != 0 || r >= ti.size) return 0.0;
-        double x = R < F.c ? xp[F.first_col + R] : 0.0;
-        const int e1 = amap_row[aoff + R + 1];
-        for (int e = amap_row[aoff + R]; e < e1; ++e) x += __ldcg(fv + (int64_t)amap_ent[e]);
-        return x;
+        double x[1] = {R < F.c ? xp[F.first_col + R] : 0.0};
+        gather_entries<1>(amap_row + aoff + R, amap_ent, fv, 1, 1, x, ab);
+        return x[0];
     };
     auto issue = [&](int p) {
         if (p < P) {
@@ -328,7 +413,7 @@ __device__ void fwd_tile_task(int2 tk, const FrontDesc* __restrict__ fronts,
         __syncthreads();
         const int i = i0 + p / kend, k = p % kend;
         double* Yk = sm.vb(p);
-        if (!settle_slot(Yk, pb + (int64_t)k * T, min(T, F.c - k * T), 1, abort_flag, err)) {
+        if (!settle_slot(Yk, pb + (int64_t)k * T, min(T, F.c - k * T), 1, ab)) {
             ok = false;
             break;
         }
@@ -339,7 +424,7 @@ __device__ void fwd_tile_task(int2 tk, const FrontDesc* __restrict__ fronts,
             const TileRange ti = tile_range(i, F.m, F.c, T);
             double v = acc + __shfl_xor_sync(0xffffffffu, acc, 8);
             v += __shfl_xor_sync(0xffffffffu, v, 16);
-            if (g == 0 && r < ti.size) f[ti.start + r] = fcur - v;
+            if (g == 0 && r < ti.size) st_relaxed_f64(f + ti.start + r, fcur - v);
             acc = 0.0;
             fcur = fnext;
             if (i + 2 < i0 + cnt) fnext = gather_row(i + 2);
@@ -406,13 +491,13 @@ __device__ __forceinline__ void group_product(const TL* B, int db, const double*
 // the group's own).
 template <typename TL>
 __device__ void fwd_tile_group(int2 tk, const FrontDesc* __restrict__ fronts,
-                               double* __restrict__ pub, int* __restrict__ abort_flag,
-                               int* __restrict__ err, const int64_t* __restrict__ fv_off,
+                               double* __restrict__ pub, const SolveAbort& ab,
+                               const int64_t* __restrict__ fv_off,
                                const int* __restrict__ amap_off, const int* __restrict__ amap_row,
                                const int* __restrict__ amap_ent,
                                const int64_t* __restrict__ dinv_off, const TL* __restrict__ Ls,
                                const TL* __restrict__ Dinv, double* __restrict__ xp,
-                               double* __restrict__ fv, int n, int nrhs) {
+                               double* __restrict__ fv, int nrhs) {
     constexpr int T = kTile;
     const LevelSmem<TL, true> sm;
     const int r = threadIdx.x >> 2, q = 2 * (threadIdx.x & 3);
@@ -434,15 +519,11 @@ __device__ void fwd_tile_group(int2 tk, const FrontDesc* __restrict__ fronts,
         v[0] = v[1] = 0.0;
         if (r >= ti.size || !q0) return;
         if (R < F.c) {
-            v[0] = xp[F.first_col + R + (int64_t)q * n];
-            if (q1) v[1] = xp[F.first_col + R + (int64_t)(q + 1) * n];
+            const double* x = xp + (int64_t)(F.first_col + R) * nrhs + q;
+            v[0] = x[0];
+            if (q1) v[1] = x[1];
         }
-        const int e1 = amap_row[aoff + R + 1];
-        for (int e = amap_row[aoff + R]; e < e1; ++e) {
-            const double* w = fv + (int64_t)amap_ent[e] * nrhs + q;
-            v[0] += __ldcg(w);
-            if (q1) v[1] += __ldcg(w + 1);
-        }
+        gather_entries<2>(amap_row + aoff + R, amap_ent, fv + q, nrhs, q1 ? 2 : 1, v, ab);
     };
     auto issue = [&](int p) {
         if (p < P) {
@@ -467,8 +548,7 @@ __device__ void fwd_tile_group(int2 tk, const FrontDesc* __restrict__ fronts,
         cp_async_wait_groups<1>();
         __syncthreads();
         const int i = i0 + p / kend, k = p % kend;
-        if (!settle_slot(sm.vb(p), pb + (int64_t)k * T * nrhs, min(T, F.c - k * T), nrhs,
-                         abort_flag, err)) {
+        if (!settle_slot(sm.vb(p), pb + (int64_t)k * T * nrhs, min(T, F.c - k * T), nrhs, ab)) {
             ok = false;
             break;
         }
@@ -477,8 +557,8 @@ __device__ void fwd_tile_group(int2 tk, const FrontDesc* __restrict__ fronts,
             const TileRange ti = tile_range(i, F.m, F.c, T);
             if (r < ti.size) {
                 double* o = f + (int64_t)(ti.start + r) * nrhs + q;
-                if (q0) o[0] = fcur[0] - (acc[0][0] + acc[1][0]);
-                if (q1) o[1] = fcur[1] - (acc[0][1] + acc[1][1]);
+                if (q0) st_relaxed_f64(o, fcur[0] - (acc[0][0] + acc[1][0]));
+                if (q1) st_relaxed_f64(o + 1, fcur[1] - (acc[0][1] + acc[1][1]));
             }
 #pragma unroll
             for (int j = 0; j < 2; ++j) {
@@ -501,11 +581,11 @@ __device__ void fwd_tile_group(int2 tk, const FrontDesc* __restrict__ fronts,
     if (in) {
         double* o = pb + (int64_t)i0 * nrhs * T + r;
         if (q0) {
-            xp[F.first_col + ti.start + r + (int64_t)q * n] = y[0][0] + y[1][0];
+            xp[(int64_t)(F.first_col + ti.start + r) * nrhs + q] = y[0][0] + y[1][0];
             st_relaxed_f64(o + q * T, y[0][0] + y[1][0]);
         }
         if (q1) {
-            xp[F.first_col + ti.start + r + (int64_t)(q + 1) * n] = y[0][1] + y[1][1];
+            xp[(int64_t)(F.first_col + ti.start + r) * nrhs + q + 1] = y[0][1] + y[1][1];
             st_relaxed_f64(o + (q + 1) * T, y[0][1] + y[1][1]);
         }
     }
@@ -514,18 +594,17 @@ __device__ void fwd_tile_group(int2 tk, const FrontDesc* __restrict__ fronts,
 // Backward, update rows, task (s, j | h << 16): the partial sum
 // L(k, j)' x_k over the update row tiles k of chunk h (kGatherTiles tiles;
 // x final: ancestors, read through the row list) for pivot column tile j,
-// written as a T x nrhs vector for the pivot task to add in chunk order, then
-// counted in.  MULTI: a group of nrhs <= 8 right-hand sides on the matrix
+// published as a T x nrhs vector for the pivot task to add in chunk order.
+// MULTI: a group of nrhs <= 8 right-hand sides on the matrix
 // instructions; one: warp w takes columns 8w .. 8w + 7, lane (c1 = column,
 // q1 = row phase) the rows q1, q1 + 4, ...: conflict-free reads of the stage
 // layout, the phases summed by shuffles.
 template <typename TL, bool MULTI>
 __device__ void bwd_gather_task(int2 tk, const FrontDesc* __restrict__ fronts,
                                 const int* __restrict__ rows, const int* __restrict__ gather_nch,
-                                const int* __restrict__ gather_off, int* __restrict__ gcount,
-                                const int64_t* __restrict__ dinv_off, const TL* __restrict__ Ls,
-                                const double* __restrict__ xp, double* __restrict__ part, int n,
-                                int nrhs) {
+                                const int* __restrict__ gather_off, const SolveAbort& ab,
+                                const TL* __restrict__ Ls, const double* __restrict__ xs,
+                                double* __restrict__ part, int nrhs) {
     constexpr int T = kTile, LD = blk_ld<TL>(), GC = SolveScheduleHost::kGatherTiles;
     const LevelSmem<TL, MULTI> sm;
     const int tid = threadIdx.x;
@@ -545,32 +624,7 @@ __device__ void bwd_gather_task(int2 tk, const FrontDesc* __restrict__ fronts,
         const int rr = e & (T - 1);
         sm.idx[e] = rr < tkr.size ? rw[tkr.start + rr] : -1;
     }
-    __syncthreads();
-    // two stages: the L blocks by cp.async; the ancestors' solution rows
-    // (written in this launch) through L2 into registers one stage ahead,
-    // stored into their stage after the previous stage's products
-    constexpr int VPT = MULTI ? kTile * kGroupRhs / 256 : 1;
-    double pend[VPT];
-    auto fetch = [&](int p) {
-#pragma unroll
-        for (int k = 0; k < VPT; ++k) {
-            const int e = tid + 256 * k;
-            pend[k] = 0.0;
-            if (p < P && e < T * nrhs) {
-                const int row = sm.idx[p * T + (e & (T - 1))], q = e / T;
-                if (row >= 0) pend[k] = __ldcg(xp + row + (int64_t)q * n);
-            }
-        }
-    };
-    auto put = [&](int p) {
-        if (p >= P) return;
-        double* v = sm.vb(p);
-#pragma unroll
-        for (int k = 0; k < VPT; ++k) {
-            const int e = tid + 256 * k;
-            if (e < T * nrhs) v[(e / T) * kVecLD + (e & (T - 1))] = pend[k];
-        }
-    };
+    const int pcol = F.parent >= 0 ? fronts[F.parent].first_col : -1;
     auto issue = [&](int p) {
         if (p < P) {
             const TileRange tkr = tile_range(k0 + p, F.m, F.c, T);
@@ -578,8 +632,36 @@ __device__ void bwd_gather_task(int2 tk, const FrontDesc* __restrict__ fronts,
         }
         cp_async_commit_group();
     };
-    static_assert(kSolveStages == 2, "the gather's vector pipeline has two stages");
     issue(0);
+    if (tid < 32) await_parent(pcol, xs, nrhs, ab);
+    __syncthreads();
+    // two stages: the L blocks by cp.async; the ancestors' solution rows, as
+    // they are published, into registers one stage ahead, stored into their
+    // stage after the previous stage's products
+    constexpr int VPT = MULTI ? kTile * kGroupRhs / 256 : 1;
+    double pend[VPT][1];
+    auto fetch = [&](int p) {
+        const double* src[VPT];
+#pragma unroll
+        for (int k = 0; k < VPT; ++k) {
+            const int e = tid + 256 * k;
+            const int row = p < P && e < T * nrhs ? sm.idx[p * T + (e & (T - 1))] : -1;
+            src[k] = xs + (int64_t)max(row, 0) * nrhs + e / T;
+            peek_values<1>(src[k], row >= 0, 1, pend[k]);
+        }
+#pragma unroll
+        for (int k = 0; k < VPT; ++k) await_values<1>(src[k], 1, pend[k], ab);
+    };
+    auto put = [&](int p) {
+        if (p >= P) return;
+        double* v = sm.vb(p);
+#pragma unroll
+        for (int k = 0; k < VPT; ++k) {
+            const int e = tid + 256 * k;
+            if (e < T * nrhs) v[(e / T) * kVecLD + (e & (T - 1))] = pend[k][0];
+        }
+    };
+    static_assert(kSolveStages == 2, "the gather's vector pipeline has two stages");
     fetch(0);
     put(0);
     double acc[2][2] = {};
@@ -604,340 +686,305 @@ __device__ void bwd_gather_task(int2 tk, const FrontDesc* __restrict__ fronts,
     double* out = part + ((int64_t)gather_off[s] + (int64_t)j * gather_nch[s] + h) * T * nrhs;
     if constexpr (MULTI) {
         const int l = tid >> 2, q = 2 * (tid & 3);
-        if (q < nrhs) out[l + T * q] = acc[0][0] + acc[1][0];
-        if (q + 1 < nrhs) out[l + T * (q + 1)] = acc[0][1] + acc[1][1];
+        if (q < nrhs) st_relaxed_f64(out + l + T * q, acc[0][0] + acc[1][0]);
+        if (q + 1 < nrhs) st_relaxed_f64(out + l + T * (q + 1), acc[0][1] + acc[1][1]);
     } else {
         double v = acc[0][0] + __shfl_xor_sync(0xffffffffu, acc[0][0], 8);
         v += __shfl_xor_sync(0xffffffffu, v, 16);
-        if (q1 == 0) out[c1] = v;
-    }
-    // count this chunk in for the pivot task (s, j): the CTA's stores, then
-    // a device-scope fence, then the increment
-    __syncthreads();
-    if (tid == 0) {
-        __threadfence();
-        atomicAdd(gcount + dinv_off[s] / (T * T) + j, 1);
+        if (q1 == 0) st_relaxed_f64(out + c1, v);
     }
 }
 
 // ---------------------------------------------------------------------------
-// small fronts: a warp per front, the right-hand sides in passes of NQ
-// (kWarpSolveRhs, or one), lane l holding rows l, l + 32, ... (R slots,
-// m <= 32 R) of the pass's right-hand sides in registers.  Forward: the
-// pivot value is broadcast by a shuffle and every lane updates its rows
-// below it; backward: a warp reduction per pivot column (dot product with
-// the final rows below it).  No block barriers; the children's update parts
-// are summed into a per-warp shared buffer (child by child, deterministic)
-// before the rows are taken into registers.
+// small fronts: a group of W lanes per front (W = 32: fronts of up to 160
+// rows, lane r holding rows r, r + 32, ... in R slots; W = 16, 8: one row per
+// lane, two and four fronts per warp), the right-hand sides in passes of NQ.
+// No block barriers.  Everything that does not depend on other fronts -- the
+// children's places in the front vector, the first columns of L, the
+// reciprocals of the pivots -- is loaded before the first wait, and the
+// columns of L a chunk at a time after it: the chain from a front's children to
+// its own values is one trip through L2, the assembly, and about 50 cycles per
+// pivot column (a shuffle and two FP64 operations) plus a load per chunk.
 // ---------------------------------------------------------------------------
 
-// Dependency words of the one-launch solve.  Forward: front s starts once
-// done[s] (its finished children) reaches its child count, and counts
-// itself in at its parent once its update rows are written.  Backward:
-// front s starts once done[parent] reaches target[parent] (the parent's
-// solution rows are final), and counts one completion of its own once its
-// solution rows are written.  Data written inside the launch by other CTAs
-// (children's update rows, ancestors' solution rows) are read through L2.
-struct FrontDeps {
-    int* done;
-    const int* target;  // backward only
-    int* abort_flag;
-    int* err;
-};
+template <int N>
+using Int = std::integral_constant<int, N>;
 
-// Fronts of at most W rows (W = 8, 16, 32) on a group of W lanes of a warp
-// (32 / W fronts per warp), one row per lane.  mask: the group's lanes; the
-// group's rows of the warp buffer are wbuf[q * 32 + r].
 template <int W>
 __device__ __forceinline__ unsigned group_mask() {
     return W == 32 ? 0xffffffffu : (((1u << W) - 1u) << ((threadIdx.x & 31) & ~(W - 1)));
 }
 
-// the group's first lane waits (bounded) for *word >= target; uniform result
-template <int W>
-__device__ __forceinline__ bool group_wait(const int* word, int target, const FrontDeps& d,
-                                           unsigned mask) {
-    int ok = 1;
-    if ((threadIdx.x & (W - 1)) == 0) ok = wait_flag(word, target, d.abort_flag, d.err) ? 1 : 0;
-    return __shfl_sync(mask, ok, 0, W) != 0;
+// columns of L taken at a time and the right-hand sides of a pass, by the
+// registers they take (R chunk elements of L, R NQ values)
+template <int R, int NQ>
+constexpr int solve_chunk() {
+    return R == 1 ? (NQ == 1 ? 8 : 4) : NQ == 1 ? 4 : 2;
 }
-// every lane's stores, a device-scope fence, then one increment of *word
-template <int W>
-__device__ __forceinline__ void group_signal(int* word, unsigned mask) {
-    __threadfence();
-    __syncwarp(mask);
-    if (word && (threadIdx.x & (W - 1)) == 0) atomicAdd(word, 1);
+template <int R, bool MULTI>
+constexpr int solve_pass() {
+    return !MULTI ? 1 : R == 1 ? kGroupRhs : 2;
 }
-
-template <typename TL, typename TV, int W, int NQ>
-__device__ void fwd_group_front(int s, const FrontDesc& F, const FrontDeps& deps,
-                                const FrontDesc* __restrict__ fronts,
-                                const int* __restrict__ child, const int* __restrict__ relmap,
-                                const int64_t* __restrict__ fv_off, const TL* __restrict__ Ls,
-                                TV* __restrict__ xp, TV* __restrict__ out, TV* __restrict__ fv,
-                                int n, int nrhs, TV* wbuf) {
+// Forward.  buf: the group's shared rows, row r of right-hand side q at
+// buf[32 R q + r]; rds: its reciprocals.
+template <typename TL, int W, int R, int NQ>
+__device__ void fwd_front(int s, const FrontDesc& F, const SolveAbort& ab,
+                          const FrontDesc* __restrict__ fronts, const int* __restrict__ child,
+                          const int* __restrict__ relmap, const int64_t* __restrict__ fv_off,
+                          const TL* __restrict__ Ls, double* __restrict__ xp,
+                          double* __restrict__ fv, int nrhs, double* buf, double* rds) {
+    static_assert(W == 32 || R == 1, "several rows per lane only on whole warps");
+    constexpr int stride = 32 * R;
+    constexpr int CH = solve_chunk<R, NQ>(), PC = R == 1 && NQ == 1 ? 2 : 1;
     const unsigned mask = group_mask<W>();
-    if (!group_wait<W>(deps.done + s, F.child_end - F.child_beg, deps, mask)) return;
-    const int r = threadIdx.x & (W - 1);
-    const int m = F.m, c = F.c;
+    const int lane = threadIdx.x & (W - 1);
+    const int m = F.m, c = F.c, nch = F.child_end - F.child_beg;
     const int64_t ldl = F.ldl;
     const TL* L = Ls + F.loff;
+    double* out = front_vec(fv, fv_off, s, nrhs);
+    for (int r = lane; r < c; r += W) rds[r] = 1.0 / (double)L[r + r * ldl];
+    // PC children from the h-th on: their rows' places in this front
+    int pc[PC][R];
+    const double* wp[PC];
+    auto children = [&](int h) {
+#pragma unroll
+        for (int e = 0; e < PC; ++e) {
+            const bool has = h + e < nch;
+            const int ch = has ? child[F.child_beg + h + e] : s;
+            const int gc = fronts[ch].c, uc = has ? fronts[ch].m - gc : 0;
+            const int* rm = relmap + fronts[ch].rows_off + gc;
+            wp[e] = front_vec(fv, fv_off, ch, nrhs) + (int64_t)gc * nrhs;
+#pragma unroll
+            for (int k = 0; k < R; ++k) {
+                const int r = lane + W * k;
+                pc[e][k] = -1;
+                if (r < uc) pc[e][k] = rm[r];
+            }
+        }
+    };
+    TL l[R][CH];
+    auto columns = [&](int j0) {
+#pragma unroll
+        for (int cc = 0; cc < CH; ++cc)
+#pragma unroll
+            for (int k = 0; k < R; ++k) {
+                const int r = lane + W * k, j = j0 + cc;
+                l[k][cc] = TL(0);
+                if (r > j && r < m && j < c) l[k][cc] = L[r + j * ldl];
+            }
+    };
+    children(0);
     for (int q0 = 0; q0 < nrhs; q0 += NQ) {
         const int nq = min(NQ, nrhs - q0);
+        columns(0);
 #pragma unroll
-        for (int q = 0; q < NQ; ++q)
-            if (q < nq && r < m)
-                wbuf[q * 32 + r] = r < c ? xp[F.first_col + r + (int64_t)(q0 + q) * n] : TV(0);
+        for (int k = 0; k < R; ++k) {
+            const int r = lane + W * k;
+#pragma unroll
+            for (int q = 0; q < NQ; ++q)
+                if (r < m && q < nq)
+                    buf[q * stride + r] =
+                        r < c ? xp[(int64_t)(F.first_col + r) * nrhs + q0 + q] : 0.0;
+        }
         __syncwarp(mask);
-        for (int h = F.child_beg; h < F.child_end; ++h) {  // children in order
-            const int ch = child[h];
-            const FrontDesc g = fronts[ch];
-            const int uc = g.m - g.c;
-            const TV* w = front_vec(fv, fv_off, ch, nrhs) + g.c * nrhs + q0;
-            if (r < uc) {  // uc < m <= W
-                const int p = relmap[g.rows_off + g.c + r];
+        for (int h = 0; h < nch; h += PC) {  // children in order
+            if (h > 0 || (q0 > 0 && nch > PC)) children(h);
+            double w[PC][R][NQ];
+            auto at = [&](int e, int k) { return wp[e] + (int64_t)(lane + W * k) * nrhs + q0; };
 #pragma unroll
-                for (int q = 0; q < NQ; ++q)
-                    if (q < nq) wbuf[q * 32 + p] += __ldcg(w + r * nrhs + q);
+            for (int e = 0; e < PC; ++e)
+#pragma unroll
+                for (int k = 0; k < R; ++k) peek_values<NQ>(at(e, k), pc[e][k] >= 0, nq, w[e][k]);
+#pragma unroll
+            for (int e = 0; e < PC; ++e) {
+                await_together<R, NQ>([&](int k) { return at(e, k); }, nq, w[e], mask, ab);
+#pragma unroll
+                for (int k = 0; k < R; ++k) {
+                    if (pc[e][k] >= 0)
+#pragma unroll
+                        for (int q = 0; q < NQ; ++q)
+                            if (q < nq) buf[q * stride + pc[e][k]] += w[e][k][q];
+                }
+                __syncwarp(mask);
             }
-            __syncwarp(mask);
         }
-        TV v[NQ];
+        double v[R][NQ];
 #pragma unroll
-        for (int q = 0; q < NQ; ++q) v[q] = (q < nq && r < m) ? wbuf[q * 32 + r] : TV(0);
+        for (int k = 0; k < R; ++k)
+#pragma unroll
+            for (int q = 0; q < NQ; ++q)
+                v[k][q] = (q < nq && lane + W * k < m) ? buf[q * stride + lane + W * k] : 0.0;
         __syncwarp(mask);
-        // column j of L for this lane's row, one column ahead of its use
-        TV lc = (r > 0 && r < m) ? (TV)L[r] : TV(0), d = (TV)L[0];
-        for (int j = 0; j < c; ++j) {
-            TV ln = TV(0), dn = TV(1);
-            if (j + 1 < c) {
-                const TL* cn = L + (j + 1) * ldl;
-                dn = (TV)cn[j + 1];
-                ln = (r > j + 1 && r < m) ? (TV)cn[r] : TV(0);
-            }
-            // several right-hand sides: one reciprocal per column
-            const TV rd = NQ > 1 ? TV(1) / d : TV(0);
 #pragma unroll
-            for (int q = 0; q < NQ; ++q) {
-                const TV sv = __shfl_sync(mask, v[q], j, W);
-                const TV y = NQ > 1 ? sv * rd : sv / d;
-                if (r == j)
-                    v[q] = y;
-                else if (r > j)
-                    v[q] -= lc * y;
-            }
-            lc = ln;
-            d = dn;
-        }
+        for (int ks = 0; ks < R; ++ks) {  // pivot columns W ks .. W ks + W - 1
+            for (int j0 = W * ks; j0 < min(c, W * (ks + 1)); j0 += CH) {
+                if (j0 > 0) columns(j0);
 #pragma unroll
-        for (int q = 0; q < NQ; ++q) {
-            if (q >= nq || r >= m) continue;
-            if (r < c)
-                xp[F.first_col + r + (int64_t)(q0 + q) * n] = v[q];
-            else
-                out[r * nrhs + q0 + q] = v[q];
-        }
-    }
-    group_signal<W>(F.parent >= 0 ? deps.done + F.parent : nullptr, mask);
-}
-
-template <typename TL, typename TV, int W, int NQ>
-__device__ void bwd_group_front(int s, const FrontDesc& F, const FrontDeps& deps,
-                                const int* __restrict__ rows, const TL* __restrict__ Ls,
-                                TV* __restrict__ xp, int n, int nrhs) {
-    const unsigned mask = group_mask<W>();
-    if (F.parent >= 0 && !group_wait<W>(deps.done + F.parent, deps.target[F.parent], deps, mask))
-        return;
-    const int r = threadIdx.x & (W - 1);
-    const int m = F.m, c = F.c;
-    const int64_t ldl = F.ldl;
-    const TL* L = Ls + F.loff;
-    // this lane's row in the solution: a pivot row, else an ancestor's
-    const int src = r < c ? F.first_col + r : (r < m ? rows[F.rows_off + r] : 0);
-    for (int q0 = 0; q0 < nrhs; q0 += NQ) {
-        const int nq = min(NQ, nrhs - q0);
-        TV v[NQ];  // y on the pivot rows (x once solved), final x on the others
+                for (int cc = 0; cc < CH; ++cc) {
+                    const int j = j0 + cc - W * ks;  // the pivot's lane
+                    if (j0 + cc >= c) break;
+                    const double rj = rds[j0 + cc];
 #pragma unroll
-        for (int q = 0; q < NQ; ++q)
-            v[q] = (q < nq && r < m) ? __ldcg(xp + src + (int64_t)(q0 + q) * n) : TV(0);
-        const int jl = c - 1;
-        TV lc = (r > jl && r < m) ? (TV)L[r + jl * ldl] : TV(0), d = (TV)L[jl + jl * ldl];
-        for (int j = jl; j >= 0; --j) {
-            TV ln = TV(0), dn = TV(1);
-            if (j > 0) {
-                const TL* cn = L + (j - 1) * ldl;
-                dn = (TV)cn[j - 1];
-                ln = (r > j - 1 && r < m) ? (TV)cn[r] : TV(0);
-            }
-            TV p[NQ];
+                    for (int q = 0; q < NQ; ++q) {
+                        const double y = __shfl_sync(mask, v[ks][q], j, W) * rj;
 #pragma unroll
-            for (int q = 0; q < NQ; ++q) p[q] = lc * v[q];
-#pragma unroll
-            for (int o = W / 2; o > 0; o >>= 1)
-#pragma unroll
-                for (int q = 0; q < NQ; ++q) p[q] += __shfl_xor_sync(mask, p[q], o, W);
-            if (r == j) {
-#pragma unroll
-                for (int q = 0; q < NQ; ++q) v[q] = (v[q] - p[q]) / d;
-            }
-            lc = ln;
-            d = dn;
-        }
-#pragma unroll
-        for (int q = 0; q < NQ; ++q)
-            if (q < nq && r < c) xp[F.first_col + r + (int64_t)(q0 + q) * n] = v[q];
-    }
-    group_signal<W>(deps.done + s, mask);
-}
-
-// Fronts of 33..160 rows: the same sweeps with the front vector kept in the
-// warp's shared buffer (ld MR rows per right-hand side) instead of registers.
-template <typename TL, typename TV, int NQ>
-__device__ void fwd_warp_front_smem(int s, const FrontDesc& F, const FrontDeps& deps,
-                                    const FrontDesc* __restrict__ fronts,
-                                    const int* __restrict__ child, const int* __restrict__ relmap,
-                                    const int64_t* __restrict__ fv_off, const TL* __restrict__ Ls,
-                                    TV* __restrict__ xp, TV* __restrict__ out, TV* __restrict__ fv,
-                                    int n, int nrhs, TV* f, int MR) {
-    if (!group_wait<32>(deps.done + s, F.child_end - F.child_beg, deps, 0xffffffffu)) return;
-    const int lane = threadIdx.x & 31;
-    const int m = F.m, c = F.c;
-    const int64_t ldl = F.ldl;
-    const TL* L = Ls + F.loff;
-    for (int q0 = 0; q0 < nrhs; q0 += NQ) {
-        const int nq = min(NQ, nrhs - q0);
-        for (int r = lane; r < m; r += 32)
-#pragma unroll
-            for (int q = 0; q < NQ; ++q)
-                if (q < nq)
-                    f[q * MR + r] = r < c ? xp[F.first_col + r + (int64_t)(q0 + q) * n] : TV(0);
-        __syncwarp();
-        for (int h = F.child_beg; h < F.child_end; ++h) {  // children in order
-            const int ch = child[h];
-            const FrontDesc g = fronts[ch];
-            const int uc = g.m - g.c;
-            const TV* w = front_vec(fv, fv_off, ch, nrhs) + g.c * nrhs + q0;
-            const int* rm = relmap + g.rows_off + g.c;
-            for (int rr = lane; rr < uc; rr += 32) {
-                const int p = rm[rr];
-#pragma unroll
-                for (int q = 0; q < NQ; ++q)
-                    if (q < nq) f[q * MR + p] += __ldcg(w + rr * nrhs + q);
-            }
-            __syncwarp();
-        }
-        for (int j = 0; j < c; ++j) {
-            const TL* col = L + j * ldl;
-            const TV d = (TV)col[j];
-            const TV rd = NQ > 1 ? TV(1) / d : TV(0);  // several right-hand sides
-            TV y[NQ];
-#pragma unroll
-            for (int q = 0; q < NQ; ++q) y[q] = NQ > 1 ? f[q * MR + j] * rd : f[q * MR + j] / d;
-            if (lane == (j & 31)) {
-#pragma unroll
-                for (int q = 0; q < NQ; ++q)
-                    if (q < nq) xp[F.first_col + j + (int64_t)(q0 + q) * n] = y[q];
-            }
-            for (int r = j + 1 + lane; r < m; r += 32) {
-                const TV l = (TV)col[r];
-#pragma unroll
-                for (int q = 0; q < NQ; ++q) f[q * MR + r] -= l * y[q];
-            }
-            __syncwarp();
-        }
-        for (int r = c + lane; r < m; r += 32)
-#pragma unroll
-            for (int q = 0; q < NQ; ++q)
-                if (q < nq) out[r * nrhs + q0 + q] = f[q * MR + r];
-        __syncwarp();
-    }
-    group_signal<32>(F.parent >= 0 ? deps.done + F.parent : nullptr, 0xffffffffu);
-}
-
-template <typename TL, typename TV, int NQ>
-__device__ void bwd_warp_front_smem(int s, const FrontDesc& F, const FrontDeps& deps,
-                                    const int* __restrict__ rows, const TL* __restrict__ Ls,
-                                    TV* __restrict__ xp, int n, int nrhs, TV* x, int MR) {
-    if (F.parent >= 0 &&
-        !group_wait<32>(deps.done + F.parent, deps.target[F.parent], deps, 0xffffffffu))
-        return;
-    const int lane = threadIdx.x & 31;
-    const int m = F.m, c = F.c;
-    const int64_t ldl = F.ldl;
-    const TL* L = Ls + F.loff;
-    const int* rw = rows + F.rows_off;
-    for (int q0 = 0; q0 < nrhs; q0 += NQ) {
-        const int nq = min(NQ, nrhs - q0);
-        for (int r = lane; r < m; r += 32) {
-            const int src = r < c ? F.first_col + r : rw[r];
-#pragma unroll
-            for (int q = 0; q < NQ; ++q)
-                x[q * MR + r] = q < nq ? __ldcg(xp + src + (int64_t)(q0 + q) * n) : TV(0);
-        }
-        __syncwarp();
-        for (int j = c - 1; j >= 0; --j) {
-            const TL* col = L + j * ldl;
-            TV p[NQ];
-#pragma unroll
-            for (int q = 0; q < NQ; ++q) p[q] = TV(0);
-            for (int r = j + 1 + lane; r < m; r += 32) {
-                const TV l = (TV)col[r];
-#pragma unroll
-                for (int q = 0; q < NQ; ++q) p[q] += l * x[q * MR + r];
-            }
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1)
-#pragma unroll
-                for (int q = 0; q < NQ; ++q) p[q] += __shfl_xor_sync(0xffffffffu, p[q], o);
-            const TV d = (TV)col[j];
-            if (lane == (j & 31)) {
-#pragma unroll
-                for (int q = 0; q < NQ; ++q) {
-                    const TV v = (x[q * MR + j] - p[q]) / d;
-                    x[q * MR + j] = v;
-                    if (q < nq) xp[F.first_col + j + (int64_t)(q0 + q) * n] = v;
+                        for (int k = ks; k < R; ++k) v[k][q] -= (double)l[k][cc] * y;
+                        if (lane == j) v[ks][q] = y;
+                    }
                 }
             }
-            __syncwarp();
+        }
+#pragma unroll
+        for (int k = 0; k < R; ++k) {
+            const int r = lane + W * k;
+#pragma unroll
+            for (int q = 0; q < NQ; ++q) {
+                if (q >= nq || r >= m) continue;
+                if (r < c)
+                    xp[(int64_t)(F.first_col + r) * nrhs + q0 + q] = v[k][q];
+                else
+                    st_relaxed_f64(out + r * nrhs + q0 + q, v[k][q]);
+            }
         }
     }
-    group_signal<32>(deps.done + s, 0xffffffffu);
 }
 
-// dispatch on the front's rows: registers up to 32, the shared buffer above
-template <typename TL, typename TV, int NQ>
-__device__ void fwd_warp_front(int s, const FrontDeps& deps, const FrontDesc* __restrict__ fronts,
-                               const int* __restrict__ child, const int* __restrict__ relmap,
-                               const int64_t* __restrict__ fv_off, const TL* __restrict__ Ls,
-                               TV* __restrict__ xp, TV* __restrict__ fv, int n, int nrhs,
-                               TV* wbuf, int MR) {
-    const FrontDesc F = fronts[s];
-    TV* out = front_vec(fv, fv_off, s, nrhs);
-    if (F.m <= 32)
-        fwd_group_front<TL, TV, 32, NQ>(s, F, deps, fronts, child, relmap, fv_off, Ls, xp, out,
-                                        fv, n, nrhs, wbuf);
-    else
-        fwd_warp_front_smem<TL, TV, NQ>(s, F, deps, fronts, child, relmap, fv_off, Ls, xp, out,
-                                        fv, n, nrhs, wbuf, MR);
+// Backward: t = L21' x over the update rows (one reduction per pivot column,
+// independent of each other), then the pivot columns from the last, lane i
+// holding column i: x_j = (y_j - t_j) / L(j, j), t_i += L(j, i) x_j, the rows j
+// of L read four at a time down each lane's own column.
+template <typename TL, int W, int R, int NQ>
+__device__ void bwd_front(const FrontDesc& F, const SolveAbort& ab,
+                          const FrontDesc* __restrict__ fronts, const int* __restrict__ rows,
+                          const TL* __restrict__ Ls, const double* __restrict__ xp,
+                          double* __restrict__ xs, int nrhs, double* rds) {
+    static_assert(W == 32 || R == 1, "several rows per lane only on whole warps");
+    constexpr int CH = NQ == 8 ? 1 : solve_chunk<R, NQ>();
+    const unsigned mask = group_mask<W>();
+    const int lane = threadIdx.x & (W - 1);
+    const int m = F.m, c = F.c;
+    const int64_t ldl = F.ldl;
+    const TL* L = Ls + F.loff;
+    int src[R];  // this lane's update rows in the solution
+#pragma unroll
+    for (int k = 0; k < R; ++k) {
+        const int r = lane + W * k;
+        src[k] = -1;
+        if (r >= c && r < m) src[k] = rows[F.rows_off + r];
+    }
+    for (int r = lane; r < c; r += W) rds[r] = 1.0 / (double)L[r + r * ldl];
+    __syncwarp(mask);
+    TL l[R][CH];
+    auto columns = [&](int j0) {
+#pragma unroll
+        for (int cc = 0; cc < CH; ++cc)
+#pragma unroll
+            for (int k = 0; k < R; ++k) {
+                const int r = lane + W * k;
+                l[k][cc] = TL(0);
+                if (r >= c && r < m && j0 + cc < c) l[k][cc] = L[r + (j0 + cc) * ldl];
+            }
+    };
+    // rows 4 b .. 4 b + 3 of L in column lane + W k
+    TL lt[R][4];
+    auto pivot_rows = [&](int b) {
+#pragma unroll
+        for (int k = 0; k < R; ++k) {
+            const int i = lane + W * k;
+#pragma unroll
+            for (int e = 0; e < 4; ++e) lt[k][e] = TL(0);
+            if (i < c && i < 4 * b + 4) ld4(L + 4 * b + i * ldl, lt[k]);
+        }
+    };
+    for (int q0 = 0; q0 < nrhs; q0 += NQ) {
+        const int nq = min(NQ, nrhs - q0);
+        double t[R][NQ], x[R][NQ];
+        columns(0);
+        if (R == 1) pivot_rows((c - 1) / 4);
+#pragma unroll
+        for (int k = 0; k < R; ++k) {
+            const int r = lane + W * k;
+#pragma unroll
+            for (int q = 0; q < NQ; ++q) {  // t starts as -y
+                t[k][q] = 0.0;
+                if (r < c && q < nq)
+                    t[k][q] = -xp[(int64_t)(F.first_col + r) * nrhs + q0 + q];
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < R; ++k)
+            peek_values<NQ>(xs + (int64_t)max(src[k], 0) * nrhs + q0, src[k] >= 0, nq, x[k]);
+        await_together<R, NQ>([&](int k) { return xs + (int64_t)max(src[k], 0) * nrhs + q0; }, nq,
+                              x, mask, ab);
+        if (m > c) {
+#pragma unroll
+            for (int ks = 0; ks < R; ++ks) {
+                for (int j0 = W * ks; j0 < min(c, W * (ks + 1)); j0 += CH) {
+                    if (j0 > 0) columns(j0);
+                    double p[CH][NQ];
+#pragma unroll
+                    for (int cc = 0; cc < CH; ++cc)
+#pragma unroll
+                        for (int q = 0; q < NQ; ++q) {
+                            p[cc][q] = 0.0;
+#pragma unroll
+                            for (int k = 0; k < R; ++k) p[cc][q] += (double)l[k][cc] * x[k][q];
+                        }
+#pragma unroll
+                    for (int o = W / 2; o > 0; o >>= 1)
+#pragma unroll
+                        for (int cc = 0; cc < CH; ++cc)
+#pragma unroll
+                            for (int q = 0; q < NQ; ++q)
+                                p[cc][q] += __shfl_xor_sync(mask, p[cc][q], o, W);
+#pragma unroll
+                    for (int cc = 0; cc < CH; ++cc)
+#pragma unroll
+                        for (int q = 0; q < NQ; ++q)
+                            if (lane == j0 + cc - W * ks) t[ks][q] += p[cc][q];
+                }
+            }
+        }
+#pragma unroll
+        for (int ks = R - 1; ks >= 0; --ks) {
+            for (int b = (min(c, W * (ks + 1)) - 1) / 4; b >= W * ks / 4; --b) {
+                if (R > 1 || 4 * b + 4 < c) pivot_rows(b);
+#pragma unroll
+                for (int e = 3; e >= 0; --e) {
+                    const int j = 4 * b + e;
+                    if (j >= c) continue;
+                    const double rj = rds[j];
+#pragma unroll
+                    for (int q = 0; q < NQ; ++q) {
+                        const double xj = -__shfl_sync(mask, t[ks][q], j - W * ks, W) * rj;
+#pragma unroll
+                        for (int k = 0; k <= ks; ++k)
+                            if (lane + W * k < j) t[k][q] += (double)lt[k][e] * xj;
+                        if (lane == j - W * ks) t[ks][q] = xj;
+                    }
+                }
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < R; ++k) {
+            const int r = lane + W * k;
+#pragma unroll
+            for (int q = 0; q < NQ; ++q)
+                if (q < nq && r < c)
+                    st_relaxed_f64(xs + (int64_t)(F.first_col + r) * nrhs + q0 + q, t[k][q]);
+        }
+    }
 }
 
-template <typename TL, typename TV, int NQ>
-__device__ void bwd_warp_front(int s, const FrontDeps& deps, const FrontDesc* __restrict__ fronts,
-                               const int* __restrict__ rows, const TL* __restrict__ Ls,
-                               TV* __restrict__ xp, int n, int nrhs, TV* wbuf, int MR) {
-    const FrontDesc F = fronts[s];
-    if (F.m <= 32)
-        bwd_group_front<TL, TV, 32, NQ>(s, F, deps, rows, Ls, xp, n, nrhs);
-    else
-        bwd_warp_front_smem<TL, TV, NQ>(s, F, deps, rows, Ls, xp, n, nrhs, wbuf, MR);
+// per-warp shared buffer of the small fronts: the reciprocals of the pivots,
+// then the rows of a pass (32 R rows of solve_pass() right-hand sides)
+constexpr int kWarpBufRows = ((Plan::kSmallMaxRows + 31) / 32) * 32;
+template <bool MULTI>
+__host__ __device__ constexpr int warp_buf() {
+    return kWarpBufRows + (MULTI ? 32 * 12 : kWarpBufRows);
 }
-
-// per-warp shared buffer of the warp path: MR = rows rounded up to 32, times
-// the right-hand sides of one pass
-__host__ __device__ constexpr int warp_rows(int msmall) { return ((msmall + 31) / 32) * 32; }
-__host__ __device__ constexpr int warp_buf_stride(int msmall, bool multi) {
-    return warp_rows(msmall) * (multi ? kWarpSolveRhs : 1);
-}
+static_assert(32 * solve_pass<1, true>() <= 32 * 12 && 32 * 5 * solve_pass<5, true>() <= 32 * 12,
+              "a pass of either kind fits the buffer");
 
 // Warp tasks of one warp item (its slice of the direction's warp list):
 // tasks [0, n1) one front each, then two fronts of 9..16 rows per task, then
@@ -949,86 +996,78 @@ struct WarpTasks {
 };
 
 
-template <typename TL, typename TV, int NQ>
-__device__ void fwd_warp_task(const WarpTasks& wt, int t, const FrontDeps& deps,
+template <typename TL, bool MULTI>
+__device__ void fwd_warp_task(const WarpTasks& wt, int t, const SolveAbort& ab,
                               const FrontDesc* __restrict__ fronts,
                               const int* __restrict__ child, const int* __restrict__ relmap,
                               const int64_t* __restrict__ fv_off, const TL* __restrict__ Ls,
-                              TV* __restrict__ xp, TV* __restrict__ fv, int n, int nrhs, TV* wbuf,
-                              int MR) {
-    const int lane = threadIdx.x & 31;
-    if (t < wt.n1) {
-        fwd_warp_front<TL, TV, NQ>(wt.list[t], deps, fronts, child, relmap, fv_off, Ls, xp, fv, n,
-                                   nrhs, wbuf, MR);
-        return;
-    }
-    t -= wt.n1;
-    const int t2 = (wt.n2 + 1) / 2;
-    if (t < t2) {
-        const int k = 2 * t + (lane >> 4);
-        if (k < wt.n2) {
-            const int s = wt.list[wt.n1 + k];
-            const FrontDesc F = fronts[s];
-            fwd_group_front<TL, TV, 16, NQ>(s, F, deps, fronts, child, relmap, fv_off, Ls, xp,
-                                            front_vec(fv, fv_off, s, nrhs), fv, n, nrhs,
-                                            wbuf + (lane & 16));
-        }
-        return;
-    }
-    const int k = 4 * (t - t2) + (lane >> 3);
-    if (k < wt.n4) {
-        const int s = wt.list[wt.n1 + wt.n2 + k];
+                              double* __restrict__ xp, double* __restrict__ fv, int nrhs,
+                              double* wbuf) {
+    const int lane = threadIdx.x & 31, t2 = (wt.n2 + 1) / 2;
+    auto front = [&](auto w, auto r, int s) {
         const FrontDesc F = fronts[s];
-        fwd_group_front<TL, TV, 8, NQ>(s, F, deps, fronts, child, relmap, fv_off, Ls, xp,
-                                       front_vec(fv, fv_off, s, nrhs), fv, n, nrhs,
-                                       wbuf + (lane & 24));
-    }
-}
-
-template <typename TL, typename TV, int NQ>
-__device__ void bwd_warp_task(const WarpTasks& wt, int t, const FrontDeps& deps,
-                              const FrontDesc* __restrict__ fronts, const int* __restrict__ rows,
-                              const TL* __restrict__ Ls, TV* __restrict__ xp, int n, int nrhs,
-                              TV* wbuf, int MR) {
-    const int lane = threadIdx.x & 31;
+        constexpr int W = decltype(w)::value, R = decltype(r)::value;
+        const int g = W < 32 ? lane & ~(W - 1) : 0;  // the group's place in the buffer
+        fwd_front<TL, W, R, solve_pass<R, MULTI>()>(s, F, ab, fronts, child, relmap, fv_off, Ls,
+                                                    xp, fv, nrhs, wbuf + kWarpBufRows + g,
+                                                    wbuf + g);
+    };
     if (t < wt.n1) {
-        bwd_warp_front<TL, TV, NQ>(wt.list[t], deps, fronts, rows, Ls, xp, n, nrhs, wbuf, MR);
-        return;
-    }
-    t -= wt.n1;
-    const int t2 = (wt.n2 + 1) / 2;
-    if (t < t2) {
+        const int s = wt.list[t];
+        const int m = fronts[s].m;
+        if (m <= 32) front(Int<32>(), Int<1>(), s);
+        else front(Int<32>(), Int<5>(), s);
+    } else if ((t -= wt.n1) < t2) {
         const int k = 2 * t + (lane >> 4);
-        if (k < wt.n2) {
-            const int s = wt.list[wt.n1 + k];
-            bwd_group_front<TL, TV, 16, NQ>(s, fronts[s], deps, rows, Ls, xp, n, nrhs);
-        }
-        return;
-    }
-    const int k = 4 * (t - t2) + (lane >> 3);
-    if (k < wt.n4) {
-        const int s = wt.list[wt.n1 + wt.n2 + k];
-        bwd_group_front<TL, TV, 8, NQ>(s, fronts[s], deps, rows, Ls, xp, n, nrhs);
+        if (k < wt.n2) front(Int<16>(), Int<1>(), wt.list[wt.n1 + k]);
+    } else {
+        const int k = 4 * (t - t2) + (lane >> 3);
+        if (k < wt.n4) front(Int<8>(), Int<1>(), wt.list[wt.n1 + wt.n2 + k]);
     }
 }
 
-// Backward, task (s, j): pivot column tile j of front s accumulates, once
-// the update-row gathers of (s, j) have all counted in, their partial sums
-// in chunk order, then acc += sum_{k > j} L(k, j)' x_k over the pivot tiles
+template <typename TL, bool MULTI>
+__device__ void bwd_warp_task(const WarpTasks& wt, int t, const SolveAbort& ab,
+                              const FrontDesc* __restrict__ fronts, const int* __restrict__ rows,
+                              const TL* __restrict__ Ls, const double* __restrict__ xp,
+                              double* __restrict__ xs, int nrhs, double* wbuf) {
+    const int lane = threadIdx.x & 31, t2 = (wt.n2 + 1) / 2;
+    auto front = [&](auto w, auto r, int s) {
+        const FrontDesc F = fronts[s];
+        constexpr int W = decltype(w)::value, R = decltype(r)::value;
+        bwd_front<TL, W, R, solve_pass<R, MULTI>()>(F, ab, fronts, rows, Ls, xp, xs, nrhs,
+                                                    wbuf + (W < 32 ? lane & ~(W - 1) : 0));
+    };
+    if (t < wt.n1) {
+        const int s = wt.list[t];
+        const int m = fronts[s].m;
+        if (m <= 32) front(Int<32>(), Int<1>(), s);
+        else front(Int<32>(), Int<5>(), s);
+    } else if ((t -= wt.n1) < t2) {
+        const int k = 2 * t + (lane >> 4);
+        if (k < wt.n2) front(Int<16>(), Int<1>(), wt.list[wt.n1 + k]);
+    } else {
+        const int k = 4 * (t - t2) + (lane >> 3);
+        if (k < wt.n4) front(Int<8>(), Int<1>(), wt.list[wt.n1 + wt.n2 + k]);
+    }
+}
+
+// Backward, task (s, j): pivot column tile j of front s accumulates the
+// partial sums of the update-row gathers of (s, j), as they are published, in
+// chunk order, then acc += sum_{k > j} L(k, j)' x_k over the pivot tiles
 // nt1-1 .. j+1 of this front as they publish, and solves
 // x_j = inv(L_jj)' (y_j - acc).  MULTI as in bwd_gather_task.
 template <typename TL, bool MULTI>
 __device__ void bwd_chain_task(int2 tk, const FrontDesc* __restrict__ fronts,
-                               double* __restrict__ pub, int* __restrict__ abort_flag,
-                               int* __restrict__ err, const int* __restrict__ gather_nch,
-                               const int* __restrict__ gather_off, const int* __restrict__ gcount,
+                               double* __restrict__ pub, const SolveAbort& ab,
+                               const int* __restrict__ gather_nch,
+                               const int* __restrict__ gather_off,
                                const double* __restrict__ part,
                                const int64_t* __restrict__ dinv_off, const TL* __restrict__ Ls,
-                               const TL* __restrict__ Dinv, double* __restrict__ xp, int n,
-                               int nrhs) {
+                               const TL* __restrict__ Dinv, const double* __restrict__ xp,
+                               double* __restrict__ xs, int nrhs) {
     constexpr int T = kTile, LD = blk_ld<TL>();
     const LevelSmem<TL, MULTI> sm;
-    __shared__ int s_ok;
     const int tid = threadIdx.x;
     // this thread's column of the tile and right-hand sides: several, two of
     // column tid / 4; one, phase 0 of column c1
@@ -1062,23 +1101,24 @@ __device__ void bwd_chain_task(int2 tk, const FrontDesc* __restrict__ fronts,
     // this tile's y_j, before the first wait
     const int64_t xj = F.first_col + tj.start + l;
     const bool in = l < tj.size;
-    const double y0 = in && own0 ? __ldcg(xp + xj + (int64_t)q * n) : 0.0;
-    const double y1 = in && own1 ? __ldcg(xp + xj + (int64_t)(q + 1) * n) : 0.0;
+    const double y0 = in && own0 ? xp[xj * nrhs + q] : 0.0;
+    const double y1 = in && own1 ? xp[xj * nrhs + q + 1] : 0.0;
     // the update-row partial sums of (s, j) (gathers hold lower tickets), in
-    // chunk order, before the chain's first wait
+    // chunk order, before the chain's first wait; two in flight
     {
         const int nch = gather_nch[s];
-        if (nch > 0) {
-            if (tid == 0) s_ok = wait_flag(gcount + tile0 + j, nch, abort_flag, err) ? 1 : 0;
-            __syncthreads();
-            if (!s_ok) {
-                cp_async_wait_groups<0>();
-                return;
-            }
-            const double* pj = part + ((int64_t)gather_off[s] + (int64_t)j * nch) * T * nrhs;
-            for (int h = 0; h < nch; ++h, pj += (int64_t)T * nrhs) {
-                if (own0) acc[0][0] += __ldcg(pj + l + T * q);
-                if (own1) acc[0][1] += __ldcg(pj + l + T * (q + 1));
+        constexpr int NP = MULTI ? 2 : 1;
+        const double* pj = part + ((int64_t)gather_off[s] + (int64_t)j * nch) * T * nrhs + l + T * q;
+        for (int h = 0; h < nch; h += 2) {
+            double v[2 * NP][1];
+            auto at = [&](int k) { return pj + (int64_t)(h + k / NP) * T * nrhs + T * (k % NP); };
+#pragma unroll
+            for (int k = 0; k < 2 * NP; ++k)
+                peek_values<1>(at(k), (k % NP == 0 ? own0 : own1) && h + k / NP < nch, 1, v[k]);
+#pragma unroll
+            for (int k = 0; k < 2 * NP; ++k) {
+                await_values<1>(at(k), 1, v[k], ab);
+                acc[0][k % NP] += v[k][0];
             }
         }
     }
@@ -1089,8 +1129,7 @@ __device__ void bwd_chain_task(int2 tk, const FrontDesc* __restrict__ fronts,
         __syncthreads();
         const int k = nt1 - 1 - p;
         double* X = sm.vb(p);
-        if (!settle_slot(X, pb + (int64_t)k * T * nrhs, tile_range(k, F.m, F.c, T).size, nrhs,
-                         abort_flag, err)) {
+        if (!settle_slot(X, pb + (int64_t)k * T * nrhs, tile_range(k, F.m, F.c, T).size, nrhs, ab)) {
             ok = false;
             break;
         }
@@ -1115,11 +1154,11 @@ __device__ void bwd_chain_task(int2 tk, const FrontDesc* __restrict__ fronts,
         double x[2][2] = {};
         group_product<TL, true>(sm.lb(P), 0, X, x);
         if (in && own0) {
-            xp[xj + (int64_t)q * n] = x[0][0] + x[1][0];
+            st_relaxed_f64(xs + xj * nrhs + q, x[0][0] + x[1][0]);
             st_relaxed_f64(pb + ((int64_t)j * nrhs + q) * T + l, x[0][0] + x[1][0]);
         }
         if (in && own1) {
-            xp[xj + (int64_t)(q + 1) * n] = x[0][1] + x[1][1];
+            st_relaxed_f64(xs + xj * nrhs + q + 1, x[0][1] + x[1][1]);
             st_relaxed_f64(pb + ((int64_t)j * nrhs + q + 1) * T + l, x[0][1] + x[1][1]);
         }
     } else {
@@ -1136,8 +1175,8 @@ __device__ void bwd_chain_task(int2 tk, const FrontDesc* __restrict__ fronts,
         x += __shfl_xor_sync(0xffffffffu, x, 8);
         x += __shfl_xor_sync(0xffffffffu, x, 16);
         if (q1 == 0 && in) {
-            xp[xj] = x;
             st_relaxed_f64(pb + (int64_t)j * T + l, x);
+            st_relaxed_f64(xs + xj, x);
         }
     }
 }
@@ -1179,22 +1218,15 @@ __device__ __forceinline__ TL ldL(const TL* p) {
 // before the current group's products.
 template <typename TL>
 __device__ void fwd_update_rt1(int s, int R0, int R1, const FrontDesc& F, double* __restrict__ pb,
-                               int* __restrict__ abort_flag, int* __restrict__ err,
-                               const int* __restrict__ amap_off, const int* __restrict__ amap_row,
+                               const SolveAbort& ab, const int* __restrict__ amap_off,
+                               const int* __restrict__ amap_row,
                                const int* __restrict__ amap_ent, const TL* __restrict__ Ls,
-                               const double* __restrict__ xp, double* __restrict__ f,
-                               const double* __restrict__ fv) {
+                               double* __restrict__ f, const double* __restrict__ fv) {
     constexpr int T = kTile;
     const Rt1Smem sm;
     const int R = R0 + threadIdx.x;
     const bool rv = R < R1;
     const TL* Lr = Ls + F.loff + R;
-    double f0 = 0.0;
-    if (rv) {
-        const int* ar = amap_row + amap_off[s] + R;
-        const int e0 = ar[0], e1 = ar[1];
-        for (int e = e0; e < e1; ++e) f0 += __ldcg(fv + amap_ent[e]);
-    }
     constexpr int GW = sizeof(TL) == 4 ? 16 : 8;  // columns per group (registers)
     constexpr int GPB = T / GW;                     // groups per 64-column block
     const int ng = (F.c + GW - 1) / GW;
@@ -1208,12 +1240,14 @@ __device__ void fwd_update_rt1(int s, int R0, int R1, const FrontDesc& F, double
     double acc = 0.0;
     TL lv[GW], ln[GW];
     load(0, lv);
+    double f0[1] = {0.0};
+    if (rv) gather_entries<1>(amap_row + amap_off[s] + R, amap_ent, fv, 1, 1, f0, ab);
     for (int cg = 0; cg < ng; ++cg) {
         if (cg + 1 < ng) load(cg + 1, ln);
         const int k = cg / GPB;
         double* Yk = sm.Ys + (k & 1) * T;
         if (cg % GPB == 0 &&
-            !poll_published(Yk, pb + (int64_t)k * T, min(T, F.c - k * T), 1, abort_flag, err))
+            !poll_published(Yk, pb + (int64_t)k * T, min(T, F.c - k * T), 1, ab))
             return;
         const double* y = Yk + GW * (cg % GPB);
 #pragma unroll
@@ -1221,69 +1255,54 @@ __device__ void fwd_update_rt1(int s, int R0, int R1, const FrontDesc& F, double
 #pragma unroll
         for (int l = 0; l < GW; ++l) lv[l] = ln[l];
     }
-    if (rv) f[R] = f0 - acc;
+    if (rv) st_relaxed_f64(f + R, f0[0] - acc);
 }
 
 // One launch per direction over all work items (the item lists, in a
 // topological order by critical-path priority, and their kinds are
 // described with the solve schedule): persistent CTAs take items by atomic
-// ticket.  An item only waits for items with lower tickets -- children's
-// (forward) and parents' (backward) items come earlier in the list, and so
-// do a front's earlier pivot tiles and its backward gathers -- and a CTA
-// takes a ticket only while it runs, so every wait is for a CTA that is
-// running or done.
-// Forward: a front's items wait for its children (the count of finished
-// children), a small front counts itself in at its parent once written, a
-// large front once its last update tile is (a per-front count of finished
-// update tiles).  Backward: a front's items wait for its parent's solution
-// rows (the parent's count of completions: one per pivot tile of a large
-// front, one for a small front); the pivot tasks wait for their gathers'
-// counts as before.  Every wait polls with an iteration limit; on timeout
-// the launch is aborted (every later wait returns at once) and the error
-// word reaches the host.
+// ticket.  An item only waits for values that items with lower tickets
+// publish -- children's (forward) and parents' (backward) items come earlier
+// in the list, and so do a front's earlier pivot tiles and its backward
+// gathers -- and a CTA takes a ticket only while it runs, so every wait is for
+// a CTA that is running or done.  Every wait polls with an iteration limit; on
+// timeout the launch is aborted (every later wait returns at once) and the
+// error word reaches the host.
 
-// a CTA's tid 0 waits (bounded) for *word >= target; uniform result
-__device__ __forceinline__ bool cta_wait(const int* word, int target, int* abort_flag, int* err) {
-    __shared__ int s_wok;
-    if (threadIdx.x == 0) s_wok = wait_flag(word, target, abort_flag, err) ? 1 : 0;
-    __syncthreads();
-    return s_wok != 0;
-}
-
-// A group's own words in the sync array (its front counts and gather counts)
-// and its slices of the work vectors.
+// Right-hand sides of a launch in groups, with the groups' slices of the work
+// vectors.
 struct SolveGroups {
-    int n, nrhs;        // unknowns, right-hand sides of the launch
-    int stride;         // sync words of a group
-    int64_t fv_total;   // work vector rows
-    __device__ int count() const { return (nrhs + kGroupRhs - 1) / kGroupRhs; }
+    int n, nrhs;       // unknowns, right-hand sides of the launch
+    int64_t fv_total;  // work vector rows
+    // (a group's right-hand sides and solution: rows of size(g) values)
+    __device__ int count() const { return nrhs == 1 ? 1 : (nrhs + kGroupRhs - 1) / kGroupRhs; }
     __device__ int size(int g) const { return min(kGroupRhs, nrhs - kGroupRhs * g); }
     __device__ int64_t xp_off(int g) const { return (int64_t)kGroupRhs * g * n; }
     __device__ int64_t fv_off(int g) const { return kGroupRhs * fv_total * g; }
 };
 
 // residency by shared memory: one right-hand side keeps three blocks of L per
-// CTA (FP32 52 KB, FP64 104 KB), a group two and its vectors (49 and 83 KB)
-template <typename TL, bool MULTI>
+// CTA (FP32 55 KB, FP64 107 KB), a group two and its vectors (49 and 84 KB);
+// by registers (the small fronts' columns of L): three CTAs
+template <typename TL>
 constexpr int solve_ctas_per_sm() {
-    return sizeof(TL) == 8 ? 2 : MULTI ? 3 : 4;
+    return sizeof(TL) == 8 ? 2 : 3;
 }
 
 template <typename TL, bool MULTI>
-__global__ void __launch_bounds__(256, solve_ctas_per_sm<TL, MULTI>())
+__global__ void __launch_bounds__(256, solve_ctas_per_sm<TL>())
     k_fwd_solve(const FrontDesc* __restrict__ fronts, const int4* __restrict__ items, int nitems,
-                int* __restrict__ counter, int64_t pub_rows, int* __restrict__ abort_flag,
-                int* __restrict__ err, int* __restrict__ fdone0, int* __restrict__ udone0,
+                int* __restrict__ counter, int64_t pub_rows, SolveAbort ab,
                 const int64_t* __restrict__ fv_off, const int* __restrict__ amap_off,
                 const int* __restrict__ amap_row, const int* __restrict__ amap_ent,
                 const int64_t* __restrict__ dinv_off, const int* __restrict__ wlist,
                 const int* __restrict__ child,
                 const int* __restrict__ relmap, const TL* __restrict__ Ls,
                 const TL* __restrict__ Dinv, double* __restrict__ xp0, double* __restrict__ fv0,
-                SolveGroups grp, int MR) {
+                SolveGroups grp) {
     constexpr int T = kTile;
     __shared__ int s_item;
-    const int ngroups = MULTI ? grp.count() : 1, n = grp.n;
+    const int ngroups = MULTI ? grp.count() : 1;
     for (;;) {
         if (threadIdx.x == 0) s_item = atomicAdd(counter, 1);
         __syncthreads();
@@ -1294,28 +1313,24 @@ __global__ void __launch_bounds__(256, solve_ctas_per_sm<TL, MULTI>())
         double* xp = xp0 + grp.xp_off(gi);
         double* fv = fv0 + grp.fv_off(gi);
         double* pub = fv + pub_rows * nrhs;
-        int* fdone = fdone0 + gi * grp.stride;
-        int* udone = udone0 + gi * grp.stride;
-        const FrontDeps deps{fdone, nullptr, abort_flag, err};
         if (it.x == SolveScheduleHost::kItemWarps) {
             extern __shared__ __align__(16) unsigned char smem_raw[];
             const WarpTasks wt{wlist + it.y, it.z & 0xff, (it.z >> 8) & 0xff, it.z >> 16};
             const int w = threadIdx.x >> 5, t = w;
-            double* wbuf = reinterpret_cast<double*>(smem_raw) + w * warp_buf_stride(MR, MULTI);
+            double* wbuf = reinterpret_cast<double*>(smem_raw) + w * warp_buf<MULTI>();
             if (t < wt.count())
-                fwd_warp_task<TL, double, MULTI ? kWarpSolveRhs : 1>(
-                    wt, t, deps, fronts, child, relmap, fv_off, Ls, xp, fv, n, nrhs, wbuf, MR);
+                fwd_warp_task<TL, MULTI>(wt, t, ab, fronts, child, relmap, fv_off, Ls, xp, fv,
+                                         nrhs, wbuf);
         } else {
-            // a tile task of a large front: its children first
             const int2 tk = make_int2(it.y, it.z);
-            const int s = tk.x, i0 = tk.y & 0xffff, cnt = tk.y >> 16;
-            const FrontDesc F = fronts[s];
-            const int nt1 = tiles_l(F.c, T);
-            if (cta_wait(fdone + s, F.child_end - F.child_beg, abort_flag, err)) {
-                if constexpr (MULTI) {
-                    fwd_tile_group<TL>(tk, fronts, pub, abort_flag, err, fv_off, amap_off,
-                                       amap_row, amap_ent, dinv_off, Ls, Dinv, xp, fv, n, nrhs);
-                } else if (i0 >= nt1 && nt1 <= kRt1MaxPivotTiles) {
+            if constexpr (MULTI) {
+                fwd_tile_group<TL>(tk, fronts, pub, ab, fv_off, amap_off, amap_row, amap_ent,
+                                   dinv_off, Ls, Dinv, xp, fv, nrhs);
+            } else {
+                const int s = tk.x, i0 = tk.y & 0xffff, cnt = tk.y >> 16;
+                const FrontDesc F = fronts[s];
+                const int nt1 = tiles_l(F.c, T);
+                if (i0 >= nt1 && nt1 <= kRt1MaxPivotTiles) {
                     // update tiles of fronts with at most kRt1MaxPivotTiles
                     // pivot tiles, one right-hand side: registers straight
                     // from L (measured faster there; the staged pipeline
@@ -1323,25 +1338,11 @@ __global__ void __launch_bounds__(256, solve_ctas_per_sm<TL, MULTI>())
                     double* pb = pub + (dinv_off[s] / (T * T)) * T;
                     const TileRange a = tile_range(i0, F.m, F.c, T);
                     const TileRange b = tile_range(i0 + cnt - 1, F.m, F.c, T);
-                    fwd_update_rt1<TL>(s, a.start, b.start + b.size, F, pb, abort_flag, err,
-                                       amap_off, amap_row, amap_ent, Ls, xp,
-                                       front_vec(fv, fv_off, s, 1), fv);
+                    fwd_update_rt1<TL>(s, a.start, b.start + b.size, F, pb, ab, amap_off,
+                                       amap_row, amap_ent, Ls, front_vec(fv, fv_off, s, 1), fv);
                 } else {
-                    fwd_tile_task<TL>(tk, fronts, pub, abort_flag, err, fv_off, amap_off,
-                                      amap_row, amap_ent, dinv_off, Ls, Dinv, xp, fv);
-                }
-                // update tiles counted in; the front's last one counts the
-                // front in at its parent
-                if (i0 >= nt1) {
-                    __syncthreads();
-                    if (threadIdx.x == 0) {
-                        __threadfence();
-                        const int ntu = tiles_l(F.m - F.c, T);
-                        if (atomicAdd(udone + s, cnt) + cnt == ntu && F.parent >= 0) {
-                            __threadfence();
-                            atomicAdd(fdone + F.parent, 1);
-                        }
-                    }
+                    fwd_tile_task<TL>(tk, fronts, pub, ab, fv_off, amap_off, amap_row, amap_ent,
+                                      dinv_off, Ls, Dinv, xp, fv);
                 }
             }
         }
@@ -1349,19 +1350,18 @@ __global__ void __launch_bounds__(256, solve_ctas_per_sm<TL, MULTI>())
     }
 }
 
+// xs (at fv0): the solution, row k's right-hand sides side by side
 template <typename TL, bool MULTI>
-__global__ void __launch_bounds__(256, solve_ctas_per_sm<TL, MULTI>())
+__global__ void __launch_bounds__(256, solve_ctas_per_sm<TL>())
     k_bwd_solve(const FrontDesc* __restrict__ fronts, const int4* __restrict__ items, int nitems,
-                int* __restrict__ counter, int64_t pub_rows, int64_t part_rows,
-                int* __restrict__ abort_flag, int* __restrict__ err, int* __restrict__ bdone0,
-                const int* __restrict__ btarget, const int* __restrict__ gather_nch,
-                const int* __restrict__ gather_off, int* __restrict__ gcount0,
+                int* __restrict__ counter, int64_t pub_rows, int64_t part_rows, SolveAbort ab,
+                const int* __restrict__ gather_nch, const int* __restrict__ gather_off,
                 const int64_t* __restrict__ dinv_off, const int* __restrict__ wlist,
                 const int* __restrict__ rows, const TL* __restrict__ Ls,
-                const TL* __restrict__ Dinv, double* __restrict__ xp0, double* __restrict__ fv0,
-                SolveGroups grp, int MR) {
+                const TL* __restrict__ Dinv, const double* __restrict__ xp0,
+                double* __restrict__ fv0, SolveGroups grp) {
     __shared__ int s_item;
-    const int ngroups = MULTI ? grp.count() : 1, n = grp.n;
+    const int ngroups = MULTI ? grp.count() : 1;
     for (;;) {
         if (threadIdx.x == 0) s_item = atomicAdd(counter, 1);
         __syncthreads();
@@ -1369,57 +1369,43 @@ __global__ void __launch_bounds__(256, solve_ctas_per_sm<TL, MULTI>())
         if (k >= nitems * ngroups) return;
         const int4 it = items[MULTI ? k / ngroups : k];
         const int gi = MULTI ? k % ngroups : 0, nrhs = MULTI ? grp.size(gi) : 1;
-        double* xp = xp0 + grp.xp_off(gi);
-        double* fv = fv0 + grp.fv_off(gi);
-        double* pub = fv + pub_rows * nrhs;
-        double* part = fv + part_rows * nrhs;
-        int* bdone = bdone0 + gi * grp.stride;
-        int* gcount = gcount0 + gi * grp.stride;
-        const FrontDeps deps{bdone, btarget, abort_flag, err};
+        const double* xp = xp0 + grp.xp_off(gi);
+        double* xs = fv0 + grp.fv_off(gi);
+        double* pub = xs + pub_rows * nrhs;
+        double* part = xs + part_rows * nrhs;
         if (it.x == SolveScheduleHost::kItemWarps) {
-            extern __shared__ __align__(16) unsigned char smem_raw[];
             const WarpTasks wt{wlist + it.y, it.z & 0xff, (it.z >> 8) & 0xff, it.z >> 16};
-            const int w = threadIdx.x >> 5, t = w;
-            double* wbuf = reinterpret_cast<double*>(smem_raw) + w * warp_buf_stride(MR, MULTI);
+            extern __shared__ __align__(16) unsigned char smem_raw[];
+            const int t = threadIdx.x >> 5;
             if (t < wt.count())
-                bwd_warp_task<TL, double, MULTI ? kWarpSolveRhs : 1>(wt, t, deps, fronts, rows, Ls,
-                                                                     xp, n, nrhs, wbuf, MR);
+                bwd_warp_task<TL, MULTI>(wt, t, ab, fronts, rows, Ls, xp, xs, nrhs,
+                                         reinterpret_cast<double*>(smem_raw) + t * kWarpBufRows);
         } else if (it.x == SolveScheduleHost::kItemGather) {
-            // the update rows' partial sums need the ancestors' solution
-            const int2 tk = make_int2(it.y, it.z);
-            const int p = fronts[tk.x].parent;
-            if (p < 0 || cta_wait(bdone + p, btarget[p], abort_flag, err))
-                bwd_gather_task<TL, MULTI>(tk, fronts, rows, gather_nch, gather_off, gcount,
-                                           dinv_off, Ls, xp, part, n, nrhs);
+            bwd_gather_task<TL, MULTI>(make_int2(it.y, it.z), fronts, rows, gather_nch, gather_off,
+                                       ab, Ls, xs, part, nrhs);
         } else {
-            // a pivot tile: its gathers (counted) waited for the ancestors
-            const int2 tk = make_int2(it.y, it.z);
-            bwd_chain_task<TL, MULTI>(tk, fronts, pub, abort_flag, err, gather_nch, gather_off,
-                                      gcount, part, dinv_off, Ls, Dinv, xp, n, nrhs);
-            __syncthreads();
-            if (threadIdx.x == 0) {
-                __threadfence();
-                atomicAdd(bdone + tk.x, 1);
-            }
+            bwd_chain_task<TL, MULTI>(make_int2(it.y, it.z), fronts, pub, ab, gather_nch,
+                                      gather_off, part, dinv_off, Ls, Dinv, xp, xs, nrhs);
         }
         __syncthreads();  // shared memory and s_item free for the next item
     }
 }
 
-// Before the sweeps: the sync words cleared, every group's publication slots
-// set to the unpublished pattern.
+// `rows` rows of every group's work vectors set to the unpublished pattern;
+// sync (may be null): the ticket counters and the abort word cleared
 __global__ void __launch_bounds__(256)
-    k_solve_init(int4* __restrict__ sync, int64_t nsync4, double* __restrict__ fv0,
-                 int64_t pub_rows, int64_t slot_rows, SolveGroups grp) {
+    k_solve_init(int4* __restrict__ sync, double* __restrict__ fv0, int64_t rows,
+                 SolveGroups grp) {
     const int64_t tid = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     const int64_t nt = (int64_t)gridDim.x * blockDim.x;
-    for (int64_t i = tid; i < nsync4; i += nt) sync[i] = make_int4(0, 0, 0, 0);
+    if (sync && tid == 0) *sync = make_int4(0, 0, 0, 0);
+    const double v = __longlong_as_double(-1ll);
     for (int g = 0; g < grp.count(); ++g) {
-        // slots start on 16 bytes and hold 64 rows each
-        double2* p = reinterpret_cast<double2*>(fv0 + grp.fv_off(g) + pub_rows * grp.size(g));
-        const int64_t cnt = slot_rows * grp.size(g) / 2;
-        const double v = __longlong_as_double(-1ll);
-        for (int64_t i = tid; i < cnt; i += nt) p[i] = make_double2(v, v);
+        double* p = fv0 + grp.fv_off(g);  // on 16 bytes
+        const int64_t cnt = rows * grp.size(g);
+        for (int64_t i = tid; 2 * i + 1 < cnt; i += nt)
+            reinterpret_cast<double2*>(p)[i] = make_double2(v, v);
+        if ((cnt & 1) && tid == 0) p[cnt - 1] = v;
     }
 }
 
@@ -1427,23 +1413,33 @@ __global__ void __launch_bounds__(256)
 // permutations
 // ---------------------------------------------------------------------------
 
+// b into groups of right-hand sides one after another, a row's right-hand
+// sides of a group side by side
 __global__ void k_perm_gather(const int* __restrict__ perm, const double* __restrict__ b,
-                              double* __restrict__ xp, int n, int nrhs, int ldb) {
-    int64_t total = (int64_t)n * nrhs;
+                              double* __restrict__ xp, SolveGroups grp, int ldb) {
+    const int n = grp.n;
+    const int64_t total = (int64_t)n * grp.nrhs;
     for (int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; idx < total;
          idx += (int64_t)gridDim.x * blockDim.x) {
-        int q = (int)(idx / n), k = (int)(idx - (int64_t)q * n);
-        xp[idx] = b[(perm ? perm[k] : k) + (int64_t)q * ldb];
+        const int q = (int)(idx / n), k = (int)(idx - (int64_t)q * n);
+        const int g = grp.nrhs == 1 ? 0 : q / kGroupRhs;
+        xp[grp.xp_off(g) + (int64_t)k * grp.size(g) + q - g * kGroupRhs] =
+            b[(perm ? perm[k] : k) + (int64_t)q * ldb];
     }
 }
 
-__global__ void k_perm_scatter(const int* __restrict__ perm, const double* __restrict__ xp,
-                               double* __restrict__ x, int n, int nrhs, int ldx) {
-    int64_t total = (int64_t)n * nrhs;
+// xs: the backward sweep's solution, groups of right-hand sides one after
+// another, fv_total rows apart, a row's right-hand sides side by side
+__global__ void k_perm_scatter(const int* __restrict__ perm, const double* __restrict__ xs,
+                               double* __restrict__ x, SolveGroups grp, int ldx) {
+    const int n = grp.n;
+    const int64_t total = (int64_t)n * grp.nrhs;
     for (int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; idx < total;
          idx += (int64_t)gridDim.x * blockDim.x) {
-        int q = (int)(idx / n), k = (int)(idx - (int64_t)q * n);
-        x[(perm ? perm[k] : k) + (int64_t)q * ldx] = xp[idx];
+        const int q = (int)(idx / n), k = (int)(idx - (int64_t)q * n);
+        const int g = grp.nrhs == 1 ? 0 : q / kGroupRhs;
+        x[(perm ? perm[k] : k) + (int64_t)q * ldx] =
+            xs[grp.fv_off(g) + (int64_t)k * grp.size(g) + q - g * kGroupRhs];
     }
 }
 
@@ -1451,22 +1447,19 @@ void permute_gather(const int* perm, const double* b, double* xp, int n, int nrh
                     cudaStream_t st) {
     int64_t total = (int64_t)n * nrhs;
     int blocks = (int)std::min<int64_t>((total + 255) / 256, 148 * 16);
-    k_perm_gather<<<blocks, 256, 0, st>>>(perm, b, xp, n, nrhs, ldb);
+    k_perm_gather<<<blocks, 256, 0, st>>>(perm, b, xp, SolveGroups{n, nrhs, 0}, ldb);
 }
 
-void permute_scatter(const int* perm, const double* xp, double* x, int n, int nrhs, int ldx,
-                     cudaStream_t st) {
-    int64_t total = (int64_t)n * nrhs;
-    int blocks = (int)std::min<int64_t>((total + 255) / 256, 148 * 16);
-    k_perm_scatter<<<blocks, 256, 0, st>>>(perm, xp, x, n, nrhs, ldx);
+void permute_solution(const DevPlan& D, const int* perm, const double* fv, double* x, int nrhs,
+                      int ldx, cudaStream_t st) {
+    const int64_t total = (int64_t)D.n * nrhs;
+    const int blocks = (int)std::min<int64_t>((total + 255) / 256, 148 * 16);
+    k_perm_scatter<<<blocks, 256, 0, st>>>(perm, fv, x, SolveGroups{D.n, nrhs, D.fv_total}, ldx);
 }
 
 // ---------------------------------------------------------------------------
 // launch sequence
 // ---------------------------------------------------------------------------
-
-// rows of a small front's warp buffer (every level's largest small front)
-constexpr int kWarpBufRows = ((Plan::kSmallMaxRows + 31) / 32) * 32;
 
 // dynamic shared memory of a solve launch: the tile tasks' stages or the
 // eight warps' buffers, whichever is larger
@@ -1474,7 +1467,7 @@ template <typename TL, bool MULTI>
 static size_t solve_smem() {
     size_t m = level_smem_bytes<TL, MULTI>();
     if (!MULTI) m = std::max(m, rt1_smem_bytes<TL>());
-    return std::max(m, 8 * (size_t)warp_buf_stride(kWarpBufRows, MULTI) * sizeof(double));
+    return std::max(m, 8 * (size_t)warp_buf<MULTI>() * sizeof(double));
 }
 
 template <typename TL, bool MULTI>
@@ -1491,79 +1484,59 @@ void init_solve_kernels() {
     set_solve_attributes<float, true>();
 }
 
-int solve_groups(int nrhs) { return nrhs == 1 ? 1 : (nrhs + kGroupRhs - 1) / kGroupRhs; }
-int64_t solve_sync_words(int nflags, int nfronts, int groups) {
-    return (4 + (int64_t)groups * (nflags + 3 * (int64_t)nfronts) + 3) & ~(int64_t)3;
-}
-
 template <typename TL, bool MULTI>
 static void solve_launch(const DevPlan& D, const TL* Ls, const TL* Dinv, double* xp, double* fv,
                          int nrhs, cudaStream_t st) {
     const SolveSchedule& S = D.solve;
-    static_assert(Plan::kSmallMaxRows <= 32 * 5, "the warp path holds 160 rows in shared memory");
-    // sync: the two ticket counters and the abort word, then per group the
-    // gathers' counts per pivot tile, and per front the forward
-    // finished-children and finished-update-tile counts and the backward
-    // completions
-    int* counters = S.sync;
-    int* abort_flag = S.sync + 2;
-    int* gcount = S.sync + 4;
-    int* fdone = gcount + S.nflags;
-    int* udone = fdone + S.nfronts;
-    int* bdone = udone + S.nfronts;
-    const SolveGroups grp{D.n, nrhs, S.nflags + 3 * S.nfronts, D.fv_total};
+    static_assert(Plan::kSmallMaxRows <= 32 * 5, "the warp path holds 160 rows in registers");
+    // sync: the two ticket counters and the abort word
+    const SolveAbort ab{S.sync + 2, S.err};
+    const SolveGroups grp{D.n, nrhs, D.fv_total};
     const int64_t slots = (int64_t)S.nflags * kTile;  // rows of one direction
-    const int64_t nsync = solve_sync_words(S.nflags, S.nfronts, solve_groups(nrhs));
     const int sms = D.num_sms > 0 ? D.num_sms : 148;
-    {
-        const int64_t work = std::max(nsync / 4, slots * nrhs);
-        const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>((work + 1023) / 1024, sms * 8));
-        k_solve_init<<<blocks, 256, 0, st>>>(reinterpret_cast<int4*>(S.sync), nsync / 4, fv,
-                                             D.fv_pub_off, 2 * slots, grp);
-    }
+    auto init = [&](int4* sync, int64_t rows) {
+        const int64_t work = rows * nrhs / 2;
+        const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>((work + 511) / 512, sms * 8));
+        k_solve_init<<<blocks, 256, 0, st>>>(sync, fv, rows, grp);
+    };
     const size_t sm = solve_smem<TL, MULTI>();
-    const int grid = sms * solve_ctas_per_sm<TL, MULTI>();
-    const int ng = MULTI ? solve_groups(nrhs) : 1;
+    const int grid = sms * solve_ctas_per_sm<TL>();
+    const int ng = MULTI ? (nrhs + kGroupRhs - 1) / kGroupRhs : 1;
     double fbytes = 0, bbytes = 0;
     for (int l = 0; l < D.nlevels; ++l) {
         fbytes += (S.small_elems[l] + S.fwd_elems[l]) * sizeof(TL);
         bbytes += (S.small_elems[l] + S.bwd_elems[l]) * sizeof(TL);
     }
+    init(reinterpret_cast<int4*>(S.sync), D.fv_total);
     if (S.nfwd_items > 0) {
         ProfScope ps(D.prof, KC_SOLVE_LARGE, st, 0, fbytes);
         k_fwd_solve<TL, MULTI><<<std::min(grid, S.nfwd_items * ng), 256, sm, st>>>(
-            D.fronts, S.fwd_items, S.nfwd_items, counters, D.fv_pub_off, abort_flag,
-            S.err, fdone, udone, D.fv_off, S.amap_off, S.amap_row, S.amap_ent, D.dinv_off,
-            S.fwd_wlist, D.child, D.relmap, Ls, Dinv, xp, fv, grp, kWarpBufRows);
+            D.fronts, S.fwd_items, S.nfwd_items, S.sync, D.fv_pub_off, ab, D.fv_off, S.amap_off,
+            S.amap_row, S.amap_ent, D.dinv_off, S.fwd_wlist, D.child, D.relmap, Ls, Dinv, xp, fv,
+            grp);
     }
+    // the solution takes the place of the front vectors (at least n rows)
+    init(nullptr, D.n);
     if (S.nbwd_items > 0) {
         ProfScope ps(D.prof, KC_SOLVE_LARGE, st, 0, bbytes);
         k_bwd_solve<TL, MULTI><<<std::min(grid, S.nbwd_items * ng), 256, sm, st>>>(
-            D.fronts, S.bwd_items, S.nbwd_items, counters + 1, D.fv_pub_off + slots, D.fv_fronts,
-            abort_flag, S.err, bdone, S.bwd_target, S.gather_nch, S.gather_off, gcount,
-            D.dinv_off, S.bwd_wlist, D.rows, Ls, Dinv, xp, fv, grp, kWarpBufRows);
+            D.fronts, S.bwd_items, S.nbwd_items, S.sync + 1, D.fv_pub_off + slots, D.fv_fronts, ab,
+            S.gather_nch, S.gather_off, D.dinv_off, S.bwd_wlist, D.rows, Ls, Dinv, xp, fv, grp);
     }
 }
 
-template <typename TL, typename TV>
-void solve_levels(const DevPlan& D, const TL* Ls, const TL* Dinv, TV* xp, TV* fv, int nrhs,
+template <typename TL>
+void solve_levels(const DevPlan& D, const TL* Ls, const TL* Dinv, double* xp, double* fv, int nrhs,
                   cudaStream_t st) {
-    // as many groups of right-hand sides per launch as the sync words hold
-    // (the work vectors are reused by the next launch)
-    const int pass = kGroupRhs * D.solve.sync_groups;
-    for (int q0 = 0; q0 < nrhs; q0 += pass) {
-        const int nq = std::min(pass, nrhs - q0);
-        double* x = xp + (int64_t)q0 * D.n;
-        if (nq == 1)
-            solve_launch<TL, false>(D, Ls, Dinv, x, fv, nq, st);
-        else
-            solve_launch<TL, true>(D, Ls, Dinv, x, fv, nq, st);
-    }
+    if (nrhs == 1)
+        solve_launch<TL, false>(D, Ls, Dinv, xp, fv, nrhs, st);
+    else
+        solve_launch<TL, true>(D, Ls, Dinv, xp, fv, nrhs, st);
 }
 
-template void solve_levels<double, double>(const DevPlan&, const double*, const double*, double*,
-                                           double*, int, cudaStream_t);
-template void solve_levels<float, double>(const DevPlan&, const float*, const float*, double*,
-                                          double*, int, cudaStream_t);
+template void solve_levels<double>(const DevPlan&, const double*, const double*, double*, double*,
+                                   int, cudaStream_t);
+template void solve_levels<float>(const DevPlan&, const float*, const float*, double*, double*, int,
+                                  cudaStream_t);
 
 }  // namespace mdgpu
