@@ -1,9 +1,10 @@
 // Numeric factorization kernels (scalar T = double or float).
 //
-// Small fronts (m <= 160): one CTA per front does everything in shared memory:
-// zero the front, scatter A's values, extend-add every child's update matrix
-// (children one after another, so the sum is deterministic), factor the c
-// pivot columns, write the L panel and the Schur complement U = F22 - L21 L21'.
+// Small fronts (m <= 160): a CTA, a warp or a part of a warp per front does
+// everything in shared memory and registers: zero the front, scatter A's values,
+// extend-add every child's update matrix (children one after another, so the
+// sum is deterministic), factor the c pivot columns, write the L panel and the
+// Schur complement U = F22 - L21 L21'.
 //
 // Large fronts: a tiled right-looking partial Cholesky over the [L | U] split
 // storage, batched over all large fronts of one tree level:
@@ -25,89 +26,275 @@
 namespace mdgpu {
 
 // ---------------------------------------------------------------------------
-// fused small-front kernel
+// small fronts
 // ---------------------------------------------------------------------------
 
-template <typename T>
-__global__ void k_small_front(const FrontDesc* __restrict__ fronts, const int* __restrict__ list,
-                              const int* __restrict__ child, const int* __restrict__ relmap,
-                              const int* __restrict__ a_src, const int* __restrict__ a_pos,
-                              const double* __restrict__ Ax, T* __restrict__ Ls,
-                              T* __restrict__ Us, int LD, int* __restrict__ status) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    T* F = reinterpret_cast<T*>(smem_raw);
-    int* rel = reinterpret_cast<int*>(F + (size_t)LD * (LD - 1));
-    const int s = list[blockIdx.x];
-    const FrontDesc f = fronts[s];
-    const int m = f.m, c = f.c, u = m - c;
-    const int tid = threadIdx.x, nt = blockDim.x;
+// Most small fronts have one to a few pivot columns, so their time is the
+// chain of dependent memory trips and barriers of the assembly, not
+// arithmetic: descriptions of up to 32 children are loaded by the lanes at
+// once, a warp takes eight columns of a child's update matrix at a time, lane =
+// row, with the next eight on their way, across children too, and no index is
+// divided.  (With a division per element, a barrier or two per child and per
+// pivot column: fronts of 33..160 rows 11.5 ms, now 4.2, and up to 32 rows 1.1,
+// now 0.74, over 130 + 26 launches of a batch of 2D and 3D grids, FP32; a root
+// of 149 columns FP64 478 us, now 85.)  What is left of a level of a few tiny
+// fronts, 4 to 8 us, is mostly its cold instructions: about ten cycles each.
 
-    for (int idx = tid; idx < m * LD; idx += nt) F[idx] = T(0);
-    __syncthreads();
-    for (int e = f.a_beg + tid; e < f.a_end; e += nt) {
-        int src = a_src[e];
-        if (src >= 0) {
-            int pos = a_pos[e];
-            F[(pos & 0xffff) + (pos >> 16) * LD] = (T)Ax[src];
-        }
-    }
-    __syncthreads();
-    for (int h = f.child_beg; h < f.child_end; ++h) {
-        const FrontDesc g = fronts[child[h]];
-        const int uc = g.m - g.c;
-        if (uc <= 0) continue;
-        for (int i = tid; i < uc; i += nt) rel[i] = relmap[g.rows_off + g.c + i];
-        __syncthreads();
-        const T* U = Us + g.uoff;
-        for (int idx = tid; idx < uc * uc; idx += nt) {
-            int j = idx / uc, i = idx - j * uc;
-            if (i >= j) F[rel[i] + rel[j] * LD] += U[i + (int64_t)j * g.ldu];
-        }
-        __syncthreads();
-    }
-    // partial Cholesky of the c pivot columns (right-looking, panel only)
-    for (int k = 0; k < c; ++k) {
-        const T dkk = F[k + k * LD];
-        const T d = sqrt(dkk);
-        if (tid == 0 && !(dkk > T(0))) flag_pivot(status, f.first_col + k);
-        const T inv = T(1) / d;
-        for (int i = k + 1 + tid; i < m; i += nt) F[i + k * LD] *= inv;
-        __syncthreads();
-        if (tid == 0) F[k + k * LD] = d;
-        const int rows = m - k - 1, w = c - k - 1;
-        for (int idx = tid; idx < rows * w; idx += nt) {
-            int jj = idx / rows, ii = idx - jj * rows;
-            int i = k + 1 + ii, j = k + 1 + jj;
-            if (i >= j) F[i + j * LD] -= F[i + k * LD] * F[j + k * LD];
-        }
-        __syncthreads();
-    }
-    // Schur complement straight to the update store
-    if (f.uoff >= 0) {
-        T* Ud = Us + f.uoff;
-        for (int idx = tid; idx < u * u; idx += nt) {
-            int j = idx / u, i = idx - j * u;
-            if (i >= j) {
-                T acc = F[(c + i) + (c + j) * LD];
-                const T* a = F + c + i;
-                const T* b = F + c + j;
-#pragma unroll 4
-                for (int k = 0; k < c; ++k) acc -= a[k * LD] * b[k * LD];
-                Ud[i + (int64_t)j * f.ldu] = acc;
-            }
-        }
-    }
-    T* Ld = Ls + f.loff;
-    for (int idx = tid; idx < m * c; idx += nt) {
-        int j = idx / m, i = idx - j * m;
-        Ld[i + (int64_t)j * f.ldl] = (i >= j) ? F[i + j * LD] : T(0);
+// sqrt(x) and 1 / sqrt(x) from one reciprocal square root, each corrected by
+// one Newton step (infinity keeps its own)
+template <typename T>
+__device__ __forceinline__ void pivot_root(T x, T& root, T& inv) {
+    const T y = recip_sqrt(x), s = x * y;
+    const T h = T(0.5) * y;
+    inv = y == T(0) ? y : fma(h, fma(-s, y, T(1)), y);
+    root = y == T(0) ? x : fma(h, fma(-s, s, x), s);
+}
+
+// 8 neighbouring elements on 16 bytes
+__device__ __forceinline__ void vec8_ld(const float* p, float (&v)[8]) {
+    const float4 a = reinterpret_cast<const float4*>(p)[0];
+    const float4 b = reinterpret_cast<const float4*>(p)[1];
+    v[0] = a.x, v[1] = a.y, v[2] = a.z, v[3] = a.w;
+    v[4] = b.x, v[5] = b.y, v[6] = b.z, v[7] = b.w;
+}
+__device__ __forceinline__ void vec8_ld(const double* p, double (&v)[8]) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const double2 a = reinterpret_cast<const double2*>(p)[i];
+        v[2 * i] = a.x, v[2 * i + 1] = a.y;
     }
 }
 
-// Fronts of at most 32 rows: a group of W lanes per front (W = 32, 16, 8:
-// one, two or four fronts per warp), the front in the group's own W x (W + 1)
-// shared slice; the same steps and sums in the same order as k_small_front,
-// with group syncs only.
+// leading dimension of a front of up to MB rows in shared memory (columns on
+// 16 bytes)
+template <typename T>
+__host__ __device__ constexpr int small_ld(int MB) {
+    return MB + 16 / (int)sizeof(T);
+}
+
+// One front of up to MB rows by `nw` warps (ceil(MB / 32) or fewer, up to the
+// block's), F: MB columns of LD = small_ld(MB) elements; sync: a barrier over
+// the nw warps.
+template <typename T, typename Sync>
+__device__ __forceinline__ void small_front(const FrontDesc& f, T* F, int LD, int warp, int nw,
+                                            Sync&& sync, const FrontDesc* __restrict__ fronts,
+                                            const int* __restrict__ child,
+                                            const int* __restrict__ relmap,
+                                            const int* __restrict__ a_src,
+                                            const int* __restrict__ a_pos,
+                                            const double* __restrict__ Ax, T* __restrict__ Ls,
+                                            T* __restrict__ Us, int* __restrict__ status) {
+    constexpr unsigned ALL = 0xffffffffu;
+    constexpr int CG = 8;  // columns at a time: most fronts' pivot columns fit one panel
+    const int m = f.m, c = f.c, lane = threadIdx.x & 31;
+    const int tid = 32 * warp + lane, nt = 32 * nw;
+    // the chains of loads before the first barrier side by side: an A entry's
+    // place and value, and child, description, update matrix
+    int src = -1, pos = 0;
+    if (f.a_beg + tid < f.a_end) {
+        src = a_src[f.a_beg + tid];
+        pos = a_pos[f.a_beg + tid];
+    }
+    int g_id = -1;
+    if (f.child_beg + lane < f.child_end) g_id = child[f.child_beg + lane];
+    for (int idx = tid; idx < m * LD * (int)sizeof(T) / 16; idx += nt)
+        reinterpret_cast<int4*>(F)[idx] = make_int4(0, 0, 0, 0);
+
+    // the children of a batch of up to 32, one per lane
+    int64_t g_u = 0;
+    int g_uc = 0, g_ldu = 0, g_rel = 0;
+    // the trip of this warp: CG columns from j0 on of child h of the batch, rows
+    // i0 + lane; h == nb at the end
+    int hb = f.child_beg, nb = 0, h = 0, j0 = 0, i0 = 0, uc = 0;
+    auto settle = [&]() {  // skips children with no trip left
+        while (j0 >= uc) {
+            if (++h >= nb) return;
+            uc = __shfl_sync(ALL, g_uc, h);
+            j0 = CG * warp;
+            i0 = j0 & ~31;
+        }
+    };
+    auto describe = [&]() {
+        nb = min(32, f.child_end - hb);
+        g_uc = 0;
+        if (g_id >= 0) {
+            const FrontDesc& g = fronts[g_id];
+            g_uc = g.m - g.c;
+            g_ldu = g.ldu;
+            g_rel = g.rows_off + g.c;
+            g_u = g.uoff;
+        }
+    };
+    auto begin = [&]() {
+        h = -1, j0 = uc = 0;
+        settle();
+    };
+    T v[CG];
+    int ri = 0, rj = 0;  // the trip's row of this lane, column of lane & 7
+    auto fetch = [&]() {
+        if (h >= nb) return;
+        const T* U = Us + __shfl_sync(ALL, g_u, h);
+        const int ldu = __shfl_sync(ALL, g_ldu, h);
+        const int* rm = relmap + __shfl_sync(ALL, g_rel, h);
+        const int i = i0 + lane;
+#pragma unroll
+        for (int e = 0; e < CG; ++e) {
+            v[e] = T(0);
+            if (i < uc && i >= j0 + e) v[e] = U[i + (int64_t)(j0 + e) * ldu];
+        }
+        ri = i < uc ? rm[i] : 0;
+        rj = j0 + (lane & 7) < uc ? rm[j0 + (lane & 7)] : 0;
+    };
+    describe();
+    const T av = src >= 0 ? (T)Ax[src] : T(0);
+    begin();
+    fetch();
+    sync();
+    if (src >= 0) F[(pos & 0xffff) + (pos >> 16) * LD] = av;
+    for (int e = f.a_beg + nt + tid; e < f.a_end; e += nt) {
+        src = a_src[e];
+        if (src >= 0) {
+            pos = a_pos[e];
+            F[(pos & 0xffff) + (pos >> 16) * LD] = (T)Ax[src];
+        }
+    }
+    // children in order, a barrier after each
+    for (;;) {
+        for (int done = -1; done < nb;) {
+            // to the child of the trip at hand
+            for (; done < h; ++done) sync();
+            if (h >= nb) break;
+            T w[CG];
+#pragma unroll
+            for (int e = 0; e < CG; ++e) w[e] = v[e];
+            const int wi = ri, wj = rj, cnt = uc, i = i0 + lane, jb = j0;
+            i0 += 32;
+            if (i0 >= uc) {
+                j0 += CG * nw;
+                i0 = j0 & ~31;
+                settle();
+            }
+            fetch();
+            T* at[CG];  // distinct columns: all reads before the writes
+#pragma unroll
+            for (int e = 0; e < CG; ++e) {
+                at[e] = F + wi + __shfl_sync(ALL, wj, e) * LD;
+                if (i < cnt && i >= jb + e) w[e] += *at[e];
+            }
+#pragma unroll
+            for (int e = 0; e < CG; ++e)
+                if (i < cnt && i >= jb + e) *at[e] = w[e];
+        }
+        hb += 32;
+        if (hb >= f.child_end) break;
+        g_id = hb + lane < f.child_end ? child[hb + lane] : -1;
+        describe();
+        begin();
+        fetch();
+    }
+
+    // pivot columns in panels of eight, lane = row, every warp factoring the
+    // diagonal block along with its rows (its multipliers by shuffles), then the
+    // trailing update; the last panel's goes straight to the update store
+    for (int p = 0; p < c; p += CG) {
+        const int n = min(CG, c - p), pe = p + n;
+        T a[CG];
+        // (the first block last: its diagonal rows wait for the barrier)
+        const int nrb = (m - p + 31) / 32;
+        for (int rb = warp + (nrb - 1 - warp) / nw * nw; warp < nrb && rb >= 0; rb -= nw) {
+            const int r = p + 32 * rb + lane;
+            T d[CG];
+#pragma unroll
+            for (int j = 0; j < CG; ++j) {
+                d[j] = a[j] = T(0);
+                if (j < n) {
+                    d[j] = F[p + (lane & 7) + (p + j) * LD];
+                    if (r < m) a[j] = F[r + (p + j) * LD];
+                }
+            }
+#pragma unroll
+            for (int k = 0; k < CG; ++k) {
+                if (k >= n) break;
+                const T piv = __shfl_sync(ALL, d[k], k);
+                T root, inv;
+                pivot_root(piv, root, inv);
+                if (rb == 0 && lane == k && !(piv > T(0))) flag_pivot(status, f.first_col + p + k);
+                const T ld = d[k] * inv, lr = a[k] * inv;
+                a[k] = r == p + k ? root : lr;
+#pragma unroll
+                for (int j = k + 1; j < CG; ++j) {
+                    const T t = __shfl_sync(ALL, ld, j);
+                    d[j] -= ld * t;
+                    a[j] -= lr * t;
+                }
+            }
+            if (r >= pe && r < m)
+#pragma unroll
+                for (int j = 0; j < CG; ++j)
+                    if (j < n) F[r + (p + j) * LD] = a[j];
+        }
+        sync();
+        if (warp == 0 && lane < n)
+#pragma unroll
+            for (int j = 0; j < CG; ++j)
+                if (j <= lane) F[p + lane + (p + j) * LD] = a[j];
+        const bool last = pe == c;
+        if (last && f.uoff < 0) break;
+        for (int jg = (pe & ~(CG - 1)) + CG * warp; jg < m; jg += CG * nw) {
+            // rows from the first one on or below the group's diagonal
+            for (int r0 = max(jg, pe); r0 < m; r0 += 32) {
+                const int r = r0 + lane;
+                T acc[CG];
+#pragma unroll
+                for (int e = 0; e < CG; ++e) acc[e] = r < m ? F[r + (jg + e) * LD] : T(0);
+#pragma unroll 4
+                for (int k = p; k < pe; ++k) {
+                    T b[CG];
+                    vec8_ld(F + jg + k * LD, b);
+                    const T x = r < m ? F[r + k * LD] : T(0);
+#pragma unroll
+                    for (int e = 0; e < CG; ++e) acc[e] -= x * b[e];
+                }
+#pragma unroll
+                for (int e = 0; e < CG; ++e) {
+                    const int j = jg + e;
+                    if (r >= m || r < j || j < pe) continue;
+                    if (last)
+                        Us[f.uoff + (r - c) + (int64_t)(j - c) * f.ldu] = acc[e];
+                    else
+                        F[r + j * LD] = acc[e];
+                }
+            }
+        }
+        if (!last) sync();
+    }
+    sync();
+    for (int j = warp; j < c; j += nw) {
+        T* Lj = Ls + f.loff + (int64_t)j * f.ldl;
+        for (int r = lane; r < m; r += 32) Lj[r] = r >= j ? F[r + j * LD] : T(0);
+    }
+}
+
+// Fronts of 33..160 rows: a CTA each.
+template <typename T>
+__global__ void __launch_bounds__(512)
+    k_small_front(const FrontDesc* __restrict__ fronts, const int* __restrict__ list,
+                  const int* __restrict__ child, const int* __restrict__ relmap,
+                  const int* __restrict__ a_src, const int* __restrict__ a_pos,
+                  const double* __restrict__ Ax, T* __restrict__ Ls, T* __restrict__ Us, int LD,
+                  int* __restrict__ status) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const FrontDesc f = fronts[list[blockIdx.x]];
+    small_front<T>(f, reinterpret_cast<T*>(smem_raw), LD, threadIdx.x >> 5, blockDim.x >> 5,
+                   [] { __syncthreads(); }, fronts, child, relmap, a_src, a_pos, Ax, Ls, Us,
+                   status);
+}
+
+// Fronts of at most 16 (8) rows: W = 16 (8) lanes per front, two (four) fronts
+// per warp, in step with each other: every loop runs to the warp's longest, so
+// that the lanes stay together and a shuffle costs a shuffle.  Lane = row, the
+// whole row in registers after the assembly in the group's W x (W + 1) slice
+// of shared memory.  s < 0: no front for this group.
 constexpr int kTinyFrontRows = 32;
 
 template <typename T, int W>
@@ -116,69 +303,133 @@ __device__ void tiny_front_group(int s, const FrontDesc* __restrict__ fronts,
                                  const int* __restrict__ a_src, const int* __restrict__ a_pos,
                                  const double* __restrict__ Ax, T* __restrict__ Ls,
                                  T* __restrict__ Us, int* __restrict__ status, T* Fm) {
-    constexpr int LD = W + 1;
-    const unsigned mask =
-        W == 32 ? 0xffffffffu : (((1u << W) - 1u) << ((threadIdx.x & 31) & ~(W - 1)));
+    constexpr unsigned ALL = 0xffffffffu;
+    constexpr int LD = W + 1, CG = 8;
     const int gl = threadIdx.x & (W - 1);
-    const FrontDesc f = fronts[s];
-    const int m = f.m, c = f.c, u = m - c;
-    for (int idx = gl; idx < m * LD; idx += W) Fm[idx] = T(0);
-    __syncwarp(mask);
-    for (int e = f.a_beg + gl; e < f.a_end; e += W) {
-        const int src = a_src[e];
-        if (src >= 0) {
-            const int pos = a_pos[e];
-            Fm[(pos & 0xffff) + (pos >> 16) * LD] = (T)Ax[src];
-        }
+    FrontDesc f;
+    f.m = f.c = f.child_beg = f.child_end = f.a_beg = f.a_end = 0;
+    f.uoff = -1;
+    if (s >= 0) f = fronts[s];
+    const int m = f.m, c = f.c, nch = f.child_end - f.child_beg;
+    int src = -1, pos = 0;
+    if (f.a_beg + gl < f.a_end) {
+        src = a_src[f.a_beg + gl];
+        pos = a_pos[f.a_beg + gl];
     }
-    __syncwarp(mask);
-    for (int h = f.child_beg; h < f.child_end; ++h) {
-        const FrontDesc g = fronts[child[h]];
-        const int uc = g.m - g.c;
-        if (uc <= 0) continue;
-        const int* rm = relmap + g.rows_off + g.c;
-        const T* U = Us + g.uoff;
-        for (int idx = gl; idx < uc * uc; idx += W) {
-            const int j = idx / uc, i = idx - j * uc;
-            if (i >= j) Fm[rm[i] + rm[j] * LD] += U[i + (int64_t)j * g.ldu];
+    int g_id = gl < nch ? child[f.child_beg + gl] : -1;
+#pragma unroll
+    for (int j = 0; j < W; ++j) Fm[gl + j * LD] = T(0);
+    // the children of a batch of up to W, one per lane; the trip at hand: CG
+    // columns from j0 on of child h of the batch, maxuc the warp's longest
+    const int maxch = __reduce_max_sync(ALL, nch);
+    int64_t g_u = 0;
+    int g_uc = 0, g_ldu = 0, g_rel = 0;
+    int h = 0, nb = 0, j0 = 0, uc = 0, maxuc = 0;
+    auto describe = [&]() {
+        g_uc = 0;
+        if (g_id >= 0) {
+            const FrontDesc& g = fronts[g_id];
+            g_uc = g.m - g.c;
+            g_ldu = g.ldu;
+            g_rel = g.rows_off + g.c;
+            g_u = g.uoff;
         }
-        __syncwarp(mask);
-    }
-    // partial Cholesky of the c pivot columns (right-looking, panel only):
-    // lane i of the group owns row i and touches only it; the multipliers of
-    // the other rows arrive by shuffles
-    for (int k = 0; k < c; ++k) {
-        const T dkk = Fm[k + k * LD];
-        if (gl == 0 && !(dkk > T(0))) flag_pivot(status, f.first_col + k);
-        const T d = sqrt(dkk);
-        const T inv = T(1) / d;
-        const T lik = (gl > k && gl < m) ? Fm[gl + k * LD] * inv : T(0);
-        if (gl == k) Fm[k + k * LD] = d;
-        if (gl > k && gl < m) Fm[gl + k * LD] = lik;
-        for (int j = k + 1; j < c; ++j) {
-            const T ljk = __shfl_sync(mask, lik, j, W);
-            if (gl >= j && gl < m) Fm[gl + j * LD] -= lik * ljk;
+    };
+    T v[CG];
+    int ri = 0;
+    auto fetch = [&]() {  // child h's columns j0 .., rows lane
+        if (h >= nb) return;
+        if (j0 == 0) {
+            uc = __shfl_sync(ALL, g_uc, h, W);
+            maxuc = __reduce_max_sync(ALL, uc);
+            const int* rm = relmap + __shfl_sync(ALL, g_rel, h, W);
+            ri = gl < uc ? rm[gl] : 0;
         }
-        __syncwarp(mask);
-    }
-    // Schur complement straight to the update store
-    if (f.uoff >= 0) {
-        T* Ud = Us + f.uoff;
-        for (int idx = gl; idx < u * u; idx += W) {
-            const int j = idx / u, i = idx - j * u;
-            if (i >= j) {
-                T acc = Fm[(c + i) + (c + j) * LD];
-                for (int k = 0; k < c; ++k) acc -= Fm[(c + i) + k * LD] * Fm[(c + j) + k * LD];
-                Ud[i + (int64_t)j * f.ldu] = acc;
+        const int ldu = __shfl_sync(ALL, g_ldu, h, W);
+        const T* U = Us + __shfl_sync(ALL, g_u, h, W);
+#pragma unroll
+        for (int e = 0; e < CG; ++e) {
+            v[e] = T(0);
+            if (gl < uc && gl >= j0 + e) v[e] = U[gl + (int64_t)(j0 + e) * ldu];
+        }
+    };
+    describe();
+    const T av = src >= 0 ? (T)Ax[src] : T(0);
+    nb = min(W, maxch);
+    fetch();
+    __syncwarp();
+    if (src >= 0) Fm[(pos & 0xffff) + (pos >> 16) * LD] = av;
+    const int na = __reduce_max_sync(ALL, f.a_end - f.a_beg);
+    for (int e0 = W; e0 < na; e0 += W) {
+        const int e = f.a_beg + e0 + gl;
+        if (e < f.a_end) {
+            src = a_src[e];
+            if (src >= 0) {
+                pos = a_pos[e];
+                Fm[(pos & 0xffff) + (pos >> 16) * LD] = (T)Ax[src];
             }
         }
     }
-    T* Ld = Ls + f.loff;
-    for (int idx = gl; idx < m * c; idx += W) {
-        const int j = idx / m, i = idx - j * m;
-        Ld[i + (int64_t)j * f.ldl] = (i >= j) ? Fm[i + j * LD] : T(0);
+    __syncwarp();
+    for (int hb = 0; hb < maxch;) {
+        while (h < nb) {
+            T w[CG];
+#pragma unroll
+            for (int e = 0; e < CG; ++e) w[e] = v[e];
+            const int cnt = uc, wi = ri, jb = j0;
+            j0 += CG;
+            if (j0 >= maxuc) ++h, j0 = 0;
+            fetch();
+            T* at[CG];  // distinct columns: all reads before the writes
+#pragma unroll
+            for (int e = 0; e < CG; ++e) {
+                at[e] = Fm + wi + __shfl_sync(ALL, wi, jb + e, W) * LD;
+                if (gl < cnt && gl >= jb + e) w[e] += *at[e];
+            }
+#pragma unroll
+            for (int e = 0; e < CG; ++e)
+                if (gl < cnt && gl >= jb + e) *at[e] = w[e];
+            __syncwarp();
+        }
+        hb += W;
+        if (hb >= maxch) break;
+        h = 0;
+        nb = min(W, maxch - hb);
+        g_id = hb + gl < nch ? child[f.child_beg + hb + gl] : -1;
+        describe();
+        fetch();
     }
-    __syncwarp(mask);  // the slice is reused by the group's next front
+    T a[W];
+#pragma unroll
+    for (int j = 0; j < W; ++j) a[j] = Fm[gl + j * LD];
+    const int maxc = __reduce_max_sync(ALL, c);
+#pragma unroll
+    for (int k = 0; k < W; ++k) {
+        if (k >= maxc) break;
+        const T piv = __shfl_sync(ALL, a[k], k, W);
+        T root, inv;
+        pivot_root(piv, root, inv);
+        if (k < c && gl == k && !(piv > T(0))) flag_pivot(status, f.first_col + k);
+        const T l = k < c && gl >= k ? a[k] * inv : T(0);
+        if (k < c) a[k] = gl == k ? root : l;
+#pragma unroll
+        for (int j = k + 1; j < W; ++j) a[j] -= l * __shfl_sync(ALL, l, j, W);
+    }
+    const int maxm = __reduce_max_sync(ALL, m);
+    T* pl = Ls + f.loff + gl;
+    T* pu = Us + f.uoff + (gl - c);
+#pragma unroll
+    for (int j = 0; j < W; ++j) {
+        if (j >= maxm) break;
+        const bool pivot = j < c;
+        if (j < m && gl < m && (pivot || (gl >= j && f.uoff >= 0)))
+            *(pivot ? pl : pu) = gl >= j ? a[j] : T(0);
+        if (pivot)
+            pl += f.ldl;
+        else
+            pu += f.ldu;
+    }
+    __syncwarp();  // the slice is reused by the group's next front
 }
 
 // One level's fronts of at most 32 rows as warp tasks over a rows-descending
@@ -192,25 +443,24 @@ __global__ void __launch_bounds__(128)
                   const int* __restrict__ a_src, const int* __restrict__ a_pos,
                   const double* __restrict__ Ax, T* __restrict__ Ls, T* __restrict__ Us,
                   int* __restrict__ status) {
-    constexpr int LD = kTinyFrontRows + 1;
+    constexpr int LD = small_ld<T>(kTinyFrontRows);
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, wpb = blockDim.x >> 5;
     T* slice = reinterpret_cast<T*>(smem_raw) + (size_t)warp * kTinyFrontRows * LD;
     const int t16 = (n16 + 1) / 2, t8 = (n8 + 3) / 4, ntask = n32 + t16 + t8;
     for (int t = blockIdx.x * wpb + warp; t < ntask; t += gridDim.x * wpb) {
         if (t < n32) {
-            tiny_front_group<T, 32>(list[t], fronts, child, relmap, a_src, a_pos, Ax, Ls, Us,
-                                    status, slice);
+            const FrontDesc f = fronts[list[t]];
+            small_front<T>(f, slice, LD, 0, 1, [] { __syncwarp(); }, fronts, child, relmap, a_src,
+                           a_pos, Ax, Ls, Us, status);
         } else if (t < n32 + t16) {
             const int k = 2 * (t - n32) + (lane >> 4);
-            if (k < n16)
-                tiny_front_group<T, 16>(list[n32 + k], fronts, child, relmap, a_src, a_pos, Ax,
-                                        Ls, Us, status, slice + (lane >> 4) * 16 * 17);
+            tiny_front_group<T, 16>(k < n16 ? list[n32 + k] : -1, fronts, child, relmap, a_src,
+                                    a_pos, Ax, Ls, Us, status, slice + (lane >> 4) * 16 * 17);
         } else {
             const int k = 4 * (t - n32 - t16) + (lane >> 3);
-            if (k < n8)
-                tiny_front_group<T, 8>(list[n32 + n16 + k], fronts, child, relmap, a_src, a_pos,
-                                       Ax, Ls, Us, status, slice + (lane >> 3) * 8 * 9);
+            tiny_front_group<T, 8>(k < n8 ? list[n32 + n16 + k] : -1, fronts, child, relmap, a_src,
+                                   a_pos, Ax, Ls, Us, status, slice + (lane >> 3) * 8 * 9);
         }
         __syncwarp();
     }
@@ -570,7 +820,7 @@ void launch_small_fronts(const DevPlan& D, int level, T* Ls, T* Us, const double
             for (int b = 0; b < Plan::kTinyBuckets; ++b)
                 by += D.h_small_bytes[level * kSmallBuckets + b];
             ProfScope ps(D.prof, KC_SMALL_FRONT, st, 0, by * sizeof(T) / 8.0);
-            const size_t smem = (size_t)4 * kTinyFrontRows * (kTinyFrontRows + 1) * sizeof(T);
+            const size_t smem = (size_t)4 * kTinyFrontRows * small_ld<T>(kTinyFrontRows) * sizeof(T);
             // the level's slice of the rows-descending warp list: its fronts
             // of 17..32 rows end the part above 16 rows, then 9..16, then <= 8
             const int* cnt = D.solve.warp_cnt.data() + 3 * level;
@@ -589,8 +839,8 @@ void launch_small_fronts(const DevPlan& D, int level, T* Ls, T* Us, const double
         int end = D.h_small_ptr[level * kSmallBuckets + b + 1];
         if (end == beg) continue;
         int MB = Plan::small_limit[b];
-        int LD = MB + 1;
-        size_t smem = (size_t)MB * LD * sizeof(T) + (size_t)MB * sizeof(int);
+        int LD = small_ld<T>(MB);
+        size_t smem = (size_t)MB * LD * sizeof(T);
         const int threads = D.small_threads[b];
         const cudaStream_t st = sts[1 + b - Plan::kTinyBuckets];
         ProfScope ps(D.prof, KC_SMALL_FRONT, st, 0,

@@ -162,9 +162,10 @@ struct DevPlan {
     // launch shapes of the small-front factor kernels, chosen by
     // mdgpu_autotune (these defaults otherwise): the tiny-front kernel's grid
     // cap (blocks of four warps) and the threads of k_small_front per size
-    // bucket
+    // bucket (16 warps where shared memory leaves one or two CTAs per SM: 256
+    // threads took 1.2 to 1.4 times as long there)
     int tiny_blocks_cap = 148 * 8;
-    int small_threads[kSmallBuckets] = {64, 128, 256, 256, 256, 256};
+    int small_threads[kSmallBuckets] = {64, 128, 128, 256, 512, 512};
     // the factor runs a level's small fronts beside its large fronts (both
     // depend only on lower levels), and the small fronts' pieces (the tiny
     // fronts, then each k_small_front size bucket) beside one another: a

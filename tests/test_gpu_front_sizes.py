@@ -23,6 +23,32 @@ SIZES = [(1, 2, 161), (33, 97, 64), (64, 65, 127), (63, 129, 128), (161, 31, 130
          (256, 257, 191), (300, 64, 257)]
 
 
+# leaves of the pivot columns given, under a root of u rows, all of them fronts
+# of at most 160 rows: the edges of the 8, 16 and 32 rows of a lane group, of the
+# eight-column panels, of the 32-row blocks; more children than a warp has lanes
+SMALL = [((1, 2, 7), 1), ((1, 3), 6), ((4, 1), 12), ((9, 1), 7), ((1,) * 70, 15), ((17, 8, 1), 24),
+         ((7, 8, 9), 23), ((1,) * 33 + (31, 32), 33), ((16, 64), 65), ((63, 1, 33), 96),
+         ((24, 95, 40), 64), ((1,) * 40 + (127,), 33), ((2, 80, 60), 80), ((1, 31), 129),
+         ((152,), 8), ((3, 5), 155)]
+
+
+def _leaves(cs, u, seed=0):
+    """Dense symmetric matrix of the pattern of the leaves, its lower CSC."""
+    beg = np.concatenate([[0], np.cumsum(cs)])
+    n = beg[-1] + u
+    leaf = np.concatenate([np.repeat(np.arange(len(cs)), cs), np.full(u, -1)])
+    r = np.random.default_rng(seed)
+    A = r.uniform(-1.0, 1.0, (n, n))
+    A = 0.5 * (A + A.T)
+    A[(leaf[:, None] != leaf[None, :]) & (leaf[:, None] >= 0) & (leaf[None, :] >= 0)] = 0.0
+    np.fill_diagonal(A, 1.5 * np.abs(A).sum(axis=1))
+    Ai = [j + np.flatnonzero((leaf[j:] == leaf[j]) | (leaf[j:] < 0)) for j in range(n)]
+    cols = np.repeat(np.arange(n), [len(a) for a in Ai])
+    Ap = np.concatenate([[0], np.cumsum([len(a) for a in Ai])])
+    Ai = np.concatenate(Ai)
+    return n, A, Ap.astype(np.int32), Ai.astype(np.int32), A[Ai, cols]
+
+
 def _two_leaves(c1, c2, u, seed=0):
     """Dense symmetric matrix of the two-leaf pattern and its lower CSC."""
     n = c1 + c2 + u
@@ -132,3 +158,14 @@ def test_reverse_mode(c1, c2, u):
     cols = np.repeat(np.arange(n), np.diff(Ap))
     ref = H[Ai, cols] * np.where(Ai == cols, 1.0, 2.0)
     assert np.linalg.norm(S.adjoint(lbar) - ref) <= 1e-11 * np.linalg.norm(ref)
+
+
+# tolerances as for the large fronts' factors above (n below 250 here)
+@pytest.mark.parametrize("cs,u", SMALL)
+@pytest.mark.parametrize("prec,tol", [(M.FP64, 1e-12), (M.FP32, 2e-5)])
+def test_small_fronts(cs, u, prec, tol):
+    n, A, Ap, Ai, Ax = _leaves(cs, u)
+    S = M.Solver(n, Ap, Ai, ordering=M.ORDER_NATURAL)
+    S.factor(torch.from_numpy(Ax).cuda(), prec)
+    ref = np.linalg.cholesky(A)
+    assert np.linalg.norm(_dense_L(S) - ref) <= tol * np.linalg.norm(ref)
