@@ -119,8 +119,7 @@ __device__ bool poll_published(double* dst, const double* src, int nk, int nrhs,
 }
 
 // NQ neighbouring published values p[0 .. nq - 1]: a first look (the loads of
-// several places are issued together), then the wait for the ones not there
-// yet, each thread for its own, with a short sleep between the looks.
+// several places are issued together).
 template <int NQ>
 __device__ __forceinline__ void peek_values(const double* p, bool need, int nq, double (&v)[NQ]) {
 #pragma unroll
@@ -129,29 +128,9 @@ __device__ __forceinline__ void peek_values(const double* p, bool need, int nq, 
         if (need && q < nq) v[q] = ld_relaxed_f64(p + q);
     }
 }
-template <int NQ>
-__device__ __forceinline__ void await_values(const double* p, int nq, double (&v)[NQ],
-                                             const SolveAbort& ab) {
-    for (int it = 1;; ++it) {
-        bool miss = false;
-#pragma unroll
-        for (int q = 0; q < NQ; ++q) miss = miss || is_unpublished(v[q]);
-        if (!miss) return;
-        if (it > 2) __nanosleep(it < 64 ? 40 : 200);
-        if ((it & 15) == 0) {
-            if (it >= kSolveWaitPolls) {
-                atomicExch(ab.flag, 1);
-                atomicOr(ab.err, 1);
-            }
-            if (ld_relaxed_gpu(ab.flag)) return;
-        }
-#pragma unroll
-        for (int q = 0; q < NQ; ++q)
-            if (is_unpublished(v[q])) v[q] = ld_relaxed_f64(p + q);
-    }
-}
 
-// The same for the lanes of `mask` together (converged), each with values from
+// Then the wait for the ones not there yet, with a short sleep between the
+// looks, by the lanes of `mask` together (converged), each with values from
 // R places: the rounds are uniform, so the lanes leave converged.  After loops
 // of their own lanes ran the rest of a front in pieces, also past a
 // __syncwarp, and every shuffle waited about 500 cycles for the pieces to meet
@@ -252,7 +231,7 @@ __device__ __forceinline__ void load_block_async(TL* dst, const TL* src, int64_t
 }
 
 // ---------------------------------------------------------------------------
-// large-front tile tasks: a pipeline of two stages streams the L blocks a
+// large-front tile tasks: a pipeline of two or three stages streams the L blocks a
 // task multiplies, each with the vector block it is multiplied by (a pivot
 // tile's published solution, or gathered solution rows), by cp.async; the
 // block in use is consumed while the next ones load.  Published vectors come
@@ -260,7 +239,12 @@ __device__ __forceinline__ void load_block_async(TL* dst, const TL* src, int64_t
 // sentinel falls back to polling that slot.
 // ---------------------------------------------------------------------------
 
-constexpr int kSolveStages = 2;
+// three where they leave three CTAs per SM: one right-hand side, FP32 (two: 3.66 +
+// 3.26 ms in twelve solves of the 24^3 three-unknown grid, three: 3.51 + 3.23)
+template <typename TL, bool MULTI>
+__host__ __device__ constexpr int solve_stages() {
+    return sizeof(TL) == 4 && !MULTI ? 3 : 2;
+}
 
 // shared memory of a tile task: the stages' L blocks, their vector blocks, a
 // vector, the gather's row indices; one right-hand side also keeps the
@@ -268,13 +252,15 @@ constexpr int kSolveStages = 2;
 // after the last L block)
 template <typename TL, bool MULTI>
 __host__ __device__ constexpr size_t level_smem_bytes() {
-    return ((size_t)(kSolveStages + (MULTI ? 0 : 1)) * kTile * blk_ld<TL>()) * sizeof(TL) +
-           (size_t)(kSolveStages + 1) * kVecLD * (MULTI ? kGroupRhs : 1) * sizeof(double) +
+    return ((size_t)(solve_stages<TL, MULTI>() + (MULTI ? 0 : 1)) * kTile * blk_ld<TL>()) *
+               sizeof(TL) +
+           (size_t)(solve_stages<TL, MULTI>() + 1) * kVecLD * (MULTI ? kGroupRhs : 1) * sizeof(double) +
            (size_t)SolveScheduleHost::kGatherTiles * kTile * sizeof(int);
 }
 
 template <typename TL, bool MULTI>
 struct LevelSmem {
+    static constexpr int S = solve_stages<TL, MULTI>();
     static constexpr int VB = kVecLD * (MULTI ? kGroupRhs : 1);
     TL* Lst;      // stages x T x LD
     TL* Dk;       // T x LD (one right-hand side)
@@ -285,13 +271,13 @@ struct LevelSmem {
         constexpr int T = kTile, LD = blk_ld<TL>();
         extern __shared__ __align__(16) unsigned char smem_raw[];
         Lst = reinterpret_cast<TL*>(smem_raw);
-        Dk = Lst + kSolveStages * T * LD;
+        Dk = Lst + S * T * LD;
         Vst = reinterpret_cast<double*>(Dk + (MULTI ? 0 : T * LD));
-        Y = Vst + kSolveStages * VB;
+        Y = Vst + S * VB;
         idx = reinterpret_cast<int*>(Y + VB);
     }
-    __device__ TL* lb(int p) const { return Lst + (p % kSolveStages) * kTile * blk_ld<TL>(); }
-    __device__ double* vb(int p) const { return Vst + (p % kSolveStages) * VB; }
+    __device__ TL* lb(int p) const { return Lst + (p % S) * kTile * blk_ld<TL>(); }
+    __device__ double* vb(int p) const { return Vst + (p % S) * VB; }
 };
 
 // a published T x nrhs slot into a stage (16-byte copies through L2; T * nrhs
@@ -322,24 +308,49 @@ __device__ __forceinline__ bool settle_slot(double* v, const double* src, int nk
     return poll_published(v, src, nk, nrhs, ab);
 }
 
+// Forward, one right-hand side, 64 x 64 blocks: thread (row r, phase g) sums
+// over the column pairs 8 u + 2 g, + 1: no bank conflicts between the phases,
+// the vector in 16-byte reads, four chains of sums (an FP64 multiply-add takes
+// about 40 cycles to the next one that needs it, so one chain of 16 took 640
+// of a tile's 3400 cycles, twice; 1.90 -> 1.75 us per tile of a chain, FP64).
+// The backward sweep's column-wise reads conflict that way, and it keeps one
+// chain.  B: the thread's row.
+template <typename TL>
+__device__ __forceinline__ double row_dot(const TL* B, const double* V, int g) {
+    constexpr int LD = blk_ld<TL>();
+    double a[4] = {};
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+        const double2 v = *reinterpret_cast<const double2*>(V + 8 * u + 2 * g);
+        a[u & 3] += (double)B[(8 * u + 2 * g) * LD] * v.x;
+        a[u & 3] += (double)B[(8 * u + 2 * g + 1) * LD] * v.y;
+    }
+    return (a[0] + a[1]) + (a[2] + a[3]);
+}
+
 // x[q] += the front-vector rows that the assembly map adds into a row (fv row
 // e at fv + e * nrhs; NQ neighbouring right-hand sides), in child order, every
-// entry waited for, two in flight.  ar: the row's entry range.
+// entry waited for, two in flight; a whole warp together, lanes with need
+// (ar: the row's entry range) and without.
 template <int NQ>
-__device__ __forceinline__ void gather_entries(const int* ar, const int* __restrict__ amap_ent,
-                                               const double* fv, int nrhs, int nq, double (&x)[NQ],
+__device__ __forceinline__ void gather_entries(bool need, const int* ar,
+                                               const int* __restrict__ amap_ent, const double* fv,
+                                               int nrhs, int nq, double (&x)[NQ],
                                                const SolveAbort& ab) {
-    const int e1 = ar[1];
-    for (int e = ar[0]; e < e1; e += 2) {
-        const double* p0 = fv + (int64_t)amap_ent[e] * nrhs;
-        const double* p1 = e + 1 < e1 ? fv + (int64_t)amap_ent[e + 1] * nrhs : p0;
-        double v[NQ], w[NQ];
-        peek_values<NQ>(p0, true, nq, v);
-        peek_values<NQ>(p1, e + 1 < e1, nq, w);
-        await_values<NQ>(p0, nq, v, ab);
-        await_values<NQ>(p1, nq, w, ab);
+    int e = 0, e1 = 0;
+    if (need) e = ar[0], e1 = ar[1];
+    const int rounds = __reduce_max_sync(0xffffffffu, e1 - e);
+    for (int k = 0; k < rounds; k += 2, e += 2) {
+        const double* p[2] = {fv, fv};
+        double v[2][NQ];
 #pragma unroll
-        for (int q = 0; q < NQ; ++q) x[q] = (x[q] + v[q]) + w[q];
+        for (int i = 0; i < 2; ++i) {
+            if (e + i < e1) p[i] += (int64_t)amap_ent[e + i] * nrhs;
+            peek_values<NQ>(p[i], e + i < e1, nq, v[i]);
+        }
+        await_together<2, NQ>([&](int i) { return p[i]; }, nq, v, 0xffffffffu, ab);
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) x[q] = (x[q] + v[0][q]) + v[1][q];
     }
 }
 
@@ -384,9 +395,9 @@ __device__ void fwd_tile_task(int2 tk, const FrontDesc* __restrict__ fronts,
     auto gather_row = [&](int i) -> double {
         const TileRange ti = tile_range(i, F.m, F.c, T);
         const int R = ti.start + r;
-        if (g != 0 || r >= ti.size) return 0.0;
-        double x[1] = {R < F.c ? xp[F.first_col + R] : 0.0};
-        gather_entries<1>(amap_row + aoff + R, amap_ent, fv, 1, 1, x, ab);
+        const bool own = g == 0 && r < ti.size;
+        double x[1] = {own && R < F.c ? xp[F.first_col + R] : 0.0};
+        gather_entries<1>(own, amap_row + aoff + R, amap_ent, fv, 1, 1, x, ab);
         return x[0];
     };
     auto issue = [&](int p) {
@@ -403,13 +414,13 @@ __device__ void fwd_tile_task(int2 tk, const FrontDesc* __restrict__ fronts,
         const TileRange ti = tile_range(i0, F.m, F.c, T);
         load_block_async(sm.Dk, Dinv + dinv_off[s] + (int64_t)i0 * T * T, T, 0, ti.size, ti.size);
     }
-    issue(0);
+    for (int p = 0; p + 1 < sm.S; ++p) issue(p);
     double fcur = gather_row(i0), acc = 0.0;
     double fnext = cnt > 1 ? gather_row(i0 + 1) : 0.0;
     bool ok = true;
     for (int p = 0; p < P; ++p) {
-        issue(p + 1);
-        cp_async_wait_groups<1>();
+        issue(p + sm.S - 1);
+        cp_async_wait_groups<sm.S - 1>();
         __syncthreads();
         const int i = i0 + p / kend, k = p % kend;
         double* Yk = sm.vb(p);
@@ -417,9 +428,7 @@ __device__ void fwd_tile_task(int2 tk, const FrontDesc* __restrict__ fronts,
             ok = false;
             break;
         }
-        const TL* B = sm.lb(p);
-#pragma unroll
-        for (int l = 0; l < 16; ++l) acc += (double)B[db + r + (g + 4 * l) * LD] * Yk[g + 4 * l];
+        acc += row_dot(sm.lb(p) + db + r, Yk, g);
         if (!pivot && k == kend - 1) {  // update tile i complete: f_i - acc to the front vector
             const TileRange ti = tile_range(i, F.m, F.c, T);
             double v = acc + __shfl_xor_sync(0xffffffffu, acc, 8);
@@ -438,14 +447,11 @@ __device__ void fwd_tile_task(int2 tk, const FrontDesc* __restrict__ fronts,
     // same way
     const TileRange ti = tile_range(i0, F.m, F.c, T);
     double* Y = sm.Y;
-    const TL* Dk = sm.Dk;
     double a = acc + __shfl_xor_sync(0xffffffffu, acc, 8);
     a += __shfl_xor_sync(0xffffffffu, a, 16);
     if (g == 0) Y[r] = r < ti.size ? fcur - a : 0.0;
     __syncthreads();
-    double y = 0.0;
-#pragma unroll
-    for (int l = 0; l < 16; ++l) y += (double)Dk[r + (g + 4 * l) * LD] * Y[g + 4 * l];
+    double y = row_dot(sm.Dk + r, Y, g);
     y += __shfl_xor_sync(0xffffffffu, y, 8);
     y += __shfl_xor_sync(0xffffffffu, y, 16);
     if (g == 0 && r < ti.size) {
@@ -516,14 +522,14 @@ __device__ void fwd_tile_group(int2 tk, const FrontDesc* __restrict__ fronts,
     auto gather_row = [&](int i, double (&v)[2]) {
         const TileRange ti = tile_range(i, F.m, F.c, T);
         const int R = ti.start + r;
+        const bool own = r < ti.size && q0;
         v[0] = v[1] = 0.0;
-        if (r >= ti.size || !q0) return;
-        if (R < F.c) {
+        if (own && R < F.c) {
             const double* x = xp + (int64_t)(F.first_col + R) * nrhs + q;
             v[0] = x[0];
             if (q1) v[1] = x[1];
         }
-        gather_entries<2>(amap_row + aoff + R, amap_ent, fv + q, nrhs, q1 ? 2 : 1, v, ab);
+        gather_entries<2>(own, amap_row + aoff + R, amap_ent, fv + q, nrhs, q1 ? 2 : 1, v, ab);
     };
     auto issue = [&](int p) {
         if (p < P) {
@@ -538,14 +544,14 @@ __device__ void fwd_tile_group(int2 tk, const FrontDesc* __restrict__ fronts,
         }
         cp_async_commit_group();
     };
-    issue(0);
+    for (int p = 0; p + 1 < sm.S; ++p) issue(p);
     double fcur[2], fnext[2] = {0.0, 0.0}, acc[2][2] = {};
     gather_row(i0, fcur);
     if (cnt > 1) gather_row(i0 + 1, fnext);
     bool ok = true;
     for (int p = 0; p < P; ++p) {
-        issue(p + 1);
-        cp_async_wait_groups<1>();
+        issue(p + sm.S - 1);
+        cp_async_wait_groups<sm.S - 1>();
         __syncthreads();
         const int i = i0 + p / kend, k = p % kend;
         if (!settle_slot(sm.vb(p), pb + (int64_t)k * T * nrhs, min(T, F.c - k * T), nrhs, ab)) {
@@ -632,10 +638,10 @@ __device__ void bwd_gather_task(int2 tk, const FrontDesc* __restrict__ fronts,
         }
         cp_async_commit_group();
     };
-    issue(0);
+    for (int p = 0; p + 1 < sm.S; ++p) issue(p);
     if (tid < 32) await_parent(pcol, xs, nrhs, ab);
     __syncthreads();
-    // two stages: the L blocks by cp.async; the ancestors' solution rows, as
+    // the stages: the L blocks by cp.async; the ancestors' solution rows, as
     // they are published, into registers one stage ahead, stored into their
     // stage after the previous stage's products
     constexpr int VPT = MULTI ? kTile * kGroupRhs / 256 : 1;
@@ -649,8 +655,7 @@ __device__ void bwd_gather_task(int2 tk, const FrontDesc* __restrict__ fronts,
             src[k] = xs + (int64_t)max(row, 0) * nrhs + e / T;
             peek_values<1>(src[k], row >= 0, 1, pend[k]);
         }
-#pragma unroll
-        for (int k = 0; k < VPT; ++k) await_values<1>(src[k], 1, pend[k], ab);
+        await_together<VPT, 1>([&](int k) { return src[k]; }, 1, pend, 0xffffffffu, ab);
     };
     auto put = [&](int p) {
         if (p >= P) return;
@@ -661,14 +666,13 @@ __device__ void bwd_gather_task(int2 tk, const FrontDesc* __restrict__ fronts,
             if (e < T * nrhs) v[(e / T) * kVecLD + (e & (T - 1))] = pend[k][0];
         }
     };
-    static_assert(kSolveStages == 2, "the gather's vector pipeline has two stages");
     fetch(0);
     put(0);
     double acc[2][2] = {};
     for (int p = 0; p < P; ++p) {
-        issue(p + 1);
+        issue(p + sm.S - 1);
         fetch(p + 1);
-        cp_async_wait_groups<1>();
+        cp_async_wait_groups<sm.S - 1>();
         __syncthreads();
         const TL* Bk = sm.lb(p);
         const double* X = sm.vb(p);
@@ -1096,7 +1100,7 @@ __device__ void bwd_chain_task(int2 tk, const FrontDesc* __restrict__ fronts,
         cp_async_commit_group();
     };
     if (!MULTI) load_inv(sm.Dk);
-    issue(0);
+    for (int p = 0; p + 1 < sm.S; ++p) issue(p);
     double acc[2][2] = {};
     // this tile's y_j, before the first wait
     const int64_t xj = F.first_col + tj.start + l;
@@ -1115,17 +1119,15 @@ __device__ void bwd_chain_task(int2 tk, const FrontDesc* __restrict__ fronts,
 #pragma unroll
             for (int k = 0; k < 2 * NP; ++k)
                 peek_values<1>(at(k), (k % NP == 0 ? own0 : own1) && h + k / NP < nch, 1, v[k]);
+            await_together<2 * NP, 1>(at, 1, v, 0xffffffffu, ab);
 #pragma unroll
-            for (int k = 0; k < 2 * NP; ++k) {
-                await_values<1>(at(k), 1, v[k], ab);
-                acc[0][k % NP] += v[k][0];
-            }
+            for (int k = 0; k < 2 * NP; ++k) acc[0][k % NP] += v[k][0];
         }
     }
     bool ok = true;
     for (int p = 0; p < P; ++p) {
-        issue(p + 1);
-        cp_async_wait_groups<1>();
+        issue(p + sm.S - 1);
+        cp_async_wait_groups<sm.S - 1>();
         __syncthreads();
         const int k = nt1 - 1 - p;
         double* X = sm.vb(p);
@@ -1241,7 +1243,7 @@ __device__ void fwd_update_rt1(int s, int R0, int R1, const FrontDesc& F, double
     TL lv[GW], ln[GW];
     load(0, lv);
     double f0[1] = {0.0};
-    if (rv) gather_entries<1>(amap_row + amap_off[s] + R, amap_ent, fv, 1, 1, f0, ab);
+    gather_entries<1>(rv, amap_row + amap_off[s] + R, amap_ent, fv, 1, 1, f0, ab);
     for (int cg = 0; cg < ng; ++cg) {
         if (cg + 1 < ng) load(cg + 1, ln);
         const int k = cg / GPB;
@@ -1281,9 +1283,9 @@ struct SolveGroups {
     __device__ int64_t fv_off(int g) const { return kGroupRhs * fv_total * g; }
 };
 
-// residency by shared memory: one right-hand side keeps three blocks of L per
-// CTA (FP32 55 KB, FP64 107 KB), a group two and its vectors (49 and 84 KB);
-// by registers (the small fronts' columns of L): three CTAs
+// residency by shared memory: one right-hand side keeps the stages' blocks of L
+// and an inverse per CTA (FP32 four blocks, 72 KB, FP64 three, 107 KB), a group
+// two and its vectors (49 and 84 KB); by registers (the small fronts' columns of L): three CTAs
 template <typename TL>
 constexpr int solve_ctas_per_sm() {
     return sizeof(TL) == 8 ? 2 : 3;
