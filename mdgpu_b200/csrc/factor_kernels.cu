@@ -790,6 +790,23 @@ __global__ void __launch_bounds__(256)
     }
 }
 
+// Columns c0 .. of L into compressed columns, a warp per column.
+template <typename T>
+__global__ void __launch_bounds__(256)
+    k_pack_columns(const FrontDesc* __restrict__ fronts, const int* __restrict__ col_front,
+                   const int64_t* __restrict__ Lp, const T* __restrict__ Ls, int c0, int c1,
+                   double* __restrict__ out) {
+    const int lane = threadIdx.x & 31;
+    for (int col = c0 + (int)(blockIdx.x * 8 + (threadIdx.x >> 5)); col < c1;
+         col += gridDim.x * 8) {
+        const FrontDesc& f = fronts[col_front[col]];
+        const int j = col - f.first_col, m = f.m;
+        const T* src = Ls + f.loff + (int64_t)j * f.ldl;
+        double* dst = out + (Lp[col] - Lp[c0]) - j;
+        for (int i = j + lane; i < m; i += 32) dst[i] = (double)src[i];
+    }
+}
+
 // ---------------------------------------------------------------------------
 // host launchers
 // ---------------------------------------------------------------------------
@@ -968,6 +985,16 @@ static void launch_large_level_panels(const DevPlan& D, int level, T* Ls, T* Us,
         }
     }
 }
+
+template <typename T>
+void pack_columns(const DevPlan& D, const T* Ls, int c0, int c1, double* out, cudaStream_t st) {
+    const int sms = D.num_sms > 0 ? D.num_sms : 148;
+    k_pack_columns<T><<<std::min((c1 - c0 + 7) / 8, 8 * sms), 256, 0, st>>>(
+        D.fronts, D.adj.col_front, D.adj.Lp, Ls, c0, c1, out);
+}
+template void pack_columns<double>(const DevPlan&, const double*, int, int, double*,
+                                   cudaStream_t);
+template void pack_columns<float>(const DevPlan&, const float*, int, int, double*, cudaStream_t);
 
 template <typename T>
 static void set_factor_attributes() {

@@ -152,6 +152,7 @@ struct AdjSchedule {
     int* before = nullptr;
     std::vector<WorkList> h_gather;  // per level
     int64_t* Lp = nullptr;
+    int* col_front = nullptr;  // the front of each column of L
     int64_t* woff = nullptr;
     int64_t wtotal = 0;
 };
@@ -245,6 +246,11 @@ struct DevPlan {
 // one-time kernel attribute setup (dynamic shared memory limits); must run
 // before any launch sequence is captured into a CUDA graph
 void init_factor_kernels();
+
+// The columns [c0, c1) of L as doubles, packed (the rows on and below the
+// diagonal, column after column) into out.
+template <typename T>
+void pack_columns(const DevPlan& D, const T* Ls, int c0, int c1, double* out, cudaStream_t st);
 void init_solve_kernels();
 void init_schur_tc();
 void init_schur_f64();

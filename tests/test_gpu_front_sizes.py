@@ -169,3 +169,24 @@ def test_small_fronts(cs, u, prec, tol):
     S.factor(torch.from_numpy(Ax).cuda(), prec)
     ref = np.linalg.cholesky(A)
     assert np.linalg.norm(_dense_L(S) - ref) <= tol * np.linalg.norm(ref)
+
+
+# L's columns are packed on the device 8 M values at a time: above that, several
+# rounds.  ||L L' v - A v|| <= (m + 1) eps || |L| |L'| |v| || for a factor with m
+# terms per row sum; rows of L here hold below 1e4 terms.
+@pytest.mark.parametrize("prec,eps", [(M.FP64, 2.0 ** -52), (M.FP32, 2.0 ** -23)])
+def test_get_L_in_rounds(prec, eps):
+    sp = pytest.importorskip("scipy.sparse")
+    from mdgpu_b200 import matgen as mg
+    n, Ap, Ai, Ax = mg.laplacian_3d_varcoef(36)
+    S = M.Solver(n, Ap, Ai)
+    S.factor(np.asarray(Ax, np.float64), prec)
+    Lp, Li, Lx = S.get_L()
+    assert Lp[-1] > 8 << 20
+    L = sp.csc_matrix((Lx, Li, Lp), shape=(n, n))
+    A = mg.lower_to_full_scipy(n, Ap, Ai, Ax).tocsr()
+    p = S.array("perm")  # new -> old
+    v = np.random.default_rng(3).uniform(-1.0, 1.0, n)
+    r = L @ (L.T @ v) - A[p][:, p] @ v
+    bound = 1e4 * eps * (abs(L) @ (abs(L).T @ abs(v)))
+    assert (np.abs(r) <= bound).all()
