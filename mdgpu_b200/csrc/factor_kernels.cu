@@ -40,14 +40,12 @@ namespace mdgpu {
 // of 149 columns FP64 478 us, now 85.)  What is left of a level of a few tiny
 // fronts, 4 to 8 us, is mostly its cold instructions: about ten cycles each.
 
-// sqrt(x) and 1 / sqrt(x) from one reciprocal square root, each corrected by
-// one Newton step (infinity keeps its own)
+// (correctly rounded both: a reciprocal square root with a Newton step for each
+// took 1 to 2 % less of the kernels' time, and moved L by roundings)
 template <typename T>
 __device__ __forceinline__ void pivot_root(T x, T& root, T& inv) {
-    const T y = recip_sqrt(x), s = x * y;
-    const T h = T(0.5) * y;
-    inv = y == T(0) ? y : fma(h, fma(-s, y, T(1)), y);
-    root = y == T(0) ? x : fma(h, fma(-s, s, x), s);
+    root = sqrt(x);
+    inv = T(1) / root;
 }
 
 // 8 neighbouring elements on 16 bytes
