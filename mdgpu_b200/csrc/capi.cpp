@@ -349,9 +349,8 @@ void upload_plan(mdgpu_handle_s* h, bool check = false) {
         std::vector<int> ll(std::max(P.nsuper, 1)), nxt(D.h_level_ptr.begin(), D.h_level_ptr.end() - 1);
         for (int s = 0; s < P.nsuper; ++s) ll[nxt[lv[s]]++] = s;
         D.level_list = h->keep(upload(ll));
-        // Y scratch: m x 16 for a small front (one CTA), 2 m x 64 for a
-        // large one (Y of the even and the odd block steps); a level's
-        // fronts side by side, levels reuse it
+        // Y scratch of the large fronts, 2 m x 64 (Y of the even and the odd
+        // block steps); a level's fronts side by side, levels reuse it
         std::vector<char> large(P.nsuper, 0);
         for (int s : P.large_list) large[s] = 1;
         std::vector<int64_t> yo(P.nsuper, 0);
@@ -361,7 +360,7 @@ void upload_plan(mdgpu_handle_s* h, bool check = false) {
             for (int q = D.h_level_ptr[l]; q < D.h_level_ptr[l + 1]; ++q) {
                 const int s = ll[q];
                 yo[s] = off;
-                off += (int64_t)P.fronts[s].m * (large[s] ? 2 * selinv_tile() : selinv_block());
+                if (large[s]) off += (int64_t)P.fronts[s].m * 2 * selinv_tile();
             }
             D.yscr_total = std::max(D.yscr_total, off);
         }

@@ -325,7 +325,6 @@ void launch_adjoint(const DevPlan& D, int nnz, const double* Ls, const double* D
                     const double* Lbar, double* Fb, double* Fu, double* Wscr, double* part,
                     double* Abar, cudaStream_t st);
 int64_t adjoint_parts(const DevPlan& D);
-int selinv_block();  // pivot columns per block of the one-CTA (small-front) kernel
 int selinv_tile();   // pivot columns per block step of the large fronts
 
 }  // namespace mdgpu

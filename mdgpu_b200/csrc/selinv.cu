@@ -12,8 +12,8 @@
 // blocks, its update part Z_UU is the parent front's Z on the front's update
 // rows (gathered through the relative map -- the transpose of the
 // extend-add).  So the fronts are processed level by level from the root:
-// small fronts one CTA each (blocks of 16 columns), large fronts in blocks of
-// 64 columns over many CTAs per front (below); Z of the pivot columns goes to
+// small fronts a CTA or a warp each (blocks of 8 columns), large fronts in blocks
+// of 64 columns over many CTAs per front (below); Z of the pivot columns goes to
 // a store laid out like the L panels, Z_UU to the selected inverse's own
 // update store.
 //
@@ -32,8 +32,6 @@
 
 namespace mdgpu {
 
-constexpr int kSelBlock = 16;  // pivot columns per block of the recurrence
-
 // Z(r, col), r >= col, front-local indices of front f
 // (Z's update part of front f at zoff in the Zu store)
 __device__ __forceinline__ double& zelem(double* Zs, double* Zu, const FrontDesc& f,
@@ -42,96 +40,217 @@ __device__ __forceinline__ double& zelem(double* Zs, double* Zu, const FrontDesc
     return Zu[zoff + (r - f.c) + (int64_t)(col - f.c) * f.ldu];
 }
 
-__global__ void __launch_bounds__(256, 2)
-    k_selinv_front(const FrontDesc* __restrict__ fronts, const int* __restrict__ list,
-                   const int* __restrict__ relmap, const double* __restrict__ Ls,
-                   double* __restrict__ Zs, double* __restrict__ Zu,
-                   const int64_t* __restrict__ zuoff, double* __restrict__ Yscr,
-                   const int64_t* __restrict__ yoff) {
-    constexpr int NB = kSelBlock;
-    __shared__ double Lk[NB][NB + 1];
-    __shared__ double Wk[NB][NB + 1];
-    const int tid = threadIdx.x, nt = blockDim.x;
-    const int s = list[blockIdx.x];
+// Small fronts, the recurrence in blocks of eight pivot columns with the whole
+// symmetric Z of the front in shared memory: most have one to a few pivot
+// columns, so the gather of Z_UU from the parent is most of the work -- a warp
+// takes eight of its columns at a time, lane = row, all loads before the
+// stores.  Y = L_RK inv(L_KK) is a substitution per row (thread = row); Z_RK
+// = -Z_RR Y takes lane = row, Z's columns read side by side and Y's rows
+// broadcast, the sum over R split over the warps that the rows leave; Z_KK
+// takes a warp per entry.  (A CTA per front straight on global memory, a
+// column of the gather at a time, took 3.77 ms on a 32^3 grid; now 1.77, 1.5 of
+// it in the fronts of more than 32 rows, the pieces beside each other.)
+// Z: MB columns of MB + 1; Y: rows of kSelYS; P: partial sums, `slices` of them
+// where the rows leave warps (1: none); SM: L_KK and inv(L_KK), 8 x 8 in rows
+// of 9.
+constexpr int kSelNB = 8;
+constexpr int kSelYS = kSelNB + 2;  // 16-byte rows, fewer conflicts than 8
+constexpr int kSelLD = 9;
+constexpr int kSelSm = 2 * kSelNB * kSelLD;
+
+template <typename Sync>
+__device__ __forceinline__ void sel_small_front(int s, double* Z, int LD, double* Y, double* P,
+                                                int max_slices, double* SM, int warp, int nw,
+                                                Sync&& sync, const FrontDesc* __restrict__ fronts,
+                                                const int* __restrict__ relmap,
+                                                const double* __restrict__ Ls,
+                                                double* __restrict__ Zs, double* __restrict__ Zu,
+                                                const int64_t* __restrict__ zuoff) {
+    constexpr int NB = kSelNB;
+    constexpr unsigned ALL = 0xffffffffu;
+    const int lane = threadIdx.x & 31, tid = 32 * warp + lane;
     const FrontDesc f = fronts[s];
     const int m = f.m, c = f.c, u = m - c;
-    const int64_t zf = (f.parent >= 0 && u > 0) ? zuoff[s] : -1;
+    double *Lk = SM, *Wk = SM + NB * kSelLD;
+    // this thread's row of the block's columns of L, and its entry of L_KK
+    double l[NB], lk = 0.0;
+    auto load = [&](int k0) {
+        const int k1 = min(k0 + NB, c), r = k1 + tid;
+#pragma unroll
+        for (int k = 0; k < NB; ++k) {
+            l[k] = 0.0;
+            if (k0 + k < c && r < m) l[k] = Ls[f.loff + r + (int64_t)(k0 + k) * f.ldl];
+        }
+    };
+    auto load_diag = [&](int k0) {
+        for (int e = tid; e < NB * NB; e += 32 * nw) {
+            const int i = e & (NB - 1), j = e / NB;
+            lk = 0.0;
+            if (k0 + i < c && i >= j) lk = Ls[f.loff + k0 + i + (int64_t)(k0 + j) * f.ldl];
+            Lk[i * kSelLD + j] = lk;
+        }
+    };
+    load((c - 1) & ~(NB - 1));
     // the update part: the parent's Z on this front's update rows
     if (f.parent >= 0 && u > 0) {
         const FrontDesc p = fronts[f.parent];
-        const int64_t zp = zuoff[f.parent];
+        const int64_t zp = zuoff[f.parent], zf = zuoff[s];
         const int* rm = relmap + f.rows_off + c;
-        for (int b = 0; b < u; ++b) {
-            const int pb = rm[b];
-            for (int a = b + tid; a < u; a += nt)
-                Zu[zf + a + (int64_t)b * f.ldu] = zelem(Zs, Zu, p, zp, rm[a], pb);
-        }
-        __syncthreads();
-    }
-    double* Y = Yscr + yoff[s];  // (m - k1) x NB, row-major
-    const double* L = Ls + f.loff;
-    const int nblk = (c + NB - 1) / NB;
-    for (int kb = nblk - 1; kb >= 0; --kb) {
-        const int k0 = kb * NB, k1 = min(k0 + NB, c), nb = k1 - k0;
-        // W = inv(L_KK): a column per thread, forward substitution
-        for (int e = tid; e < NB * NB; e += nt) {
-            const int i = e % NB, j = e / NB;
-            Lk[i][j] = (i < nb && j < nb && i >= j) ? L[(k0 + i) + (int64_t)(k0 + j) * f.ldl] : 0.0;
-        }
-        __syncthreads();
-        if (tid < NB) {
-            const int j = tid;
-            for (int i = 0; i < NB; ++i) {
-                double v = 0.0;
-                if (i < nb && j < nb && i >= j) {
-                    v = (i == j) ? 1.0 : 0.0;
-                    for (int k = j; k < i; ++k) v -= Lk[i][k] * Wk[k][j];
-                    v /= Lk[i][i];
+        for (int j0 = NB * warp; j0 < u; j0 += NB * nw) {
+            const int rj = j0 + (lane & 7) < u ? rm[j0 + (lane & 7)] : 0;
+            for (int i0 = j0 & ~31; i0 < u; i0 += 32) {
+                const int i = i0 + lane;
+                const int ri = i < u ? rm[i] : 0;
+                double v[NB];
+#pragma unroll
+                for (int e = 0; e < NB; ++e) {
+                    const int col = __shfl_sync(ALL, rj, e);
+                    v[e] = 0.0;
+                    if (i < u && i >= j0 + e) v[e] = zelem(Zs, Zu, p, zp, ri, col);
                 }
-                Wk[i][j] = v;
+#pragma unroll
+                for (int e = 0; e < NB; ++e) {
+                    const int j = j0 + e;
+                    if (i >= u || i < j) continue;
+                    Z[(c + i) + (c + j) * LD] = Z[(c + j) + (c + i) * LD] = v[e];
+                    Zu[zf + i + (int64_t)j * f.ldu] = v[e];
+                }
             }
         }
-        __syncthreads();
-        // Y = L_RK W, a row per thread
-        for (int a = k1 + tid; a < m; a += nt) {
-            double l[NB];
+    }
+    for (int k0 = (c - 1) & ~(NB - 1); k0 >= 0; k0 -= NB) {
+        const int k1 = min(k0 + NB, c), nb = k1 - k0, nR = m - k1;
+        load_diag(k0);
+        sync();
+        // Y = L_RK inv(L_KK), from the last column; padding columns stay zero
+        if (tid < nR) {
+            double y[NB];
 #pragma unroll
-            for (int k = 0; k < NB; ++k) l[k] = k < nb ? L[a + (int64_t)(k0 + k) * f.ldl] : 0.0;
-            double* y = Y + (int64_t)(a - k1) * NB;
-#pragma unroll 1
+            for (int j = NB - 1; j >= 0; --j) {
+                double v = l[j];
+#pragma unroll
+                for (int k = j + 1; k < NB; ++k) v -= y[k] * Lk[k * kSelLD + j];
+                y[j] = j < nb ? v / Lk[j * kSelLD + j] : 0.0;
+            }
+#pragma unroll
+            for (int j = 0; j < NB; ++j) Y[tid * kSelYS + j] = y[j];
+        }
+        if (k0 >= NB) load(k0 - NB);
+        // W = inv(L_KK), a column per lane of the last warp
+        if (warp == nw - 1 && lane < nb) {
+            double w[NB];
+#pragma unroll
+            for (int i = 0; i < NB; ++i) {
+                double v = i == lane ? 1.0 : 0.0;
+#pragma unroll
+                for (int k = 0; k < i; ++k) v -= Lk[i * kSelLD + k] * w[k];
+                w[i] = i < nb && i >= lane ? v / Lk[i * kSelLD + i] : 0.0;
+                Wk[i * kSelLD + lane] = w[i];
+            }
+        }
+        sync();
+        // Z_RK = -Z_RR Y
+        const int RB = (nR + 31) / 32, NS = RB > 0 ? max(1, min(max_slices, nw / RB)) : 1;
+        const int per = (nR + NS - 1) / NS;
+        auto put = [&](int a, const double (&v)[NB]) {
+#pragma unroll
             for (int j = 0; j < NB; ++j) {
-                double v = 0.0;
-#pragma unroll
-                for (int k = 0; k < NB; ++k) v += l[k] * Wk[k][j];
-                y[j] = v;
+                if (j >= nb) continue;
+                Z[(k1 + a) + (k0 + j) * LD] = Z[(k0 + j) + (k1 + a) * LD] = -v[j];
+                Zs[f.loff + k1 + a + (int64_t)(k0 + j) * f.ldl] = -v[j];
             }
-        }
-        __syncthreads();
-        // Z_RK = -Z_RR Y, a row per thread
-        for (int a = k1 + tid; a < m; a += nt) {
+        };
+        for (int t = warp; t < RB * NS; t += nw) {
+            const int rb = t % RB, sl = t / RB, a = 32 * rb + lane;
             double acc[NB];
 #pragma unroll
             for (int j = 0; j < NB; ++j) acc[j] = 0.0;
-            for (int b = k1; b < m; ++b) {
-                const double z = b <= a ? zelem(Zs, Zu, f, zf, a, b) : zelem(Zs, Zu, f, zf, b, a);
-                const double* y = Y + (int64_t)(b - k1) * NB;
+            const int b1 = min(nR, (sl + 1) * per);
+#pragma unroll 2
+            for (int b = sl * per; b < b1; ++b) {
+                const double z = a < nR ? Z[(k1 + a) + (k1 + b) * LD] : 0.0;
+                const double2* y = reinterpret_cast<const double2*>(Y + b * kSelYS);
 #pragma unroll
-                for (int j = 0; j < NB; ++j) acc[j] += z * y[j];
+                for (int j = 0; j < NB / 2; ++j) {
+                    const double2 yy = y[j];
+                    acc[2 * j] += z * yy.x;
+                    acc[2 * j + 1] += z * yy.y;
+                }
             }
-            for (int j = 0; j < nb; ++j) Zs[f.loff + a + (int64_t)(k0 + j) * f.ldl] = -acc[j];
+            if (NS == 1) {
+                if (a < nR) put(a, acc);
+            } else {
+                double2* o = reinterpret_cast<double2*>(P + (int64_t)(t * 32 + lane) * kSelYS);
+#pragma unroll
+                for (int j = 0; j < NB / 2; ++j) o[j] = make_double2(acc[2 * j], acc[2 * j + 1]);
+            }
         }
-        __syncthreads();
-        // Z_KK = W'W - Y' Z_RK, lower part, an entry per thread
-        for (int e = tid; e < NB * NB; e += nt) {
-            const int i = e % NB, j = e / NB;
-            if (i >= nb || j >= nb || i < j) continue;
+        sync();
+        if (NS > 1) {  // the slices in order
+            if (tid < nR) {
+                double acc[NB];
+#pragma unroll
+                for (int j = 0; j < NB; ++j) acc[j] = 0.0;
+                for (int sl = 0; sl < NS; ++sl)
+#pragma unroll
+                    for (int j = 0; j < NB; ++j) acc[j] += P[(sl * RB * 32 + tid) * kSelYS + j];
+                put(tid, acc);
+            }
+            sync();
+        }
+        // Z_KK = W'W - Y' Z_RK, lower part, a warp per entry
+        for (int e = warp; e < nb * nb; e += nw) {
+            const int i = e % nb, j = e / nb;
+            if (i < j) continue;
             double v = 0.0;
-            for (int k = i; k < nb; ++k) v += Wk[k][i] * Wk[k][j];
-            for (int a = k1; a < m; ++a)
-                v -= Y[(int64_t)(a - k1) * NB + i] * Zs[f.loff + a + (int64_t)(k0 + j) * f.ldl];
-            Zs[f.loff + (k0 + i) + (int64_t)(k0 + j) * f.ldl] = v;
+            for (int a = lane; a < nR; a += 32) v -= Y[a * kSelYS + i] * Z[(k1 + a) + (k0 + j) * LD];
+            if (lane >= i && lane < nb) v += Wk[lane * kSelLD + i] * Wk[lane * kSelLD + j];
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(ALL, v, o);
+            if (lane == 0) {
+                Z[(k0 + i) + (k0 + j) * LD] = Z[(k0 + j) + (k0 + i) * LD] = v;
+                Zs[f.loff + k0 + i + (int64_t)(k0 + j) * f.ldl] = v;
+            }
         }
-        __syncthreads();
+        sync();
+    }
+}
+
+// shared memory (doubles) of a front of up to MB rows with nw warps
+__host__ __device__ constexpr int sel_slices(int MB, int nw) {
+    return nw == 1 || MB > 128 ? 1 : nw;
+}
+__host__ __device__ constexpr size_t sel_small_doubles(int MB, int nw) {
+    return (((size_t)MB * (MB + 1) + 1) & ~(size_t)1) + (size_t)MB * kSelYS +
+           (sel_slices(MB, nw) > 1 ? (size_t)nw * 32 * kSelYS : 0) + kSelSm;
+}
+
+// Fronts of up to MB rows, more than 32: a CTA of eight warps each (every
+// row a thread); up to 32: a warp each.
+constexpr int kSelTinyRows = 32;
+template <bool TINY>
+__global__ void __launch_bounds__(256)
+    k_selinv_front(const FrontDesc* __restrict__ fronts, const int* __restrict__ list, int nlist,
+                   int MB, const int* __restrict__ relmap, const double* __restrict__ Ls,
+                   double* __restrict__ Zs, double* __restrict__ Zu,
+                   const int64_t* __restrict__ zuoff) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const int warp = threadIdx.x >> 5, nw = TINY ? 1 : blockDim.x >> 5;
+    const int MR = TINY ? kSelTinyRows : MB, LD = MR + 1;
+    double* Z = reinterpret_cast<double*>(smem_raw) +
+                (TINY ? warp * sel_small_doubles(kSelTinyRows, 1) : 0);
+    double* Y = Z + ((MR * LD + 1) & ~1);
+    double* P = Y + MR * kSelYS;
+    const int slices = sel_slices(MR, nw);
+    double* SM = P + (slices > 1 ? nw * 32 * kSelYS : 0);
+    if (TINY) {
+        const int k = blockIdx.x * (blockDim.x >> 5) + warp;
+        if (k < nlist)
+            sel_small_front(list[k], Z, LD, Y, P, slices, SM, 0, 1, [] { __syncwarp(); }, fronts,
+                            relmap, Ls, Zs, Zu, zuoff);
+    } else {
+        sel_small_front(list[blockIdx.x], Z, LD, Y, P, slices, SM, warp, nw,
+                        [] { __syncthreads(); }, fronts, relmap, Ls, Zs, Zu, zuoff);
     }
 }
 
@@ -463,8 +582,8 @@ int64_t selinv_partials(const DevPlan& D) {
     return (p + q) * kSelT * kSelT;
 }
 
-// Level by level from the root: the small fronts one CTA each
-// (k_selinv_front) on a stream of their own, the large fronts by the tiled
+// Level by level from the root: the small fronts (k_selinv_front) in pieces on
+// streams of their own, the large fronts by the tiled
 // phases above beside them, block step by block step (fronts with fewer
 // pivot blocks join the later steps).
 void launch_selinv(const DevPlan& D, const double* Ls, const double* Dinv, double* Zs,
@@ -485,16 +604,32 @@ void launch_selinv(const DevPlan& D, const double* Ls, const double* Dinv, doubl
     for (int l = D.nlevels - 1; l >= 0; --l) {
         const int sb = D.h_small_ptr[l * kSmallBuckets], se = D.h_small_ptr[(l + 1) * kSmallBuckets];
         const int q0 = S.h_step_beg[l], q1 = S.h_step_beg[l + 1];
-        const bool fork = se > sb && q1 > q0 && D.piece_st[0];
-        const cudaStream_t ss = fork ? D.piece_st[0] : st;
-        if (fork) {
-            cudaEventRecord(D.fork_ev, st);
-            cudaStreamWaitEvent(ss, D.fork_ev, 0);
+        // the pieces of the small fronts: at most 32 rows, then each size bucket
+        int pb[DevPlan::kSmallPieces + 1], npieces = 0;
+        pb[0] = sb;
+        for (int i = 0; i < DevPlan::kSmallPieces; ++i) {
+            pb[i + 1] = D.h_small_ptr[l * kSmallBuckets + Plan::kTinyBuckets + i];
+            npieces += pb[i + 1] > pb[i];
         }
-        if (se > sb)
-            k_selinv_front<<<se - sb, 256, 0, ss>>>(D.fronts, D.small_list + sb, D.relmap, Ls, Zs,
-                                                    Zu, D.zuoff, Yscr, D.yoff);
-        if (fork) cudaEventRecord(D.piece_join[0], ss);
+        const bool fork = D.piece_st[0] && npieces > 0 && npieces + (q1 > q0) > 1;
+        if (fork) cudaEventRecord(D.fork_ev, st);
+        for (int i = 0; i < DevPlan::kSmallPieces; ++i) {
+            const int n = pb[i + 1] - pb[i];
+            if (n == 0) continue;
+            const cudaStream_t ss = fork ? D.piece_st[i] : st;
+            if (fork) cudaStreamWaitEvent(ss, D.fork_ev, 0);
+            if (i == 0) {
+                k_selinv_front<true><<<(n + 7) / 8, 256,
+                                       8 * sel_small_doubles(kSelTinyRows, 1) * sizeof(double),
+                                       ss>>>(D.fronts, D.small_list + pb[i], n, kSelTinyRows,
+                                             D.relmap, Ls, Zs, Zu, D.zuoff);
+            } else {
+                const int MB = Plan::small_limit[Plan::kTinyBuckets + i - 1];
+                k_selinv_front<false><<<n, 256, sel_small_doubles(MB, 8) * sizeof(double), ss>>>(
+                    D.fronts, D.small_list + pb[i], n, MB, D.relmap, Ls, Zs, Zu, D.zuoff);
+            }
+            if (fork) cudaEventRecord(D.piece_join[i], ss);
+        }
         if (q1 > q0) {
             const SelList y = list(S.h_steps[q0]);
             if (y.nctas > 0)
@@ -517,7 +652,8 @@ void launch_selinv(const DevPlan& D, const double* Ls, const double* Dinv, doubl
             }
             k_sel_zkk<<<w.nitems * kSelSlabs, 256, 0, st>>>(data, w);
         }
-        if (fork) cudaStreamWaitEvent(st, D.piece_join[0], 0);
+        for (int i = 0; i < DevPlan::kSmallPieces; ++i)
+            if (fork && pb[i + 1] > pb[i]) cudaStreamWaitEvent(st, D.piece_join[i], 0);
     }
 }
 
@@ -537,12 +673,15 @@ template void launch_logdet<double>(const DevPlan&, const double*, double*, doub
 template void launch_logdet<float>(const DevPlan&, const float*, double*, double*, cudaStream_t);
 
 int logdet_partials() { return kLogdetBlocks; }
-int selinv_block() { return kSelBlock; }
 
 void init_selinv() {
     const int sm = (int)t64::SMEM_BYTES;
     cudaFuncSetAttribute(k_sel_zrk<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
     cudaFuncSetAttribute(k_sel_zrk<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
+    cudaFuncSetAttribute(k_selinv_front<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         227 * 1024);
+    cudaFuncSetAttribute(k_selinv_front<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         227 * 1024);
     cudaFuncSetAttribute(k_sel_fin, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
 }
 int selinv_tile() { return kSelT; }

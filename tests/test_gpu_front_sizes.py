@@ -190,3 +190,15 @@ def test_get_L_in_rounds(prec, eps):
     r = L @ (L.T @ v) - A[p][:, p] @ v
     bound = 1e4 * eps * (abs(L) @ (abs(L).T @ abs(v)))
     assert (np.abs(r) <= bound).all()
+
+
+@pytest.mark.parametrize("cs,u", SMALL)
+def test_selected_inverse_of_small_fronts(cs, u):
+    """As test_selected_inverse above."""
+    n, A, Ap, Ai, Ax = _leaves(cs, u)
+    S = M.Solver(n, Ap, Ai, ordering=M.ORDER_NATURAL)
+    S.factor(torch.from_numpy(Ax).cuda(), M.FP64)
+    S.selinv()
+    cols = np.repeat(np.arange(n), np.diff(Ap))
+    Z = np.linalg.inv(A)[Ai, cols] * np.where(Ai == cols, 1.0, 2.0)
+    assert np.linalg.norm(S.grad_lower() - Z) <= 1e-12 * np.linalg.norm(Z)
