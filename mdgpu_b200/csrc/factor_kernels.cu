@@ -413,19 +413,24 @@ __device__ void tiny_front_group(int s, const FrontDesc* __restrict__ fronts,
 #pragma unroll
         for (int j = k + 1; j < W; ++j) a[j] -= l * __shfl_sync(ALL, l, j, W);
     }
+    // (one warp alone issues an instruction every five cycles or so: pointers
+    // walked along the columns, and no branch but the loops')
+    const int row = gl < m ? gl : -1;
+    T* o = Ls + f.loff + gl;
+#pragma unroll
+    for (int j = 0; j < W; ++j) {
+        if (j >= maxc) break;
+        if ((j < c) & (row >= 0)) *o = gl >= j ? a[j] : T(0);
+        o += f.ldl;
+    }
     const int maxm = __reduce_max_sync(ALL, m);
-    T* pl = Ls + f.loff + gl;
-    T* pu = Us + f.uoff + (gl - c);
+    const int first = f.uoff >= 0 ? c : W;
+    o = Us + f.uoff + (gl - c) - (int64_t)c * f.ldu;
 #pragma unroll
     for (int j = 0; j < W; ++j) {
         if (j >= maxm) break;
-        const bool pivot = j < c;
-        if (j < m && gl < m && (pivot || (gl >= j && f.uoff >= 0)))
-            *(pivot ? pl : pu) = gl >= j ? a[j] : T(0);
-        if (pivot)
-            pl += f.ldl;
-        else
-            pu += f.ldu;
+        if ((j >= first) & (j <= row)) *o = a[j];
+        o += f.ldu;
     }
     __syncwarp();  // the slice is reused by the group's next front
 }
@@ -844,9 +849,17 @@ void launch_small_fronts(const DevPlan& D, int level, T* Ls, T* Us, const double
             const int n16 = cnt[1], n8 = cnt[2];
             const int ntask = n32 + (n16 + 1) / 2 + (n8 + 3) / 4;
             const int blocks = std::min((ntask + 3) / 4, D.tiny_blocks_cap);
-            k_tiny_fronts<T><<<blocks, 128, smem, st>>>(
-                D.fronts, D.solve.warp_list + beg + (cnt[0] - n32), n32, n16, n8, D.child,
-                D.relmap, D.a_src, D.a_pos, Ax, Ls, Us, status);
+            // a few fronts of 17..32 rows alone: four warps each (a warp each
+            // leaves the GPU idle; 24 x 23 grid: 8.5 -> 5.9 us a level, a root of 29
+            // columns 21 -> 13.5)
+            if (n16 + n8 == 0 && n32 <= 2 * (D.num_sms > 0 ? D.num_sms : 148))
+                k_small_front<T><<<n32, 128, smem / 4, st>>>(
+                    D.fronts, D.solve.warp_list + beg + (cnt[0] - n32), D.child, D.relmap, D.a_src,
+                    D.a_pos, Ax, Ls, Us, small_ld<T>(kTinyFrontRows), status);
+            else
+                k_tiny_fronts<T><<<blocks, 128, smem, st>>>(
+                    D.fronts, D.solve.warp_list + beg + (cnt[0] - n32), n32, n16, n8, D.child,
+                    D.relmap, D.a_src, D.a_pos, Ax, Ls, Us, status);
         }
     }
     for (int b = Plan::kTinyBuckets; b < kSmallBuckets; ++b) {
