@@ -548,16 +548,22 @@ __global__ void __launch_bounds__(256)
     }
 }
 
-// Warp-per-column variant: no block barriers, only warp syncs.  Each warp
-// builds its column in windows of W rows (W a multiple of 16) in its own
-// shared slice, so the slice does not grow with the front.  A child's columns
-// landing in the CTA's block of CB columns are at most CB (the relative map
-// is injective): the child column that lands in parent column jj is found by
-// one ballot over the child's range.  The child rows landing in a window are
-// one contiguous range (increasing relative map), read from the per-16-row
-// block table asm_range.  Every front entry gets its A value (or zero), then
-// the children's contributions in child order: the sums of a child-by-child
-// extend-add.
+// Warp-per-column variant: no block barriers but the one behind the table of
+// the block's children.  Each warp builds its column in windows of W rows (W a
+// multiple of 16) in its own shared slice, so the slice does not grow with the
+// front.  A child's columns landing in the CTA's block of CB columns are at most
+// CB (the relative map is injective); which of them lands in which column, and
+// where the child's values are, sits in the table for fronts of up to 32
+// children (others look it up per column, by one ballot over the child's
+// range).  The child rows landing in a window are one contiguous range
+// (increasing relative map), read from the per-16-row block table asm_range where
+// the window is not the whole column.  Every front entry gets its A value (or
+// zero), then the children's contributions in child order: the sums of a
+// child-by-child extend-add.  The next 256 values of the children are under way
+// while the last are added.  Bound by instruction issue (two slots of three taken
+// at 0.95 TB/s on fronts of a few hundred rows), so neither two columns per
+// warp nor fewer values per trip gained: 48^3 FP64 2.10 -> 1.93 ms, 64^3 FP32
+// 3.72 -> 3.60 against the lookup per column with no load ahead.
 template <typename T>
 __global__ void __launch_bounds__(256)
     k_big_assemble_warp(const FrontDesc* __restrict__ fronts, const int* __restrict__ items,
@@ -569,6 +575,13 @@ __global__ void __launch_bounds__(256)
                         const double* __restrict__ Ax, T* __restrict__ Ls, T* __restrict__ Us,
                         int W) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
+    constexpr unsigned ALL = 0xffffffffu;
+    constexpr int KIDS = 32, NL = 8;
+    // the block's children: update matrix, row map, and per column of the
+    // block the child's column that lands there (-1: none)
+    __shared__ int64_t s_u[KIDS];
+    __shared__ int s_rm[KIDS], s_ldu[KIDS], s_uc[KIDS];
+    __shared__ int s_jc[KIDS][kAssembleCols];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5;
     T* colbuf = reinterpret_cast<T*>(smem_raw) + (size_t)warp * W;
     const int it = find_item(before, nitems, blockIdx.x);
@@ -580,11 +593,77 @@ __global__ void __launch_bounds__(256)
     const int* rtab = asm_range + asm_off[s];  // [16-row block][child] -> [lo, hi)
     const int* ranges = rtab + blk * nch * 2;
     const int* cp = j0 < f.c ? a_colptr + a_colptr_off[s] : nullptr;
+    const bool table = nch <= KIDS;
+    if (table) {
+        for (int h = warp; h < nch; h += nw) {
+            const FrontDesc& g = fronts[child[f.child_beg + h]];
+            const int jlo = ranges[2 * h], jhi = ranges[2 * h + 1];
+            if (lane < kAssembleCols) s_jc[h][lane] = -1;
+            if (lane == 0) {
+                s_u[h] = g.uoff;
+                s_ldu[h] = g.ldu;
+                s_uc[h] = g.m - g.c;
+                s_rm[h] = g.rows_off + g.c;
+            }
+            __syncwarp();
+            if (jlo + lane < jhi)
+                s_jc[h][__ldg(relmap + g.rows_off + g.c + jlo + lane) - j0] = jlo + lane;
+        }
+        __syncthreads();
+    }
     for (int jj = j0 + warp; jj < j1; jj += nw) {
         const bool inL = jj < f.c;
         const int rlo = inL ? 0 : jj;
         for (int R0 = (rlo / W) * W; R0 < f.m; R0 += W) {
             const int R1 = min(R0 + W, f.m), w0 = max(R0, rlo);
+            const int b0 = R0 / 16, b1 = (R1 - 1) / 16;
+            // the trip at hand: NL x 32 of child h's rows >= its column, from
+            // ic0 on; h == nch at the end.  One trip's loads are under way while
+            // the one before is added.
+            int h = -1, ic0 = 0, ihi = 0;
+            const int* rm = nullptr;
+            const T* ucol = nullptr;
+            auto settle = [&]() {
+                while (ic0 >= ihi) {
+                    if (++h >= nch) return;
+                    int jc = -1, uc = 0;
+                    if (table) {
+                        jc = s_jc[h][jj - j0];
+                        if (jc < 0) continue;
+                        uc = s_uc[h];
+                        rm = relmap + s_rm[h];
+                        ucol = Us + s_u[h] + (int64_t)jc * s_ldu[h];
+                    } else {
+                        const int jlo = ranges[2 * h], jhi = ranges[2 * h + 1];
+                        if (jlo == jhi) continue;
+                        const FrontDesc& g = fronts[child[f.child_beg + h]];
+                        rm = relmap + g.rows_off + g.c;
+                        const int cand = jlo + lane;
+                        const unsigned hit =
+                            __ballot_sync(ALL, cand < jhi && __ldg(rm + cand) == jj);
+                        if (!hit) continue;
+                        jc = jlo + __ffs(hit) - 1;
+                        uc = g.m - g.c;
+                        ucol = Us + g.uoff + (int64_t)jc * g.ldu;
+                    }
+                    // child rows >= jc landing in rows [R0, R1) of the parent
+                    ic0 = R0 <= jj ? jc : max(jc, rtab[(b0 * nch + h) * 2]);
+                    ihi = R1 == f.m ? uc : rtab[(b1 * nch + h) * 2 + 1];
+                }
+            };
+            int pr[NL];
+            T v[NL];
+            auto fetch = [&]() {
+                if (h >= nch) return;
+#pragma unroll
+                for (int u = 0; u < NL; ++u) {
+                    const int ic = ic0 + lane + u * 32;
+                    pr[u] = ic < ihi ? __ldg(rm + ic) : -1;
+                    v[u] = ic < ihi ? __ldg(ucol + ic) : T(0);
+                }
+            };
+            settle();
+            fetch();
             for (int r = w0 + lane; r < R1; r += 32) colbuf[r - R0] = T(0);
             __syncwarp();
             if (inL) {
@@ -595,34 +674,21 @@ __global__ void __launch_bounds__(256)
                 }
                 __syncwarp();
             }
-            const int b0 = R0 / 16, b1 = (R1 - 1) / 16;
-            for (int h = 0; h < nch; ++h) {
-                const int jlo = ranges[2 * h], jhi = ranges[2 * h + 1];
-                if (jlo == jhi) continue;
-                const FrontDesc g = fronts[child[f.child_beg + h]];
-                const int* rm = relmap + g.rows_off + g.c;
-                const int cand = jlo + lane;
-                const unsigned hit =
-                    __ballot_sync(0xffffffffu, cand < jhi && __ldg(rm + cand) == jj);
-                if (!hit) continue;
-                const int jc = jlo + __ffs(hit) - 1;
-                // child rows >= jc landing in rows [R0, R1) of the parent
-                const int ilo = max(jc, rtab[(b0 * nch + h) * 2]);
-                const int ihi = rtab[(b1 * nch + h) * 2 + 1];
-                const T* ucol = Us + g.uoff + (int64_t)jc * g.ldu;
-                for (int ic0 = ilo + lane; ic0 < ihi; ic0 += 8 * 32) {
-                    int pr[8];
-                    T v[8];
+            while (h < nch) {  // children in order
+                int q[NL];
+                T x[NL];
 #pragma unroll
-                    for (int u = 0; u < 8; ++u) {
-                        const int ic = ic0 + u * 32;
-                        pr[u] = ic < ihi ? __ldg(rm + ic) : -1;
-                        v[u] = ic < ihi ? __ldg(ucol + ic) : T(0);
-                    }
+                for (int u = 0; u < NL; ++u) q[u] = pr[u] - R0, x[u] = v[u];
+                ic0 += NL * 32;
+                settle();
+                fetch();
+                // distinct rows: all reads before the writes
 #pragma unroll
-                    for (int u = 0; u < 8; ++u)
-                        if (pr[u] >= 0) colbuf[pr[u] - R0] += v[u];
-                }
+                for (int u = 0; u < NL; ++u)
+                    if (q[u] + R0 >= 0) x[u] += colbuf[q[u]];
+#pragma unroll
+                for (int u = 0; u < NL; ++u)
+                    if (q[u] + R0 >= 0) colbuf[q[u]] = x[u];
                 __syncwarp();
             }
             if (inL) {
