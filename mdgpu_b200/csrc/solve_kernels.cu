@@ -831,8 +831,10 @@ __device__ void fwd_front(int s, const FrontDesc& F, const SolveAbort& ab,
 #pragma unroll
                     for (int q = 0; q < NQ; ++q) {
                         const double y = __shfl_sync(mask, v[ks][q], j, W) * rj;
+                        // only the rows below: 0 y is a NaN for an infinite y
+                        if (lane > j) v[ks][q] -= (double)l[ks][cc] * y;
 #pragma unroll
-                        for (int k = ks; k < R; ++k) v[k][q] -= (double)l[k][cc] * y;
+                        for (int k = ks + 1; k < R; ++k) v[k][q] -= (double)l[k][cc] * y;
                         if (lane == j) v[ks][q] = y;
                     }
                 }
