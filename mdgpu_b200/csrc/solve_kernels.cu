@@ -855,9 +855,9 @@ __device__ void fwd_front(int s, const FrontDesc& F, const SolveAbort& ab,
     }
 }
 
-// Backward: t = L21' x over the update rows (one reduction per pivot column,
+// Backward: t = y - L21' x over the update rows (one reduction per pivot column,
 // independent of each other), then the pivot columns from the last, lane i
-// holding column i: x_j = (y_j - t_j) / L(j, j), t_i += L(j, i) x_j, the rows j
+// holding column i: x_j = t_j / L(j, j), t_i -= L(j, i) x_j, the rows j
 // of L read four at a time down each lane's own column.
 template <typename TL, int W, int R, int NQ>
 __device__ void bwd_front(const FrontDesc& F, const SolveAbort& ab,
@@ -911,10 +911,10 @@ __device__ void bwd_front(const FrontDesc& F, const SolveAbort& ab,
         for (int k = 0; k < R; ++k) {
             const int r = lane + W * k;
 #pragma unroll
-            for (int q = 0; q < NQ; ++q) {  // t starts as -y
+            for (int q = 0; q < NQ; ++q) {
                 t[k][q] = 0.0;
                 if (r < c && q < nq)
-                    t[k][q] = -xp[(int64_t)(F.first_col + r) * nrhs + q0 + q];
+                    t[k][q] = xp[(int64_t)(F.first_col + r) * nrhs + q0 + q];
             }
         }
 #pragma unroll
@@ -947,7 +947,7 @@ __device__ void bwd_front(const FrontDesc& F, const SolveAbort& ab,
                     for (int cc = 0; cc < CH; ++cc)
 #pragma unroll
                         for (int q = 0; q < NQ; ++q)
-                            if (lane == j0 + cc - W * ks) t[ks][q] += p[cc][q];
+                            if (lane == j0 + cc - W * ks) t[ks][q] -= p[cc][q];
                 }
             }
         }
@@ -962,10 +962,10 @@ __device__ void bwd_front(const FrontDesc& F, const SolveAbort& ab,
                     const double rj = rds[j];
 #pragma unroll
                     for (int q = 0; q < NQ; ++q) {
-                        const double xj = -__shfl_sync(mask, t[ks][q], j - W * ks, W) * rj;
+                        const double xj = __shfl_sync(mask, t[ks][q], j - W * ks, W) * rj;
 #pragma unroll
                         for (int k = 0; k <= ks; ++k)
-                            if (lane + W * k < j) t[k][q] += (double)lt[k][e] * xj;
+                            if (lane + W * k < j) t[k][q] -= (double)lt[k][e] * xj;
                         if (lane == j - W * ks) t[ks][q] = xj;
                     }
                 }

@@ -57,3 +57,15 @@ def test_infinite_right_hand_side(cs, u, prec, nrhs):
         np.testing.assert_array_equal(x[~fin, 0], ref[~fin])
         assert np.abs(x[fin, 0] - ref[fin]).max(initial=0.0) <= 1e-12
         assert np.array_equal(x[:, 1:], clean[:, 1:])  # the other columns are untouched
+
+
+# A zero right-hand side: every product and sum is a zero, and a difference of
+# zeros of the same sign is +0, so the solution is +0 throughout.
+@pytest.mark.parametrize("cs,u", SMALL)
+@pytest.mark.parametrize("nrhs", [1, 3])
+def test_zero_right_hand_side(cs, u, nrhs):
+    n, A, Ap, Ai, Ax = _leaves(cs, u)
+    S = M.Solver(n, Ap, Ai, ordering=M.ORDER_NATURAL)
+    S.factor(torch.from_numpy(Ax).cuda(), M.FP64)
+    x = S.solve(np.zeros((n, nrhs), order="F"))
+    assert not x.any() and not np.signbit(x).any()
