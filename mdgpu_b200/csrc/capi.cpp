@@ -83,7 +83,9 @@ int device_available() {
 
 }  // namespace
 
-constexpr int64_t kPackDoubles = 8 << 20;  // mdgpu_get_L's packing buffer
+// mdgpu_get_L's packing buffer: at most 64 MB during a call (8 MB rounds: 48^3
+// FP64 123 ms, 64 MB: 116), at most 8 MB kept between calls
+constexpr int64_t kPackDoubles = 8 << 20, kPackKept = 1 << 20;
 
 struct mdgpu_handle_s {
     Symbolic sym;
@@ -134,7 +136,8 @@ struct mdgpu_handle_s {
            *d_Abar = nullptr, *d_adjpart = nullptr;
     double* d_Y = nullptr;         // its Y scratch
     double* d_selpart = nullptr;   // its partial sums
-    // mdgpu_get_L's packed columns (at most kPackDoubles, or the longest column)
+    // mdgpu_get_L's packed columns (at most kPackKept between calls, or the
+    // longest column), given back where another allocation needs the room
     double* d_pack = nullptr;
     int64_t pack_cap = 0;
     double* d_logdet = nullptr;    // logdet partial sums, then the result
@@ -152,6 +155,23 @@ struct mdgpu_handle_s {
     T* keep(T* p) {
         owned.push_back(p);
         return p;
+    }
+    // storage of a numeric call; the packing buffer (idle between calls) makes
+    // room for it if it has to
+    template <typename T>
+    T* store(size_t count) {
+        if (!d_pack) return dalloc<T>(count);
+        try {
+            return dalloc<T>(count);
+        } catch (const std::bad_alloc&) {
+            drop_pack();
+            return dalloc<T>(count);
+        }
+    }
+    void drop_pack() {
+        if (d_pack) cudaFree(d_pack);
+        d_pack = nullptr;
+        pack_cap = 0;
     }
     void drop_solve_graphs() {
         for (auto& kv : sgraph) cudaGraphExecDestroy(kv.second);
@@ -605,16 +625,16 @@ cudaStream_t pick_stream(mdgpu_handle_s* h, void* s) {
 void ensure_factor_storage(mdgpu_handle_s* h, int precision) {
     const Plan& P = h->plan;
     if (precision == MDGPU_FP64) {
-        if (!h->dL64) h->dL64 = dalloc<double>(P.lstore);
-        if (!h->dU64) h->dU64 = dalloc<double>(P.ustore);
-        if (!h->dD64) h->dD64 = dalloc<double>(P.dinv_total);
+        if (!h->dL64) h->dL64 = h->store<double>(P.lstore);
+        if (!h->dU64) h->dU64 = h->store<double>(P.ustore);
+        if (!h->dD64) h->dD64 = h->store<double>(P.dinv_total);
     } else {
         if (!h->dL32) {
-            h->dL32 = dalloc<float>(P.lstore);
+            h->dL32 = h->store<float>(P.lstore);
             // the split panel scratch and its TMA descriptors (3xTF32
             // tensor-core Schur updates)
             if (h->use_tensor_cores && !P.large_list.empty()) {
-                h->D.pscr = h->keep(dalloc<float>(std::max<int64_t>(h->D.pscr_total, 1)));
+                h->D.pscr = h->keep(h->store<float>(std::max<int64_t>(h->D.pscr_total, 1)));
                 std::vector<CUtensorMap> maps;
                 std::vector<int> idx;
                 if (build_panel_maps(P, h->D.pscr, h->pscr_off, maps, idx, false) == 0) {
@@ -623,8 +643,8 @@ void ensure_factor_storage(mdgpu_handle_s* h, int precision) {
                 }
             }
         }
-        if (!h->dU32) h->dU32 = dalloc<float>(P.ustore);
-        if (!h->dD32) h->dD32 = dalloc<float>(P.dinv_total);
+        if (!h->dU32) h->dU32 = h->store<float>(P.ustore);
+        if (!h->dD32) h->dD32 = h->store<float>(P.dinv_total);
         // the same scratch read as the BF16 copy of the panels (BF16 Schur
         // updates)
         if (precision == MDGPU_BF16 && !h->D.tmaps_bf16 && h->D.pscr) {
@@ -651,13 +671,13 @@ void ensure_solve_storage(mdgpu_handle_s* h, int nrhs) {
     }
     int64_t n = h->plan.n;
     int chunk = std::min(nrhs, 64);
-    h->d_xp = dalloc<double>(n * nrhs);
-    h->d_fv = dalloc<double>(h->D.fv_total * chunk);
-    h->d_B = dalloc<double>(n * nrhs);
-    h->d_X = dalloc<double>(n * nrhs);
-    h->d_R = dalloc<double>(n * nrhs);
-    h->d_D = dalloc<double>(n * nrhs);
-    h->d_norms = dalloc<unsigned long long>(1 + 3 * nrhs);
+    h->d_xp = h->store<double>(n * nrhs);
+    h->d_fv = h->store<double>(h->D.fv_total * chunk);
+    h->d_B = h->store<double>(n * nrhs);
+    h->d_X = h->store<double>(n * nrhs);
+    h->d_R = h->store<double>(n * nrhs);
+    h->d_D = h->store<double>(n * nrhs);
+    h->d_norms = h->store<unsigned long long>(1 + 3 * nrhs);
     h->nrhs_cap = nrhs;
 }
 
@@ -848,6 +868,30 @@ struct DeviceGmresOps {
     }
 };
 
+// mdgpu_get_L without the packing buffer: runs of panels downloaded, packed here
+template <typename T>
+void download_L(mdgpu_handle_s* h, const T* Ls, double* Lx) {
+    const Plan& P = h->plan;
+    std::vector<T> panels;
+    for (int s0 = 0, s1; s0 < P.nsuper; s0 = s1) {
+        const int64_t base = P.fronts[s0].loff;  // panels lie in front order
+        auto end = [&](int s) { return P.fronts[s].loff + (int64_t)P.fronts[s].ldl * P.fronts[s].c; };
+        for (s1 = s0 + 1; s1 < P.nsuper && end(s1) - base <= kPackDoubles;) ++s1;
+        panels.resize(end(s1 - 1) - base);
+        ck(cudaMemcpyAsync(panels.data(), Ls + base, panels.size() * sizeof(T),
+                           cudaMemcpyDeviceToHost, h->stream),
+           "download L");
+        ck(cudaStreamSynchronize(h->stream), "download L");
+        for (int s = s0; s < s1; ++s) {
+            const FrontDesc& f = P.fronts[s];
+            for (int j = 0; j < f.c; ++j) {
+                const T* col = panels.data() + (f.loff - base) + (int64_t)j * f.ldl;
+                std::copy(col + j, col + f.m, Lx + P.Lp[f.first_col + j]);
+            }
+        }
+    }
+}
+
 int do_gmres_ir(mdgpu_handle_s* h, const double* dB, int ldb, double* dX, int ldx, int nrhs,
                 const GmresIrParams& prm, double* berr, int* outer, int* inner, cudaStream_t st) {
     NvtxRange nvtx("mdgpu_gmres_ir");
@@ -861,7 +905,7 @@ int do_gmres_ir(mdgpu_handle_s* h, const double* dB, int ldb, double* dX, int ld
         if (h->d_gm) cudaFree(h->d_gm);
         h->d_gm = nullptr;
         h->gm_cap = 0;
-        h->d_gm = dalloc<double>(need);
+        h->d_gm = h->store<double>(need);
         h->gm_cap = need;
     }
     DeviceGmresOps ops;
@@ -1631,7 +1675,7 @@ int mdgpu_logdet(mdgpu_handle h, double* logdet, void* stream) {
     return guarded([&]() -> int {
         cudaStream_t st = pick_stream(h, stream);
         ck(cudaSetDevice(h->device), "cudaSetDevice");
-        if (!h->d_logdet) h->d_logdet = dalloc<double>(logdet_partials() + 1);
+        if (!h->d_logdet) h->d_logdet = h->store<double>(logdet_partials() + 1);
         double* out = h->d_logdet + logdet_partials();
         if (h->factored == MDGPU_FP64)
             launch_logdet<double>(h->D, h->dL64, h->d_logdet, out, st);
@@ -1651,10 +1695,10 @@ int mdgpu_selinv(mdgpu_handle h, void* stream) {
     return guarded([&]() -> int {
         cudaStream_t st = pick_stream(h, stream);
         ck(cudaSetDevice(h->device), "cudaSetDevice");
-        if (!h->dZ64) h->dZ64 = dalloc<double>(h->plan.lstore);
-        if (!h->dZu64) h->dZu64 = dalloc<double>(h->plan.zustore);
-        if (!h->d_Y) h->d_Y = dalloc<double>(std::max<int64_t>(h->D.yscr_total, 1));
-        if (!h->d_selpart) h->d_selpart = dalloc<double>(selinv_partials(h->D));
+        if (!h->dZ64) h->dZ64 = h->store<double>(h->plan.lstore);
+        if (!h->dZu64) h->dZu64 = h->store<double>(h->plan.zustore);
+        if (!h->d_Y) h->d_Y = h->store<double>(std::max<int64_t>(h->D.yscr_total, 1));
+        if (!h->d_selpart) h->d_selpart = h->store<double>(selinv_partials(h->D));
         NvtxRange nvtx("mdgpu_selinv");
         launch_selinv(h->D, h->dL64, h->dD64, h->dZ64, h->dZu64, h->d_Y, h->d_selpart, st);
         ck(cudaGetLastError(), "selected inverse launch");
@@ -1686,8 +1730,8 @@ int mdgpu_grad_lower(mdgpu_handle h, const double* x, double* G, void* stream) {
         cudaStream_t st = pick_stream(h, stream);
         ck(cudaSetDevice(h->device), "cudaSetDevice");
         const int64_t n = h->plan.n, nnz = h->plan.nnz_user;
-        if (!h->d_gx) h->d_gx = dalloc<double>(n);
-        if (!h->d_gG) h->d_gG = dalloc<double>(std::max<int64_t>(nnz, 1));
+        if (!h->d_gx) h->d_gx = h->store<double>(n);
+        if (!h->d_gG) h->d_gG = h->store<double>(std::max<int64_t>(nnz, 1));
         if (x) ck(cudaMemcpyAsync(h->d_gx, x, n * sizeof(double), cudaMemcpyHostToDevice, st), "x");
         int rc = mdgpu_grad_lower_device(h, x ? h->d_gx : nullptr, h->d_gG, stream);
         if (rc != MDGPU_OK) return rc;
@@ -1789,10 +1833,10 @@ int mdgpu_adjoint_device(mdgpu_handle h, const double* dLbar, double* dAbar, voi
         cudaStream_t st = pick_stream(h, stream);
         ck(cudaSetDevice(h->device), "cudaSetDevice");
         const Plan& P = h->plan;
-        if (!h->d_Fb) h->d_Fb = dalloc<double>(P.lstore);
-        if (!h->d_Fu) h->d_Fu = dalloc<double>(P.zustore);
-        if (!h->d_W) h->d_W = dalloc<double>(h->D.adj.wtotal);
-        if (!h->d_adjpart) h->d_adjpart = dalloc<double>(adjoint_parts(h->D));
+        if (!h->d_Fb) h->d_Fb = h->store<double>(P.lstore);
+        if (!h->d_Fu) h->d_Fu = h->store<double>(P.zustore);
+        if (!h->d_W) h->d_W = h->store<double>(h->D.adj.wtotal);
+        if (!h->d_adjpart) h->d_adjpart = h->store<double>(adjoint_parts(h->D));
         launch_adjoint(h->D, (int)P.a_src.size(), h->dL64, h->dD64, dLbar, h->d_Fb, h->d_Fu,
                        h->d_W, h->d_adjpart, dAbar, st);
         ck(cudaGetLastError(), "adjoint launch");
@@ -1808,8 +1852,8 @@ int mdgpu_adjoint(mdgpu_handle h, const double* Lbar, double* Abar, void* stream
         cudaStream_t st = pick_stream(h, stream);
         ck(cudaSetDevice(h->device), "cudaSetDevice");
         const int64_t lnz = h->plan.lnz, nnz = h->plan.nnz_user;
-        if (!h->d_Lbar) h->d_Lbar = dalloc<double>(std::max<int64_t>(lnz, 1));
-        if (!h->d_Abar) h->d_Abar = dalloc<double>(std::max<int64_t>(nnz, 1));
+        if (!h->d_Lbar) h->d_Lbar = h->store<double>(std::max<int64_t>(lnz, 1));
+        if (!h->d_Abar) h->d_Abar = h->store<double>(std::max<int64_t>(nnz, 1));
         ck(cudaMemcpyAsync(h->d_Lbar, Lbar, lnz * sizeof(double), cudaMemcpyHostToDevice, st),
            "Lbar");
         int rc = mdgpu_adjoint_device(h, h->d_Lbar, h->d_Abar, stream);
@@ -1841,16 +1885,20 @@ int mdgpu_get_L(mdgpu_handle h, long long* Lp, int* Li, double* Lx) {
         ck(cudaStreamSynchronize(h->stream), "sync");
         // the columns packed on the device, as many at a time as the packing
         // buffer holds (100 x 100 grid, factor, L and solve: 1.30 ms; 1.86 with
-        // the panels downloaded and packed by a host loop)
+        // the panels downloaded and packed by a host loop, which is left where
+        // the device has no room for the buffer)
         if (!h->d_pack) {
             int64_t longest = 1;
             for (int j = 0; j < P.n; ++j) longest = std::max(longest, P.Lp[j + 1] - P.Lp[j]);
-            int64_t want = std::max(longest, std::min<int64_t>(P.Lp[P.n], kPackDoubles));
-            while (cudaMalloc(&h->d_pack, want * sizeof(double)) != cudaSuccess) {
+            const int64_t want = std::max(longest, std::min<int64_t>(P.Lp[P.n], kPackDoubles));
+            if (cudaMalloc(&h->d_pack, want * sizeof(double)) != cudaSuccess) {
                 cudaGetLastError();
                 h->d_pack = nullptr;
-                if (want == longest) throw std::runtime_error("no memory to pack L's columns");
-                want = std::max(longest, want / 2);
+                if (h->factored == MDGPU_FP64)
+                    download_L(h, h->dL64, Lx);
+                else
+                    download_L(h, h->dL32, Lx);
+                return MDGPU_OK;
             }
             h->pack_cap = want;
         }
@@ -1867,6 +1915,7 @@ int mdgpu_get_L(mdgpu_handle h, long long* Lp, int* Li, double* Lx) {
                "download L");
         }
         ck(cudaStreamSynchronize(h->stream), "download L");
+        if (h->pack_cap > kPackKept) h->drop_pack();
         return MDGPU_OK;
     });
 }

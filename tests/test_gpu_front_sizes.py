@@ -8,6 +8,8 @@ Cholesky of order n and condition k returns L to n eps k; the matrices here
 are diagonally dominant with condition below 10 and n below 1000, so 1e-12
 leaves a factor of ten over 1000 * 2.2e-16 * 0.5.
 """
+import contextlib
+
 import numpy as np
 import pytest
 
@@ -202,3 +204,57 @@ def test_selected_inverse_of_small_fronts(cs, u):
     cols = np.repeat(np.arange(n), np.diff(Ap))
     Z = np.linalg.inv(A)[Ai, cols] * np.where(Ai == cols, 1.0, 2.0)
     assert np.linalg.norm(S.grad_lower() - Z) <= 1e-12 * np.linalg.norm(Z)
+
+
+def _volume():
+    from mdgpu_b200 import matgen as mg
+    return mg.laplacian_3d_varcoef(36)
+
+
+@contextlib.contextmanager
+def _device_filled(free_bytes):
+    """Device memory taken until about free_bytes are left."""
+    torch.cuda.empty_cache()
+    held = []
+    try:
+        for step in (256 << 20, 2 << 20):
+            room = torch.cuda.mem_get_info()[0] - free_bytes
+            if room >= step:
+                held.append(torch.empty(room // step * step, dtype=torch.uint8, device="cuda"))
+        yield
+    finally:
+        held.clear()
+        torch.cuda.empty_cache()
+
+
+def test_get_L_leaves_the_memory_to_later_calls():
+    """A first solve with several right-hand sides, on a device with room for
+    little more than its storage, works after get_L as it does without."""
+    n, Ap, Ai, Ax = _volume()
+    S = M.Solver(n, Ap, Ai)
+    dAx = torch.from_numpy(Ax).cuda()
+    S.factor(dAx, M.FP64)
+    B = np.random.default_rng(5).uniform(-1.0, 1.0, (n, 64))
+    S.solve(B[:, :2])  # the path's kernels loaded
+    need = 8 * 64 * (5 * n + S.info("solve_work_rows"))
+    with _device_filled(need + (24 << 20)):
+        Lx = S.get_L()[2]
+        X = S.solve(B)
+    assert Lx.size > 8 << 20
+    x = M.Solver(n, Ap, Ai)
+    x.factor(dAx, M.FP64)
+    assert np.array_equal(x.solve(B), X)
+
+
+@pytest.mark.parametrize("prec", [M.FP64, M.FP32])
+def test_get_L_without_room_on_the_device(prec):
+    """No room for the packing buffer: the same values, packed on the host."""
+    n, Ap, Ai, Ax = _volume()
+    dAx = torch.from_numpy(Ax).cuda()
+    S, T = M.Solver(n, Ap, Ai), M.Solver(n, Ap, Ai)
+    S.factor(dAx, prec)
+    T.factor(dAx, prec)
+    ref = S.get_L()[2]
+    with _device_filled(6 << 20):
+        Lx = T.get_L()[2]
+    assert np.array_equal(Lx, ref)
