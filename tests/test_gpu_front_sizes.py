@@ -258,3 +258,27 @@ def test_get_L_without_room_on_the_device(prec):
     with _device_filled(6 << 20):
         Lx = T.get_L()[2]
     assert np.array_equal(Lx, ref)
+
+
+@pytest.mark.parametrize("systems", [147, 148, 444])
+def test_selected_inverse_of_many_systems(systems):
+    """Systems of a leaf front of 40 pivot columns and 230 rows (three 64-row
+    tiles in its step) under a root of 230 columns (the other leaf's among them;
+    one, two and three tiles in its steps).  From three tiles for each of the GPU's
+    148 SMs on (148 systems' leaves, 444 systems' roots throughout) a step's sums
+    are not split and its tiles finish in the same launch.  Bound as in
+    test_selected_inverse above."""
+    n, A, Ap, Ai, _ = _two_leaves(40, 40, 190)
+    cols = np.repeat(np.arange(n), np.diff(Ap))
+    vals = np.random.default_rng(8).uniform(-1.0, 1.0, (systems, len(Ai)))
+    vals[:, Ai == cols] = 0.0
+    D = np.zeros((systems, n, n))
+    D[:, Ai, cols] = D[:, cols, Ai] = vals
+    D[:, range(n), range(n)] = vals[:, Ai == cols] = 1.5 * np.abs(D).sum(2)
+    S = M.Solver.batch([(n, Ap, Ai)] * systems, ordering=M.ORDER_NATURAL)
+    assert S.info("large_fronts") == 2 * systems
+    S.factor(torch.from_numpy(vals.ravel()).cuda(), M.FP64)
+    S.selinv()
+    Z = np.linalg.inv(D)[:, Ai, cols] * np.where(Ai == cols, 1.0, 2.0)
+    got = S.grad_lower().reshape(Z.shape)
+    assert (np.linalg.norm(got - Z, axis=1) <= 1e-12 * np.linalg.norm(Z, axis=1)).all()
