@@ -300,8 +300,8 @@ MDGPU_API int mdgpu_adjoint_device(mdgpu_handle h, const double *dLbar, double *
  * (mdgpu.cu:1346-1352, 1859-1875): Lp[n+1] (long long), Li[lnz] row indices
  * ascending with the diagonal first, Lx[lnz] values (FP64; an FP32 factor is
  * widened).  Any of the three may be NULL.  The values are packed on the
- * device in a buffer of up to 64 MB where there is room for it; at most 8 MB of
- * it stay with the handle after the call.
+ * device in a buffer of up to 64 MB where there is room for it, which stays with
+ * the handle until a later call needs its memory.
  */
 MDGPU_API int mdgpu_get_L(mdgpu_handle h, long long *Lp, int *Li, double *Lx);
 

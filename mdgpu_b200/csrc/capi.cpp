@@ -83,9 +83,11 @@ int device_available() {
 
 }  // namespace
 
-// mdgpu_get_L's packing buffer: at most 64 MB during a call (8 MB rounds: 48^3
-// FP64 123 ms, 64 MB: 116), at most 8 MB kept between calls
-constexpr int64_t kPackDoubles = 8 << 20, kPackKept = 1 << 20;
+// mdgpu_get_L's packing buffer, at most 64 MB (48^3 FP64 116 ms; rounds of 8 MB:
+// 123).  Allocated and freed in every call it cost 0.9 ms (24^3: 2.6 -> 3.5), so it
+// stays with the handle; factors of up to kPackMin elements are downloaded whole
+// (40 dense columns: 37 us packed, 31 downloaded)
+constexpr int64_t kPackDoubles = 8 << 20, kPackMin = 4096;
 
 struct mdgpu_handle_s {
     Symbolic sym;
@@ -136,8 +138,8 @@ struct mdgpu_handle_s {
            *d_Abar = nullptr, *d_adjpart = nullptr;
     double* d_Y = nullptr;         // its Y scratch
     double* d_selpart = nullptr;   // its partial sums
-    // mdgpu_get_L's packed columns (at most kPackKept between calls, or the
-    // longest column), given back where another allocation needs the room
+    // mdgpu_get_L's packed columns (at most kPackDoubles, or the longest
+    // column), given back where another allocation of the handle needs the room
     double* d_pack = nullptr;
     int64_t pack_cap = 0;
     double* d_logdet = nullptr;    // logdet partial sums, then the result
@@ -1887,20 +1889,23 @@ int mdgpu_get_L(mdgpu_handle h, long long* Lp, int* Li, double* Lx) {
         // buffer holds (100 x 100 grid, factor, L and solve: 1.30 ms; 1.86 with
         // the panels downloaded and packed by a host loop, which is left where
         // the device has no room for the buffer)
-        if (!h->d_pack) {
+        if (!h->d_pack && P.lstore > kPackMin) {
             int64_t longest = 1;
             for (int j = 0; j < P.n; ++j) longest = std::max(longest, P.Lp[j + 1] - P.Lp[j]);
             const int64_t want = std::max(longest, std::min<int64_t>(P.Lp[P.n], kPackDoubles));
-            if (cudaMalloc(&h->d_pack, want * sizeof(double)) != cudaSuccess) {
+            if (cudaMalloc(&h->d_pack, want * sizeof(double)) == cudaSuccess) {
+                h->pack_cap = want;
+            } else {
                 cudaGetLastError();
                 h->d_pack = nullptr;
-                if (h->factored == MDGPU_FP64)
-                    download_L(h, h->dL64, Lx);
-                else
-                    download_L(h, h->dL32, Lx);
-                return MDGPU_OK;
             }
-            h->pack_cap = want;
+        }
+        if (!h->d_pack) {
+            if (h->factored == MDGPU_FP64)
+                download_L(h, h->dL64, Lx);
+            else
+                download_L(h, h->dL32, Lx);
+            return MDGPU_OK;
         }
         for (int c0 = 0, c1; c0 < P.n; c0 = c1) {
             c1 = (int)(std::upper_bound(P.Lp.begin() + c0, P.Lp.end(), P.Lp[c0] + h->pack_cap) -
@@ -1915,7 +1920,6 @@ int mdgpu_get_L(mdgpu_handle h, long long* Lp, int* Li, double* Lx) {
                "download L");
         }
         ck(cudaStreamSynchronize(h->stream), "download L");
-        if (h->pack_cap > kPackKept) h->drop_pack();
         return MDGPU_OK;
     });
 }
