@@ -831,14 +831,36 @@ __device__ void fwd_front(int s, const FrontDesc& F, const SolveAbort& ab,
 #pragma unroll
                     for (int q = 0; q < NQ; ++q) {
                         const double y = __shfl_sync(mask, v[ks][q], j, W) * rj;
-                        // only the rows below: 0 y is a NaN for an infinite y
-                        if (lane > j) v[ks][q] -= (double)l[ks][cc] * y;
 #pragma unroll
-                        for (int k = ks + 1; k < R; ++k) v[k][q] -= (double)l[k][cc] * y;
+                        for (int k = ks; k < R; ++k) v[k][q] -= (double)l[k][cc] * y;
                         if (lane == j) v[ks][q] = y;
                     }
                 }
             }
+        }
+        // An infinite y left 0 y, a NaN, on the rows above its pivot: the front
+        // again from its assembled rows, column by column in shared memory, the
+        // rows below a pivot only.
+        double z = 0.0;
+#pragma unroll
+        for (int k = 0; k < R; ++k)
+#pragma unroll
+            for (int q = 0; q < NQ; ++q) z = fma(v[k][q], 0.0, z);
+        if (__any_sync(mask, z != 0.0)) {
+            for (int j = 0; j < c; ++j)
+                for (int q = 0; q < nq; ++q) {
+                    double* b = buf + q * stride;
+                    const double y = b[j] * rds[j];
+                    __syncwarp(mask);
+                    for (int r = j + lane; r < m; r += W)
+                        b[r] = r == j ? y : b[r] - (double)L[r + j * ldl] * y;
+                    __syncwarp(mask);
+                }
+#pragma unroll
+            for (int k = 0; k < R; ++k)
+#pragma unroll
+                for (int q = 0; q < NQ; ++q)
+                    if (q < nq && lane + W * k < m) v[k][q] = buf[q * stride + lane + W * k];
         }
 #pragma unroll
         for (int k = 0; k < R; ++k) {
