@@ -330,28 +330,42 @@ __device__ __forceinline__ double row_dot(const TL* B, const double* V, int g) {
 
 // x[q] += the front-vector rows that the assembly map adds into a row (fv row
 // e at fv + e * nrhs; NQ neighbouring right-hand sides), in child order, every
-// entry waited for, two in flight; a whole warp together, lanes with need
-// (ar: the row's entry range) and without.
+// entry waited for; a whole warp together, lanes with need (ar: the row's entry
+// range) and without.  Two entries in flight, as most rows have no more, eight (four for two right-hand sides)
+// while there are that many (a root over 2000 leaves, one right-hand side FP32:
+// two 0.62 ms, now 0.38).
+template <int E, int NQ>
+__device__ __forceinline__ void gather_some(int e, int e1, const int* __restrict__ amap_ent,
+                                            const double* fv, int nrhs, int nq, double (&x)[NQ],
+                                            const SolveAbort& ab) {
+    const double* p[E];
+    double v[E][NQ];
+#pragma unroll
+    for (int i = 0; i < E; ++i) {
+        p[i] = fv;
+        if (e + i < e1) p[i] += (int64_t)amap_ent[e + i] * nrhs;
+    }
+#pragma unroll
+    for (int i = 0; i < E; ++i) peek_values<NQ>(p[i], e + i < e1, nq, v[i]);
+    await_together<E, NQ>([&](int i) { return p[i]; }, nq, v, 0xffffffffu, ab);
+#pragma unroll
+    for (int i = 0; i < E; ++i)
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) x[q] += v[i][q];
+}
 template <int NQ>
 __device__ __forceinline__ void gather_entries(bool need, const int* ar,
                                                const int* __restrict__ amap_ent, const double* fv,
                                                int nrhs, int nq, double (&x)[NQ],
                                                const SolveAbort& ab) {
+    constexpr int WIDE = NQ == 1 ? 8 : 4;
     int e = 0, e1 = 0;
     if (need) e = ar[0], e1 = ar[1];
-    const int rounds = __reduce_max_sync(0xffffffffu, e1 - e);
-    for (int k = 0; k < rounds; k += 2, e += 2) {
-        const double* p[2] = {fv, fv};
-        double v[2][NQ];
-#pragma unroll
-        for (int i = 0; i < 2; ++i) {
-            if (e + i < e1) p[i] += (int64_t)amap_ent[e + i] * nrhs;
-            peek_values<NQ>(p[i], e + i < e1, nq, v[i]);
-        }
-        await_together<2, NQ>([&](int i) { return p[i]; }, nq, v, 0xffffffffu, ab);
-#pragma unroll
-        for (int q = 0; q < NQ; ++q) x[q] = (x[q] + v[0][q]) + v[1][q];
-    }
+    int left = __reduce_max_sync(0xffffffffu, e1 - e);
+    for (; left >= WIDE; left -= WIDE, e += WIDE)
+        gather_some<WIDE, NQ>(e, e1, amap_ent, fv, nrhs, nq, x, ab);
+    for (; left > 0; left -= 2, e += 2)
+        gather_some<2, NQ>(e, e1, amap_ent, fv, nrhs, nq, x, ab);
 }
 
 // Forward, task (s, i0 | cnt << 16): row tiles i0 .. i0 + cnt - 1 of front s.

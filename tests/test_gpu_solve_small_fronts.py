@@ -47,3 +47,20 @@ def test_columns_do_not_depend_on_the_columns_beside_them(fronts, prec):
     full = S.solve(B)
     for k in (2, 3, 8, 9, 10, 17, 57):
         assert np.array_equal(S.solve(B[:, :k]), full[:, :k]), k
+
+
+# leaves of one column under a root: the entries of a row of the root's front
+# vector in trips of eight, four and two, a child at a time or two
+@pytest.mark.parametrize("leaves", [1, 2, 3, 4, 5, 7, 8, 9, 11, 16, 35])
+@pytest.mark.parametrize("u", [6, 60, 200])
+@pytest.mark.parametrize("prec,tol", [(M.FP64, 1e-14), (M.FP32, 2e-5)])
+def test_many_children(leaves, u, prec, tol):
+    n, A, Ap, Ai, Ax = _leaves((1,) * leaves, u)
+    S = M.Solver(n, Ap, Ai, ordering=M.ORDER_NATURAL)
+    S.factor(torch.from_numpy(Ax).cuda(), prec)
+    B = np.random.default_rng(9).uniform(-1.0, 1.0, (n, 10))
+    scale = np.abs(A).sum(1).max()
+    for k in (1, 2, 10):
+        X = S.solve(B[:, :k]).reshape(n, k)
+        r = np.abs(B[:, :k] - A @ X).max(0)
+        assert (r <= tol * (scale * np.abs(X).max(0) + np.abs(B[:, :k]).max(0))).all(), k
