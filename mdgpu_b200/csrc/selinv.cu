@@ -529,17 +529,32 @@ __global__ void k_grad_lower(int nnz, const FrontDesc* __restrict__ fronts,
 }
 
 // logdet = 2 sum log L(j, j): per block a fixed-order sum over its
-// supernodes, a warp each (a root of thousands of columns read by one thread
-// took 1.1 ms), then one block sums the partials (deterministic)
+// supernodes, a lane each, the wider ones then a warp each (a root of thousands of
+// columns read by one thread took 1.1 ms, a warp for every column of a 300 x 300
+// grid's nodal tree 20 us more than a lane), then one block sums the partials
+// (deterministic)
 template <typename T>
 __global__ void k_logdet_partial(int nsuper, const FrontDesc* __restrict__ fronts,
                                  const T* __restrict__ Ls, double* __restrict__ partial) {
     __shared__ double red[256];
     double v = 0.0;
-    const int lane = threadIdx.x & 31, wpb = blockDim.x >> 5;
-    for (int s = blockIdx.x * wpb + (threadIdx.x >> 5); s < nsuper; s += gridDim.x * wpb) {
-        const FrontDesc f = fronts[s];
-        for (int j = lane; j < f.c; j += 32) v += log((double)Ls[f.loff + j + (int64_t)j * f.ldl]);
+    const int lane = threadIdx.x & 31, wpb = blockDim.x >> 5, nw = gridDim.x * wpb;
+    for (int s0 = blockIdx.x * wpb + (threadIdx.x >> 5); s0 < nsuper; s0 += 32 * nw) {
+        const int s = s0 + lane * nw;  // neighbours in the tree to different warps
+        int c = 0;
+        int64_t off = 0, step = 0;
+        if (s < nsuper) {
+            const FrontDesc& f = fronts[s];
+            c = f.c, off = f.loff, step = f.ldl + 1;
+        }
+        if (c <= 4)
+            for (int j = 0; j < c; ++j) v += log((double)Ls[off + j * step]);
+        for (unsigned wide = __ballot_sync(0xffffffffu, c > 4); wide; wide &= wide - 1) {
+            const int h = __ffs(wide) - 1, hc = __shfl_sync(0xffffffffu, c, h);
+            const int64_t hoff = __shfl_sync(0xffffffffu, off, h);
+            const int64_t hstep = __shfl_sync(0xffffffffu, step, h);
+            for (int j = lane; j < hc; j += 32) v += log((double)Ls[hoff + j * hstep]);
+        }
     }
     red[threadIdx.x] = v;
     __syncthreads();

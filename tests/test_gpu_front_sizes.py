@@ -282,3 +282,19 @@ def test_selected_inverse_of_many_systems(systems):
     Z = np.linalg.inv(D)[:, Ai, cols] * np.where(Ai == cols, 1.0, 2.0)
     got = S.grad_lower().reshape(Z.shape)
     assert (np.linalg.norm(got - Z, axis=1) <= 1e-12 * np.linalg.norm(Z, axis=1)).all()
+
+
+# more supernodes than warps (a lane each; those of more than four columns a warp
+# each).  A sum of n logarithms, each within an ulp or two: (n + 2) eps times the
+# sum of their sizes.
+@pytest.mark.parametrize("tree", [M.TREE_NODAL, M.TREE_SUPER])
+@pytest.mark.parametrize("prec", [M.FP64, M.FP32])
+def test_logdet_of_many_supernodes(tree, prec):
+    from mdgpu_b200 import matgen as mg
+    n, Ap, Ai, Ax = mg.laplacian_2d_5pt(80)
+    S = M.Solver(n, Ap, Ai, tree=tree)
+    assert S.info("nsuper") > 8 * 2 * 148
+    S.factor(np.asarray(Ax, np.float64), prec)
+    Lp, _, Lx = S.get_L()
+    logs = 2.0 * np.log(Lx[Lp[:-1]])
+    assert abs(S.logdet() - logs.sum()) <= (n + 2) * 2.0 ** -52 * np.abs(logs).sum()
