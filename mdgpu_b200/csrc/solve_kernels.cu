@@ -331,9 +331,10 @@ __device__ __forceinline__ double row_dot(const TL* B, const double* V, int g) {
 // x[q] += the front-vector rows that the assembly map adds into a row (fv row
 // e at fv + e * nrhs; NQ neighbouring right-hand sides), in child order, every
 // entry waited for; a whole warp together, lanes with need (ar: the row's entry
-// range) and without.  Two entries in flight, as most rows have no more, eight (four for two right-hand sides)
-// while there are that many (a root over 2000 leaves, one right-hand side FP32:
-// two 0.62 ms, now 0.38).
+// range) and without.  Most rows have at most two entries, in flight together; in
+// a warp with more, eight (four of two right-hand sides) per trip: a root of 300
+// rows over 2000 leaves, one right-hand side FP32, 0.39 ms, two per trip 0.62 (a
+// loop of two per trip behind one of eight cost chains of large fronts 2 %).
 template <int E, int NQ>
 __device__ __forceinline__ void gather_some(int e, int e1, const int* __restrict__ amap_ent,
                                             const double* fv, int nrhs, int nq, double (&x)[NQ],
@@ -361,11 +362,12 @@ __device__ __forceinline__ void gather_entries(bool need, const int* ar,
     constexpr int WIDE = NQ == 1 ? 8 : 4;
     int e = 0, e1 = 0;
     if (need) e = ar[0], e1 = ar[1];
-    int left = __reduce_max_sync(0xffffffffu, e1 - e);
-    for (; left >= WIDE; left -= WIDE, e += WIDE)
-        gather_some<WIDE, NQ>(e, e1, amap_ent, fv, nrhs, nq, x, ab);
-    for (; left > 0; left -= 2, e += 2)
+    const int most = __reduce_max_sync(0xffffffffu, e1 - e);
+    if (most <= 2)
         gather_some<2, NQ>(e, e1, amap_ent, fv, nrhs, nq, x, ab);
+    else
+        for (int k = 0; k < most; k += WIDE)
+            gather_some<WIDE, NQ>(e + k, e1, amap_ent, fv, nrhs, nq, x, ab);
 }
 
 // Forward, task (s, i0 | cnt << 16): row tiles i0 .. i0 + cnt - 1 of front s.
@@ -864,21 +866,23 @@ __device__ void fwd_front(int s, const FrontDesc& F, const SolveAbort& ab,
                     for (int q = 0; q < NQ; ++q) {
                         const double y = __shfl_sync(mask, v[ks][q], j, W) * rj;
 #pragma unroll
-                        for (int k = ks; k < R; ++k) v[k][q] -= (double)l[k][cc] * y;
+                        for (int k = ks; k < R; ++k)
+                            if (NQ > 1 || k > ks || lane > j) v[k][q] -= (double)l[k][cc] * y;
                         if (lane == j) v[ks][q] = y;
                     }
                 }
             }
         }
-        // An infinite y left 0 y, a NaN, on the rows above its pivot: the front
-        // again from its assembled rows, column by column in shared memory, the
-        // rows below a pivot only.
+        // Several right-hand sides (a test per column cost them 4 to 9 %, one
+        // right-hand side nothing): an infinite y left 0 y, a NaN, on the rows
+        // above its pivot.  The front again from its assembled rows, column by
+        // column in shared memory, the rows below a pivot only.
         double z = 0.0;
 #pragma unroll
         for (int k = 0; k < R; ++k)
 #pragma unroll
             for (int q = 0; q < NQ; ++q) z = fma(v[k][q], 0.0, z);
-        if (__any_sync(mask, z != 0.0)) {
+        if (NQ > 1 && __any_sync(mask, z != 0.0)) {
             for (int j = 0; j < c; ++j)
                 for (int q = 0; q < nq; ++q) {
                     double* b = buf + q * stride;
