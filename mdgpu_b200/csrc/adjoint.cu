@@ -69,6 +69,19 @@ __global__ void __launch_bounds__(256)
     }
 }
 
+// odd: 1 if one of Lbar's values is infinite or a NaN (cleared by the caller).  A
+// pass of its own at the rate of the memory; beside the scatter's stores the test
+// took 0.1 ms on a 32^3 grid.
+__global__ void __launch_bounds__(256)
+    k_adj_check(int64_t lnz, const double* __restrict__ Lbar, int* __restrict__ odd) {
+    const int64_t nt = (int64_t)gridDim.x * blockDim.x;
+    int top = 0;  // the largest exponent
+#pragma unroll 4
+    for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < lnz; e += nt)
+        top = max(top, __double2hiint(Lbar[e]) & 0x7fffffff);
+    if (top >= 0x7ff00000) *odd = 1;
+}
+
 // Ubar of front s = Fbar of its parent on s's update rows (lower part): CTA
 // per 16 columns, two per warp
 __global__ void __launch_bounds__(256)
@@ -100,14 +113,12 @@ __global__ void __launch_bounds__(256)
     }
 }
 
-// One front: Lbar (pivot columns of Fb, rows 0..m) -> Fbar in place, with
-// Ubar from Fu; W: c x c scratch.
-__global__ void __launch_bounds__(256)
-    k_adj_front(const FrontDesc* __restrict__ fronts, const int* __restrict__ list,
-                const double* __restrict__ Ls, double* __restrict__ Fb,
-                const double* __restrict__ Fu, const int64_t* __restrict__ zuoff,
-                double* __restrict__ Wscr, const int64_t* __restrict__ woff) {
-    const int s = list[blockIdx.x];
+// One front by one CTA, scalar sums over the entries that L has: Lbar (pivot
+// columns of Fb, rows 0..m) -> Fbar in place, with Ubar from Fu; W: c x c scratch.
+__device__ void adj_front(int s, const FrontDesc* __restrict__ fronts,
+                          const double* __restrict__ Ls, double* __restrict__ Fb,
+                          const double* __restrict__ Fu, const int64_t* __restrict__ zuoff,
+                          double* __restrict__ Wscr, const int64_t* __restrict__ woff) {
     const FrontDesc f = fronts[s];
     const int m = f.m, c = f.c, u = m - c;
     const int tid = threadIdx.x, nt = blockDim.x;
@@ -198,8 +209,19 @@ __global__ void __launch_bounds__(256)
     }
 }
 
+__global__ void __launch_bounds__(256)
+    k_adj_front(const FrontDesc* __restrict__ fronts, const int* __restrict__ list,
+                const double* __restrict__ Ls, double* __restrict__ Fb,
+                const double* __restrict__ Fu, const int64_t* __restrict__ zuoff,
+                double* __restrict__ Wscr, const int64_t* __restrict__ woff) {
+    adj_front(list[blockIdx.x], fronts, Ls, Fb, Fu, zuoff, Wscr, woff);
+}
+
 // ---------------------------------------------------------------------------
-// large fronts
+// large fronts.  The tiles multiply zeros (above the diagonal of an inverse, past
+// a front's edge) with the gradients, a NaN where one is infinite or a NaN itself:
+// for an Lbar with such entries (odd) every front takes the scalar sums above, in
+// the last of its launches.
 // ---------------------------------------------------------------------------
 
 struct AdjData {
@@ -213,6 +235,10 @@ struct AdjData {
     double* W;      // c x c scratch per front (wide: P, X, S)
     const int64_t* woff;
     double* part;   // 64 x 64 parts of F21bar' L21, by CTA of k_adj_rows
+    const int* odd;
+    __device__ void scalar_front(int s) const {
+        adj_front(s, fronts, Ls, Fb, Fu, zuoff, W, woff);
+    }
 };
 struct AdjList {
     const int* items;
@@ -274,7 +300,7 @@ __device__ __forceinline__ double adj_l21bar(const FrontDesc& f, const double* L
 
 // MT, NT: 64-column products, or 16-column ones for fronts of c <= 16
 template <int MT, int NT>
-__device__ void adj_rows(const AdjData& D, const AdjJob& job, double* adj_sm) {
+__device__ void adj_rows(const AdjData& D, const AdjJob& job, int odd, double* adj_sm) {
     using namespace t64;
     const FrontDesc& f = job.f;
     const int c = f.c, u = f.m - c, a0 = T * job.q, rows = min(T, u - a0);
@@ -286,6 +312,7 @@ __device__ void adj_rows(const AdjData& D, const AdjJob& job, double* adj_sm) {
     double acc[MT][NT][2][4];
     zero(acc);
     if (U) adj_ubar_l21(f, L, U, a0, 0, c, adj_sm, acc);
+    if (odd) return;  // (looked at here: its load is long back)
     // R = L21bar less the sum, as the K-slowest operand [column][row]; W
     // beside it [k][column]
     double* R = adj_sm;
@@ -325,11 +352,12 @@ __device__ void adj_rows(const AdjData& D, const AdjJob& job, double* adj_sm) {
 
 __global__ void __launch_bounds__(t64::THREADS, 3) k_adj_rows(AdjData D, AdjList w) {
     extern __shared__ __align__(16) double adj_sm[];
+    const int odd = *D.odd;
     const AdjJob job(D, w);
     if (job.f.c <= 16)
-        adj_rows<1, 1>(D, job, adj_sm);
+        adj_rows<1, 1>(D, job, odd, adj_sm);
     else
-        adj_rows<2, 2>(D, job, adj_sm);
+        adj_rows<2, 2>(D, job, odd, adj_sm);
 }
 
 // The pivot block of a narrow front: L11bar less the row tiles' parts, then
@@ -337,7 +365,7 @@ __global__ void __launch_bounds__(t64::THREADS, 3) k_adj_rows(AdjData D, AdjList
 __global__ void __launch_bounds__(t64::THREADS, 3) k_adj_pivot(AdjData D, AdjList w) {
     using namespace t64;
     extern __shared__ __align__(16) double adj_sm[];
-    const int s = w.items[blockIdx.x];
+    const int odd = *D.odd, s = w.items[blockIdx.x];
     const FrontDesc f = D.fronts[s];
     const int c = f.c;
     const double* L = D.Ls + f.loff;
@@ -359,6 +387,10 @@ __global__ void __launch_bounds__(t64::THREADS, 3) k_adj_pivot(AdjData D, AdjLis
         }
         A[k * LD + i] = in ? L[k + (int64_t)i * f.ldl] : 0.0;  // L(k, i)
         B[k * LD + i] = g;                                     // L11bar(k, i)
+    }
+    if (odd) {
+        D.scalar_front(s);
+        return;
     }
     __syncthreads();
     // a warp whose rows or columns are all past c has nothing to add
@@ -396,7 +428,9 @@ __global__ void __launch_bounds__(t64::THREADS, 3) k_adj_pivot(AdjData D, AdjLis
 __global__ void __launch_bounds__(t64::THREADS, 3) k_adj_w_l21(AdjData D, AdjList w) {
     using namespace t64;
     extern __shared__ __align__(16) double adj_sm[];
+    const int odd = *D.odd;
     const AdjJob job(D, w);
+    if (odd) return;
     const FrontDesc& f = job.f;
     const int u = f.m - f.c, nrt = (u + T - 1) / T;
     const int a0 = T * (job.q % nrt), c0 = T * (job.q / nrt);
@@ -452,7 +486,9 @@ __device__ void adj_solve_rows(const FrontDesc& f, const double* L, const double
 // F21bar = L21bar L11^-1: CTA per 64 rows
 __global__ void __launch_bounds__(t64::THREADS, 3) k_adj_w_f21(AdjData D, AdjList w) {
     extern __shared__ __align__(16) double adj_sm[];
+    const int odd = *D.odd;
     const AdjJob job(D, w);
+    if (odd) return;
     const FrontDesc& f = job.f;
     const int a0 = t64::T * job.q;
     adj_solve_rows(f, D.Ls + f.loff, D.Dinv + D.dinv_off[job.s], D.Fb + f.loff + f.c + a0, f.ldl,
@@ -463,7 +499,9 @@ __global__ void __launch_bounds__(t64::THREADS, 3) k_adj_w_f21(AdjData D, AdjLis
 __global__ void __launch_bounds__(t64::THREADS, 3) k_adj_w_l11(AdjData D, AdjList w) {
     using namespace t64;
     extern __shared__ __align__(16) double adj_sm[];
+    const int odd = *D.odd;
     const AdjJob job(D, w);
+    if (odd) return;
     const FrontDesc& f = job.f;
     int bi, bj;
     lower_index(job.q, bi, bj);
@@ -491,7 +529,9 @@ __global__ void __launch_bounds__(t64::THREADS, 3) k_adj_w_l11(AdjData D, AdjLis
 __global__ void __launch_bounds__(t64::THREADS, 3) k_adj_w_phi(AdjData D, AdjList w) {
     using namespace t64;
     extern __shared__ __align__(16) double adj_sm[];
+    const int odd = *D.odd;
     const AdjJob job(D, w);
+    if (odd) return;
     const FrontDesc& f = job.f;
     int bi, bj;
     lower_index(job.q, bi, bj);
@@ -519,7 +559,9 @@ __global__ void __launch_bounds__(t64::THREADS, 3) k_adj_w_phi(AdjData D, AdjLis
 // X = P L11^-1 in the scratch's lower tiles: CTA per 64 rows
 __global__ void __launch_bounds__(t64::THREADS, 3) k_adj_w_x(AdjData D, AdjList w) {
     extern __shared__ __align__(16) double adj_sm[];
+    const int odd = *D.odd;
     const AdjJob job(D, w);
+    if (odd) return;
     const FrontDesc& f = job.f;
     const int i0 = t64::T * job.q;
     adj_solve_rows(f, D.Ls + f.loff, D.Dinv + D.dinv_off[job.s], D.W + D.woff[job.s] + i0, f.c,
@@ -532,7 +574,9 @@ __global__ void __launch_bounds__(t64::THREADS, 3) k_adj_w_x(AdjData D, AdjList 
 __global__ void __launch_bounds__(t64::THREADS, 3) k_adj_w_s(AdjData D, AdjList w) {
     using namespace t64;
     extern __shared__ __align__(16) double adj_sm[];
+    const int odd = *D.odd;
     const AdjJob job(D, w);
+    if (odd) return;
     const FrontDesc& f = job.f;
     const int c = f.c, j0 = T * job.q, cols = min(T, c - j0);
     const double* L = D.Ls + f.loff;
@@ -572,7 +616,12 @@ __global__ void __launch_bounds__(t64::THREADS, 3) k_adj_w_s(AdjData D, AdjList 
 __global__ void __launch_bounds__(t64::THREADS) k_adj_w_f11(AdjData D, AdjList w) {
     using namespace t64;
     __shared__ double tr[T][T + 1];
+    const int odd = *D.odd;
     const AdjJob job(D, w);
+    if (odd) {
+        if (job.q == 0) D.scalar_front(job.s);
+        return;
+    }
     const FrontDesc& f = job.f;
     int bi, bj;
     lower_index(job.q, bi, bj);
@@ -607,11 +656,12 @@ __global__ void k_adj_abar(int nnz, const FrontDesc* __restrict__ fronts,
     }
 }
 
-// CTAs of the largest k_adj_rows launch: the 64 x 64 parts it keeps
+// CTAs of the largest k_adj_rows launch: the 64 x 64 parts it keeps, and the odd
+// flag's place behind them
 int64_t adjoint_parts(const DevPlan& D) {
     int64_t p = 1;
     for (const AdjLevel& l : D.adj.h_large) p = std::max<int64_t>(p, l.rows.nctas);
-    return p * t64::T * t64::T;
+    return p * t64::T * t64::T + 1;
 }
 
 void launch_adjoint(const DevPlan& D, int nnz, const double* Ls, const double* Dinv,
@@ -619,7 +669,12 @@ void launch_adjoint(const DevPlan& D, int nnz, const double* Ls, const double* D
                     double* Abar, cudaStream_t st) {
     const AdjSchedule& S = D.adj;
     constexpr size_t SM = t64::SMEM_BYTES;
-    const AdjData data{D.fronts, Ls, Dinv, D.dinv_off, Fb, Fu, D.zuoff, Wscr, S.woff, part};
+    int* odd = reinterpret_cast<int*>(part + adjoint_parts(D) - 1);
+    cudaMemsetAsync(odd, 0, sizeof(int), st);
+    const int sms = D.num_sms > 0 ? D.num_sms : 148;
+    k_adj_check<<<(int)std::min<int64_t>((S.lnz + 1023) / 1024, 8 * sms), 256, 0, st>>>(S.lnz, Lbar,
+                                                                                       odd);
+    const AdjData data{D.fronts, Ls, Dinv, D.dinv_off, Fb, Fu, D.zuoff, Wscr, S.woff, part, odd};
     auto list = [&](const WorkList& w) {
         return AdjList{S.items + w.off, S.before + w.off, w.nitems, w.nctas};
     };

@@ -477,6 +477,7 @@ void upload_plan(mdgpu_handle_s* h, bool check = false) {
             AS.before = h->keep(upload(st.ctas_before));
             AS.woff = h->keep(upload(wo));
             AS.Lp = h->keep(upload(P.Lp));
+            AS.lnz = P.lnz;
             std::vector<int> cf(std::max(P.n, 1), 0);
             for (int s = 0; s < P.nsuper; ++s)
                 std::fill_n(cf.begin() + P.fronts[s].first_col, P.fronts[s].c, s);

@@ -152,6 +152,7 @@ struct AdjSchedule {
     int* before = nullptr;
     std::vector<WorkList> h_gather;  // per level
     int64_t* Lp = nullptr;
+    int64_t lnz = 0;
     int* col_front = nullptr;  // the front of each column of L
     int64_t* woff = nullptr;
     int64_t wtotal = 0;

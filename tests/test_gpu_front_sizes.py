@@ -298,3 +298,37 @@ def test_logdet_of_many_supernodes(tree, prec):
     Lp, _, Lx = S.get_L()
     logs = 2.0 * np.log(Lx[Lp[:-1]])
     assert abs(S.logdet() - logs.sum()) <= (n + 2) * 2.0 ** -52 * np.abs(logs).sum()
+
+
+@pytest.mark.parametrize("c1,c2,u", SIZES)
+@pytest.mark.parametrize("bad", [np.nan, np.inf])
+@pytest.mark.parametrize("where", ["leaf", "root"])
+def test_reverse_mode_of_an_odd_entry(c1, c2, u, bad, where):
+    """L(r, k) does not depend on A's later columns, nor, for an update row r of a
+    front, on that front's other update rows, the fronts beside it or its
+    ancestors: a NaN or an infinity in Lbar(r, k) leaves their gradients what they
+    are with a zero in its place (bound as in test_reverse_mode)."""
+    n, A, Ap, Ai, Ax = _two_leaves(c1, c2, u)
+    S = M.Solver(n, Ap, Ai, ordering=M.ORDER_NATURAL)
+    S.factor(torch.from_numpy(Ax).cuda(), M.FP64)
+    Lp, Li, _ = S.get_L(values=False)
+    cols = np.repeat(np.arange(n), np.diff(Lp))
+    lbar = np.random.default_rng(3).uniform(-1.0, 1.0, len(Li))
+    if where == "leaf":
+        k, r = c1 // 2, c1 + c2 + u // 2
+        kept = (cols > k) | ((Li >= c1) & (Li != r))
+    else:
+        k, r = c1 + c2 + u // 3, n - 1 - u // 4
+        kept = cols > k
+    at = np.flatnonzero((Li == r) & (cols == k))
+    assert len(at) == 1
+    # A's pattern is L's here: the leaves and the root are dense
+    assert np.array_equal(Lp, Ap) and np.array_equal(Li, Ai)
+    lbar[at] = 0.0
+    ref = S.adjoint(lbar)
+    lbar[at] = bad
+    got = S.adjoint(lbar)
+    assert not np.isfinite(got).all()
+    assert np.linalg.norm(got[kept] - ref[kept]) <= 1e-11 * np.linalg.norm(ref)
+    lbar[at] = 0.0
+    assert np.array_equal(S.adjoint(lbar), ref)  # nothing of it stays
