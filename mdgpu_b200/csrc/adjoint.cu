@@ -258,7 +258,7 @@ struct AdjJob {
 };
 
 // operand (Ubar + Ubar')(a0 + x, k): the stored lower entry (the diagonal
-// counted twice by the caller, see add_diag)
+// counted twice by the caller, adj_l21bar)
 struct SymU {
     const double* U;
     int ldu, a0, u;

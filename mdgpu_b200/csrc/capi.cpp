@@ -370,7 +370,6 @@ void upload_plan(mdgpu_handle_s* h, bool check = false) {
         for (int l = 0; l < P.nlevels; ++l) D.h_level_ptr[l + 1] += D.h_level_ptr[l];
         std::vector<int> ll(std::max(P.nsuper, 1)), nxt(D.h_level_ptr.begin(), D.h_level_ptr.end() - 1);
         for (int s = 0; s < P.nsuper; ++s) ll[nxt[lv[s]]++] = s;
-        D.level_list = h->keep(upload(ll));
         // Y scratch of the large fronts, 2 m x 64 (Y of the even and the odd
         // block steps); a level's fronts side by side, levels reuse it
         std::vector<char> large(P.nsuper, 0);
@@ -1060,8 +1059,7 @@ void combine_symbolic(const std::vector<Symbolic>& parts, const std::vector<int>
 }
 
 // Solve error word (d_status[2]): cleared before a public solve call, read
-// after it; bit 0 = a dependency wait of the large-front solve ran out,
-// bit 1 = a solve kernel found its ticket counter not cleared.
+// after it; bit 0 = a wait of the solve ran out.
 void solve_status_reset(mdgpu_handle_s* h, cudaStream_t st) {
     ck(cudaMemsetAsync(h->d_status + 2, 0, sizeof(int), st), "clear solve status");
 }

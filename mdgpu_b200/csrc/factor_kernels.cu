@@ -8,8 +8,12 @@
 //
 // Large fronts: a tiled right-looking partial Cholesky over the [L | U] split
 // storage, batched over all large fronts of one tree level:
-//   k_big_assemble   CTA per (front, 32-column block): zero, scatter A, pull the
-//                    children's update columns that land in the block
+//   k_big_assemble_warp  CTA per (front, 16-column block), a warp per column: A's
+//                    values and the children's update columns that land in it
+//                    (k_big_assemble: the same for the 64-wide schedule below)
+//   k_panel, k_schur_*   (files of their own) the pivot columns in panels of 256,
+//                    each followed by one update of the trailing part
+// FP32 factors with no TMA descriptors step by single tiles instead:
 //   k_tile_potrf     CTA per front: Cholesky of the first diagonal tile, and its
 //                    inverse (kept: it turns every TRSM and every solve step
 //                    with this tile into a small matrix product)
@@ -987,8 +991,8 @@ void launch_large_level(const DevPlan& D, int level, T* Ls, T* Us, T* Dinv, cons
 // Large fronts in 256-column panels: per panel one launch of dependency-
 // ordered row-tile tasks (k_panel: diagonal tiles, triangular solves and the
 // panel's own updates), then one wide Schur update of the whole trailing
-// part -- tcgen05 tensor cores (TF32) for FP32, the register-tiled FP64
-// kernel for FP64.  status[1] receives a device wait's error code (1, 2:
+// part -- tcgen05 tensor cores (TF32) for FP32, the FP64 matrix instructions
+// for FP64.  status[1] receives a device wait's error code (1, 2:
 // the tensor-core pipeline; 3: a panel dependency wait; 4: a panel ticket
 // counter not cleared).
 template <typename T>

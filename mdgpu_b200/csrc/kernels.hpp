@@ -164,8 +164,11 @@ struct DevPlan {
     // launch shapes of the small-front factor kernels, chosen by
     // mdgpu_autotune (these defaults otherwise): the tiny-front kernel's grid
     // cap (blocks of four warps) and the threads of k_small_front per size
-    // bucket (16 warps where shared memory leaves one or two CTAs per SM: 256
-    // threads took 1.2 to 1.4 times as long there)
+    // bucket, for every precision (16 warps where an SM has room for one or two
+    // CTAs: FP64 by shared memory and, with 128 registers a thread, by the register
+    // file, FP32 by shared memory above 128 rows; 256 threads took 1.2 to 1.4 times
+    // as long there.  FP32 fronts of 97..128 rows: three CTAs by shared memory, two
+    // of 512 threads by registers)
     int tiny_blocks_cap = 148 * 8;
     int small_threads[kSmallBuckets] = {64, 128, 128, 256, 512, 512};
     // the factor runs a level's small fronts beside its large fronts (both
@@ -185,9 +188,9 @@ struct DevPlan {
     int* relmap = nullptr;
     int* a_src = nullptr;
     int* a_pos = nullptr;
-    // selected inverse: every supernode by level (root level last), the
-    // Y scratch offset per supernode, and per lower-triangle entry its front
-    int* level_list = nullptr;
+    // selected inverse: the supernodes of each level (counts as offsets, root
+    // level last), the Y scratch offset per supernode, and per lower-triangle
+    // entry its front
     std::vector<int> h_level_ptr;  // nlevels + 1
     int64_t* yoff = nullptr;
     SelSchedule sel;

@@ -121,7 +121,7 @@ struct PanelProd<float> {
     // tri_col(e)
     static __device__ __forceinline__ void tri(const float* As, const float* Bs, int K,
                                                float (&acc)[16]) {
-        tile_gemm_tri<float, kTile>(As, Bs, K, reinterpret_cast<float(&)[4][4]>(acc));
+        tile_gemm_tri<kTile>(As, Bs, K, reinterpret_cast<float(&)[4][4]>(acc));
     }
     // acc += A A', its lower part
     static __device__ __forceinline__ void square(const float* As, float (&acc)[16]) {

@@ -5,8 +5,10 @@
 // on the FP64 matrix instructions (dmma.cuh): a tile is four CTAs of 64 x 64
 // (128 threads, warps of 32 x 32, three CTAs per SM, so one CTA's epilogue
 // runs under the others' products), operand chunks of 16 panel columns
-// through a three-stage cp.async ring.  Bound by the FP64 pipe (37 TFLOP/s
-// measured): 16.4 k cycles of an SM per CTA for 0.3 MB of operands and C.
+// through a three-stage cp.async ring.  The FP64 pipe is the busiest unit, 58 %
+// of the longest launch of a 40^3 factor: 16.4 k cycles of it per CTA for 0.3 MB
+// of operands and C; the rest is whole tiles at the fronts' edges, the last wave
+// and the chunk loads.
 // Measured on the 48^3 grid's FP64 factor (80 launches): 6.5 ms, 18 TFLOP/s
 // with the launches' tails, against 14.1 ms for 128 x 128 tiles of register
 // FMAs (an LDS.128 per four of them) and 7.8 ms for CTAs of 64 x 128 (two per

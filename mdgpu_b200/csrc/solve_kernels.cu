@@ -1247,33 +1247,12 @@ __device__ void bwd_chain_task(int2 tk, const FrontDesc* __restrict__ fronts,
 // forward update tiles with one right-hand side: L read straight from global
 // memory into registers, coalesced (a thread per row), the next columns'
 // loads issued before the current ones are used, no block barrier per L
-// block.  The pivot tiles' published vectors come through poll_published
-// into a shared double buffer (a buffer is rewritten two polls later, after
-// the barrier of the poll between).
-// ---------------------------------------------------------------------------
-
-// (fronts of one pivot tile only: with more, one column group of loads in
-// flight per iteration leaves a tail of one memory latency per 16 columns
+// block.  For fronts of one pivot tile, whose published vector comes through
+// poll_published into shared memory (with more tiles, one column group of loads
+// in flight per iteration leaves a tail of one memory latency per 16 columns
 // after the last pivot tile, where the staged tile path keeps two 64-column
-// blocks in flight)
-constexpr int kRt1MaxPivotTiles = 1;
-
-struct Rt1Smem {
-    double* Ys;  // 2 x T: published slots
-    __device__ Rt1Smem() {
-        extern __shared__ __align__(16) unsigned char smem_raw[];
-        Ys = reinterpret_cast<double*>(smem_raw);
-    }
-};
-template <typename TL>
-__host__ __device__ constexpr size_t rt1_smem_bytes() {
-    return 2 * (size_t)kTile * sizeof(double);
-}
-
-template <typename TL>
-__device__ __forceinline__ TL ldL(const TL* p) {
-    return __ldg(p);
-}
+// blocks in flight).
+// ---------------------------------------------------------------------------
 
 // Forward update rows [R0, R1) of front s (at most 256; one right-hand side):
 // thread = row; columns in groups of 16, the next group's loads issued
@@ -1284,19 +1263,18 @@ __device__ void fwd_update_rt1(int s, int R0, int R1, const FrontDesc& F, double
                                const int* __restrict__ amap_row,
                                const int* __restrict__ amap_ent, const TL* __restrict__ Ls,
                                double* __restrict__ f, const double* __restrict__ fv) {
-    constexpr int T = kTile;
-    const Rt1Smem sm;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    double* Y = reinterpret_cast<double*>(smem_raw);  // the pivot tile's values
     const int R = R0 + threadIdx.x;
     const bool rv = R < R1;
     const TL* Lr = Ls + F.loff + R;
     constexpr int GW = sizeof(TL) == 4 ? 16 : 8;  // columns per group (registers)
-    constexpr int GPB = T / GW;                     // groups per 64-column block
     const int ng = (F.c + GW - 1) / GW;
     auto load = [&](int cg, TL (&v)[GW]) {
 #pragma unroll
         for (int l = 0; l < GW; ++l) {
             const int col = GW * cg + l;
-            v[l] = (rv && col < F.c) ? ldL(Lr + (int64_t)col * F.ldl) : TL(0);
+            v[l] = (rv && col < F.c) ? __ldg(Lr + (int64_t)col * F.ldl) : TL(0);
         }
     };
     double acc = 0.0;
@@ -1306,12 +1284,8 @@ __device__ void fwd_update_rt1(int s, int R0, int R1, const FrontDesc& F, double
     gather_entries<1>(rv, amap_row + amap_off[s] + R, amap_ent, fv, 1, 1, f0, ab);
     for (int cg = 0; cg < ng; ++cg) {
         if (cg + 1 < ng) load(cg + 1, ln);
-        const int k = cg / GPB;
-        double* Yk = sm.Ys + (k & 1) * T;
-        if (cg % GPB == 0 &&
-            !poll_published(Yk, pb + (int64_t)k * T, min(T, F.c - k * T), 1, ab))
-            return;
-        const double* y = Yk + GW * (cg % GPB);
+        if (cg == 0 && !poll_published(Y, pb, F.c, 1, ab)) return;
+        const double* y = Y + GW * cg;
 #pragma unroll
         for (int l = 0; l < GW; ++l) acc += (double)lv[l] * y[l];
 #pragma unroll
@@ -1392,11 +1366,10 @@ __global__ void __launch_bounds__(256, solve_ctas_per_sm<TL>())
                 const int s = tk.x, i0 = tk.y & 0xffff, cnt = tk.y >> 16;
                 const FrontDesc F = fronts[s];
                 const int nt1 = tiles_l(F.c, T);
-                if (i0 >= nt1 && nt1 <= kRt1MaxPivotTiles) {
-                    // update tiles of fronts with at most kRt1MaxPivotTiles
-                    // pivot tiles, one right-hand side: registers straight
-                    // from L (measured faster there; the staged pipeline
-                    // streams long column ranges better)
+                if (i0 >= nt1 && nt1 == 1) {
+                    // update tiles of fronts of one pivot tile, one right-hand
+                    // side: registers straight from L (measured faster there;
+                    // the staged pipeline streams long column ranges better)
                     double* pb = pub + (dinv_off[s] / (T * T)) * T;
                     const TileRange a = tile_range(i0, F.m, F.c, T);
                     const TileRange b = tile_range(i0 + cnt - 1, F.m, F.c, T);
@@ -1528,7 +1501,6 @@ void permute_solution(const DevPlan& D, const int* perm, const double* fv, doubl
 template <typename TL, bool MULTI>
 static size_t solve_smem() {
     size_t m = level_smem_bytes<TL, MULTI>();
-    if (!MULTI) m = std::max(m, rt1_smem_bytes<TL>());
     return std::max(m, 8 * (size_t)warp_buf<MULTI>() * sizeof(double));
 }
 

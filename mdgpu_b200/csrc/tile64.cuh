@@ -21,7 +21,6 @@ constexpr int T = 64, KS = 32, LD = T + 4, THREADS = 128;
 constexpr int BLOCK = KS * LD;                   // doubles of one operand's stage
 constexpr size_t SMEM_BYTES = 4 * BLOCK * sizeof(double);
 using Acc = double[2][2][2][4];
-using AccThin = double[1][1][2][4];  // 64 x 16: a warp's 16 rows
 
 template <int MT, int NT>
 __device__ __forceinline__ void zero(double (&acc)[MT][NT][2][4]) {

@@ -331,29 +331,20 @@ __device__ __forceinline__ int tri_c0(int tid) {
 
 // As tile_gemm_nt_add for Bs[q][c] zero where q > c (the transposed inverse
 // of a lower triangular tile) or q >= K, at rows 4 (tid mod 16) and columns
-// tri_c0(tid): a warp stops at its own last column.
-template <typename T, int TB>
-__device__ __forceinline__ void tile_gemm_tri(const T* __restrict__ As, const T* __restrict__ Bs,
-                                              int K, T (&acc)[4][4]) {
+// tri_c0(tid): a warp stops at its own last column.  (FP32; FP64 products run on
+// the matrix instructions.)
+template <int TB>
+__device__ __forceinline__ void tile_gemm_tri(const float* __restrict__ As,
+                                              const float* __restrict__ Bs, int K,
+                                              float (&acc)[4][4]) {
     const int tid = threadIdx.x;
     const int r0 = (tid & 15) * 4, c0 = tri_c0(tid);
     const int qn = min((c0 & ~7) + 8, (K + 3) & ~3);
 #pragma unroll 4
     for (int q = 0; q < qn; ++q) {
-        T av[4], bv[4];
-        if constexpr (sizeof(T) == 4) {
-            const float4 a4 = *reinterpret_cast<const float4*>(As + q * TB + r0);
-            const float4 b4 = *reinterpret_cast<const float4*>(Bs + q * TB + c0);
-            av[0] = a4.x, av[1] = a4.y, av[2] = a4.z, av[3] = a4.w;
-            bv[0] = b4.x, bv[1] = b4.y, bv[2] = b4.z, bv[3] = b4.w;
-        } else {
-            const double2 a0 = *reinterpret_cast<const double2*>(As + q * TB + r0);
-            const double2 a1 = *reinterpret_cast<const double2*>(As + q * TB + r0 + 2);
-            const double2 b0 = *reinterpret_cast<const double2*>(Bs + q * TB + c0);
-            const double2 b1 = *reinterpret_cast<const double2*>(Bs + q * TB + c0 + 2);
-            av[0] = a0.x, av[1] = a0.y, av[2] = a1.x, av[3] = a1.y;
-            bv[0] = b0.x, bv[1] = b0.y, bv[2] = b1.x, bv[3] = b1.y;
-        }
+        const float4 a4 = *reinterpret_cast<const float4*>(As + q * TB + r0);
+        const float4 b4 = *reinterpret_cast<const float4*>(Bs + q * TB + c0);
+        const float av[4] = {a4.x, a4.y, a4.z, a4.w}, bv[4] = {b4.x, b4.y, b4.z, b4.w};
 #pragma unroll
         for (int a = 0; a < 4; ++a)
 #pragma unroll
