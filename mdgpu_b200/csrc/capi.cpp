@@ -877,7 +877,9 @@ void download_L(mdgpu_handle_s* h, const T* Ls, double* Lx) {
     std::vector<T> panels;
     for (int s0 = 0, s1; s0 < P.nsuper; s0 = s1) {
         const int64_t base = P.fronts[s0].loff;  // panels lie in front order
-        auto end = [&](int s) { return P.fronts[s].loff + (int64_t)P.fronts[s].ldl * P.fronts[s].c; };
+        auto end = [&](int s) {
+            return P.fronts[s].loff + (int64_t)P.fronts[s].ldl * P.fronts[s].c;
+        };
         for (s1 = s0 + 1; s1 < P.nsuper && end(s1) - base <= kPackDoubles;) ++s1;
         panels.resize(end(s1 - 1) - base);
         ck(cudaMemcpyAsync(panels.data(), Ls + base, panels.size() * sizeof(T),
